@@ -628,9 +628,10 @@ int pcgb_poly_mul_device(uint64_t* d_c, const uint64_t* d_a, const uint64_t* d_b
         const pcgb::NttPlan& pl = pcgb::ntt_plan(pcgb::ilog2i(N));
         uint64_t* scratch = nullptr;
         const size_t n = static_cast<size_t>(batch) * N;
-        scratch = static_cast<uint64_t*>(pcgb::pool_alloc(n * sizeof(uint64_t), st));
+        if (pcgb::poly_mul_needs_scratch(pl))
+            scratch = static_cast<uint64_t*>(pcgb::pool_alloc(n * sizeof(uint64_t), st));
         pcgb::poly_mul_device(pl, d_c, d_a, d_b, batch, scratch, st);
-        PCGB_CK(cudaFreeAsync(scratch, st));
+        if (scratch) PCGB_CK(cudaFreeAsync(scratch, st));
     });
 }
 
@@ -655,10 +656,12 @@ int pcgb_poly_mul_device_multi(int count, uint64_t* const* d_c, const uint64_t* 
         }
         for (int i = 0; i < count; ++i) {
             const pcgb::NttPlan& pl = pcgb::ntt_plan(logN[i]);
-            uint64_t* scratch = static_cast<uint64_t*>(
-                pcgb::pool_alloc(static_cast<size_t>(N[i]) * sizeof(uint64_t), st));
+            uint64_t* scratch = nullptr;
+            if (pcgb::poly_mul_needs_scratch(pl))
+                scratch = static_cast<uint64_t*>(
+                    pcgb::pool_alloc(static_cast<size_t>(N[i]) * sizeof(uint64_t), st));
             pcgb::poly_mul_device(pl, d_c[i], d_a[i], d_b[i], 1, scratch, st);
-            PCGB_CK(cudaFreeAsync(scratch, st));
+            if (scratch) PCGB_CK(cudaFreeAsync(scratch, st));
         }
     });
 }

@@ -7,8 +7,7 @@
 //   z      = sum_{i,j} a_i a_j g_ij = INTT( sum_{i<=j} (a^_i a^_j) . NTT(g_ij + g_ji) )
 //
 // The expander keeps, per shape, the a_i coefficients (Montgomery form, for
-// the sparse x product) and the c(c+1)/2 evaluation images a^_i a^_j
-// (Montgomery-scaled) resident, so an expansion is four device stages:
+// the sparse x product) and the c(c+1)/2 evaluation images a^_i a^_j resident, so an expansion is four device stages:
 // keyed tops -> fused leaf/convert/gather -> sparse x -> NTT multiply-
 // accumulate + inverse.  Blocks (i,j) and (j,i) are merged while g is
 // produced (a_i a_j = a_j a_i), so only c(c+1)/2 forward transforms run.
@@ -157,14 +156,12 @@ __global__ void scale_kernel(uint64_t* d, const uint64_t* s, size_t n, uint64_t 
     if (i < n) d[i] = mont_mul(reduce_p(s[i]), k);
 }
 
-// img = (A .* B) * R  given plain evaluations A, B (B == nullptr means 1).
+// img = A .* B of evaluations in [0, p) (B == nullptr means 1, A too then).
 __global__ void image_kernel(uint64_t* img, const uint64_t* A, const uint64_t* B, size_t n,
-                             uint64_t r2, uint64_t r3) {
+                             uint64_t r2) {
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (!A) { img[i] = mont_mul(1, r2); return; }            // 1 * R (a_0 = 1 both sides)
-    if (!B) { img[i] = mont_mul(A[i], r2); return; }         // A * R
-    img[i] = mont_mul(mont_mul(A[i], B[i]), r3);             // A*B*R
+    img[i] = !A ? 1 : !B ? A[i] : mont_mul(mont_mul(A[i], B[i]), r2);
 }
 
 __global__ void noise_kernel(uint64_t seed, int party, int ct, uint64_t bin, int t, uint64_t* pos,
@@ -292,7 +289,7 @@ pcgb_expander* expander_create(int N, int c, int t, int w, int prg, const uint64
         if (na > 0) PCGB_CK(cudaMalloc(&e->d_aR, sizeof(uint64_t) * NN * na));
         // a_i coefficients (Montgomery form) and evaluations.
         std::vector<uint64_t*> ahat(c, nullptr);
-        const uint64_t r2 = r2_mod_p(), r3 = mul_p_host(r2, r_mod_p());
+        const uint64_t r2 = r2_mod_p();
         if (na > 0) {
             uint64_t* tmp = nullptr;
             PCGB_CK(cudaMalloc(&tmp, sizeof(uint64_t) * NN * na));
@@ -308,13 +305,13 @@ pcgb_expander* expander_create(int N, int c, int t, int w, int prg, const uint64
                 const uint64_t* A = ahat[ij / c];
                 const uint64_t* B = ahat[ij % c];
                 image_kernel<<<blocks_for(NN, 256), 256, 0, st>>>(
-                    e->d_img + NN * k, A ? A : B, A ? B : nullptr, NN, r2, r3);
+                    e->d_img + NN * k, A ? A : B, A ? B : nullptr, NN, r2);
                 PCGB_POST_LAUNCH();
             }
             PCGB_CK(cudaStreamSynchronize(st));
             cudaFree(tmp);
         } else if (Qs > 0) {
-            image_kernel<<<blocks_for(NN, 256), 256, 0, st>>>(e->d_img, nullptr, nullptr, NN, r2, r3);
+            image_kernel<<<blocks_for(NN, 256), 256, 0, st>>>(e->d_img, nullptr, nullptr, NN, r2);
             PCGB_POST_LAUNCH();
         }
         if (prg == PCGB_PRG_AES) {

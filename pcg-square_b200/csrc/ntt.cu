@@ -1,4 +1,5 @@
-// Negacyclic NTT over F_p, four-step form, for N = 2^logN (1 <= logN <= 24).
+// Negacyclic NTT over F_p for N = 2^logN (1 <= logN <= 24): one row up to
+// 2^12 (N = n2, n1 = 1, a single CTA per transform), four-step above.
 //
 // N = n1 * n2 with n1 = 2^floor(logN/2), n2 = 2^ceil(logN/2); coefficient j
 // sits at row j / n2, column j % n2.  With psi a primitive 2N-th root:
@@ -9,10 +10,7 @@
 //                negacyclic NTT of length n2 on every row (root psi2 =
 //                psi^n1).  The row transform's first stage has a single
 //                root w0; it is folded into the twiddles of the row's upper
-//                half, so that stage only adds and subtracts, and each
-//                element costs one Shoup product by a (value, quotient)
-//                pair where a Montgomery twiddle product and half a
-//                butterfly product stood.
+//                half, so that stage only adds and subtracts.
 // Element (k, k2) then holds A(psi^(2*(i1 + n1*i2) + 1)) with i1 = brev(k),
 // i2 = brev(k2): the evaluations of a(x) mod x^N + 1.  The row pass stores
 // its outputs in a fixed permuted order (below) that every operand of a
@@ -21,10 +19,15 @@
 //
 // Each sub-transform is the merged-twist Cooley-Tukey (forward) /
 // Gentleman-Sande (inverse) negacyclic NTT of Longa and Naehrig (CANS 2016,
-// Algorithms 1-2) with Harvey's lazy butterflies (J. Symbolic Comput. 60,
-// 2014): forward values live in [0, 4p), inverse values in [0, 2p), which
-// 4p < 2^64 allows, and a Shoup product by a precomputed root costs one high
-// and two low 64-bit multiplies.
+// Algorithms 1-2).  Values are signed and lazily reduced: |v| < 2p < 2^63,
+// with products by table entries in (-0.05p, 1.05p) (ntt_arith.cuh).  What
+// bounds the passes is the multiplier pipe together with the register ports
+// it shares with the integer ALU: a butterfly is about 19 instructions (5
+// IMAD.WIDE for the product, one for the fold of the other operand) and 37
+// cycles a warp and sub-partition, against 26 instructions and 47 cycles for
+// Shoup products with Harvey's [0, 4p) ranges (a loop of radix-16 phases in
+// registers).  Sixteen products of 2^20 together with the launches shared by
+// both operands: 835 -> 753 us.
 //
 // Register blocking.  A thread owns E = 16 elements of one sub-transform of
 // length n = 2^L (all n when n < 16), so T = n / 16 threads share it.  The L
@@ -62,6 +65,7 @@
 #include <vector>
 
 #include "field.cuh"
+#include "ntt_arith.cuh"
 
 namespace pcgb {
 
@@ -69,68 +73,67 @@ struct NttPlan {
     int logN = 0, l1 = 0, l2 = 0;
     size_t N = 0;
     int n1 = 0, n2 = 0;
-    ulonglong2* tw1 = nullptr;    // column roots (value, shoup), phase-permuted
-    ulonglong2* tw1i = nullptr;
-    ulonglong2* tw2 = nullptr;    // row roots
-    ulonglong2* tw2i = nullptr;
-    // [n1][n2] four-step twiddles as Shoup pairs, the row transform's first
-    // (forward) / last (inverse) root folded into the upper half of each row
-    ulonglong2* Wf = nullptr;     // forward twiddle
-    ulonglong2* Wif = nullptr;    // inverse twiddle * N^-1
-    ulonglong2* WiRf = nullptr;   // Wif * 2^64: for products of two plain transforms
-    std::mutex mu;                // guards the lazy WiRf
+    NttTw* tw1 = nullptr;    // column roots, phase-permuted (none when l1 = 0)
+    NttTw* tw1i = nullptr;
+    NttTw* tw2 = nullptr;    // row roots
+    NttTw* tw2i = nullptr;
+    // [n1][n2] four-step twiddles, the row transform's first (forward) / last
+    // (inverse) root folded into the upper half of each row
+    NttTw* Wf = nullptr;     // forward twiddle
+    NttTw* Wif = nullptr;    // inverse twiddle * N^-1
+    bool direct() const { return l1 == 0; }   // one row: no column passes
 };
 
 namespace {
 
-constexpr uint64_t k2P = 2 * kPm;
+// ---- butterflies -------------------------------------------------------------
+// Values are signed and lazily reduced (ntt_arith.cuh): a product t lies in
+// [-e p, (1 + e)p], e < 0.05, for a factor below 1.7p in magnitude.
 
-// ---- lazy field arithmetic ------------------------------------------------
-
-__device__ __forceinline__ uint64_t csub(uint64_t a, uint64_t m) { return a >= m ? a - m : a; }
-
-// a*w mod p in [0, 2p) for any 64-bit a; wq = floor(w * 2^64 / p).
-__device__ __forceinline__ uint64_t shoup_lazy(uint64_t a, uint64_t w, uint64_t wq) {
-    const uint64_t q = __umul64hi(a, wq);
-    return a * w - q * kPm;
+// Forward butterfly X + wY, X - wY.  A stage with FOLD brings X back first;
+// the next one adds another product to that, shifted by p so that the range
+// stays centred, which needs the role the element had in the last stage:
+//   FIRST  X in [-e, 1 + e]p           -> both within (1 + 2e)p
+//   FOLD   |X| < 1.75p, folded to +-p/2 -> X' in [-1/2 - e, 3/2 + e]p, Y' in
+//                                         its negative
+//   XROLE  X an X' of a FOLD stage     -> both within (1.5 + 2e)p
+//   YROLE  X a Y' of a FOLD stage      -> both within (1.5 + 2e)p
+enum CtKind { kCtFirst, kCtFold, kCtXRole, kCtYRole };
+__device__ __forceinline__ void ct_bfly(int64_t& X, int64_t& Y, const NttTw& w, CtKind kind) {
+    const int64_t x = kind == kCtFold ? fold_centred(X) : X;
+    const int64_t t = mul_tw(Y, w);
+    X = (kind == kCtFirst || kind == kCtXRole) ? x + t - kPs : x + t;
+    Y = kind == kCtYRole ? x - t + kPs : x - t;
+}
+// Stage q of a phase starting at stage s0: phase 0 begins on reduced values
+// and folds at q = 1, 3; later phases fold at q = 0, 2.  xrole: the X operand
+// was an X' of the previous stage.
+__host__ __device__ constexpr CtKind ct_kind(int s0, int q, bool xrole) {
+    if (s0 + q == 0) return kCtFirst;
+    if ((q & 1) == (s0 == 0 ? 1 : 0)) return kCtFold;
+    return xrole ? kCtXRole : kCtYRole;
 }
 
-// Montgomery product a*b*2^-64 in [0, 2p) for a < 4p, b < p.
-__device__ __forceinline__ uint64_t mont_lazy(uint64_t a, uint64_t b) {
-    const uint64_t lo = a * b;
-    const uint64_t hi = __umul64hi(a, b);
-    const uint64_t m = lo * kPNegInv;
-    return hi + __umul64hi(m, kPm) + (lo != 0 ? 1 : 0);
-}
-
-// Forward butterfly: X, Y in [0, 4p) -> X + wY, X - wY in [0, 4p).
-__device__ __forceinline__ void ct_bfly(uint64_t& X, uint64_t& Y, ulonglong2 w) {
-    const uint64_t x = csub(X, k2P);
-    const uint64_t t = shoup_lazy(Y, w.x, w.y);
-    X = x + t;
-    Y = x - t + k2P;
-}
-
-// Inverse butterfly: X, Y in [0, 2p) -> X + Y, (X - Y) w in [0, 2p).
-__device__ __forceinline__ void gs_bfly(uint64_t& X, uint64_t& Y, ulonglong2 w) {
-    const uint64_t s = csub(X + Y, k2P);
-    Y = shoup_lazy(X - Y + k2P, w.x, w.y);
+// Inverse butterfly: X, Y in [-0.25p, 1.25p] -> X + Y in [0, p] up to 2d,
+// (X - Y) w in [-e p, (1 + e)p].
+__device__ __forceinline__ void gs_bfly(int64_t& X, int64_t& Y, const NttTw& w) {
+    const int64_t s = fold(X + Y - kPs);
+    Y = mul_tw(X - Y, w);
     X = s;
 }
 
 // Butterfly of a stage whose root has been folded into the per-element
 // twiddles (the row pass's first forward stage and last inverse stage):
-// X, Y in [0, 2p) -> X + Y, X - Y in [0, 4p).
-__device__ __forceinline__ void add_sub_bfly(uint64_t& X, uint64_t& Y) {
-    const uint64_t s = X + Y;
-    Y = X - Y + k2P;
+// X, Y in [-e p, (1 + e)p] -> X + Y, X - Y within (1 + 2e)p.
+__device__ __forceinline__ void add_sub_bfly(int64_t& X, int64_t& Y) {
+    const int64_t s = X + Y - kPs;
+    Y = X - Y;
     X = s;
 }
 
-// Shoup product with a per-element twiddle pair (value, quotient).
-__device__ __forceinline__ uint64_t shoup_tw(uint64_t a, const ulonglong2* __restrict__ w) {
-    const ulonglong2 v = __ldg(w);
-    return shoup_lazy(a, v.x, v.y);
+__device__ __forceinline__ NttTw ldtw(const NttTw* __restrict__ w) {
+    const int4 v = __ldg(reinterpret_cast<const int4*>(w));
+    return NttTw{v.x, v.y, v.z, v.w};
 }
 
 // ---- phase geometry ----------------------------------------------------------
@@ -167,8 +170,8 @@ __device__ __forceinline__ int perm_pos(int i) {
 // twiddles the caller applies (before the forward phases, after the inverse
 // ones), so it is a plain add/sub; its inputs are in [0, 2p).
 template <int L, int P, bool INV, bool FOLD>
-__device__ __forceinline__ void run_phase(uint64_t (&x)[Geo<L>::E], int t,
-                                          const ulonglong2* __restrict__ tw) {
+__device__ __forceinline__ void run_phase(int64_t (&x)[Geo<L>::E], int t,
+                                          const NttTw* __restrict__ tw) {
     constexpr int s0 = 4 * P, r = Geo<L>::r(P), U = Geo<L>::E >> r, ltl = L - s0 - r;
 #pragma unroll
     for (int v = 0; v < U; ++v) {
@@ -185,11 +188,13 @@ __device__ __forceinline__ void run_phase(uint64_t (&x)[Geo<L>::E], int t,
                             add_sub_bfly(x[o + kk], x[o + kk + (1 << (r - 1))]);
                         continue;
                     }
-                    const ulonglong2 w = __ldg(tw + (1 << (s0 + q)) + (sub << s0) + g);
+                    const NttTw w = ldtw(tw + (1 << (s0 + q)) + (sub << s0) + g);
 #pragma unroll
                     for (int kk = 0; kk < (1 << (r - 1 - q)); ++kk) {
                         const int k = o + (sub << (r - q)) + kk;
-                        ct_bfly(x[k], x[k + (1 << (r - 1 - q))], w);
+                        // k's bit of stage q - 1 tells its role there
+                        const bool xrole = q == 0 || ((k >> (r - q)) & 1) == 0;
+                        ct_bfly(x[k], x[k + (1 << (r - 1 - q))], w, ct_kind(s0, q, xrole));
                     }
                 }
             }
@@ -207,7 +212,7 @@ __device__ __forceinline__ void run_phase(uint64_t (&x)[Geo<L>::E], int t,
                             add_sub_bfly(x[o + kk], x[o + kk + (1 << (r - 1))]);
                         continue;
                     }
-                    const ulonglong2 w = __ldg(tw + (1 << (s0 + q)) + (sub << s0) + g);
+                    const NttTw w = ldtw(tw + (1 << (s0 + q)) + (sub << s0) + g);
 #pragma unroll
                     for (int kk = 0; kk < (1 << (r - 1 - q)); ++kk) {
                         const int k = o + (sub << (r - q)) + kk;
@@ -222,40 +227,44 @@ __device__ __forceinline__ void run_phase(uint64_t (&x)[Geo<L>::E], int t,
 // Element i of one transform in shared memory: base[(i + i/16) * S].
 template <int S>
 struct SmemLay {
-    uint64_t* base;
-    __device__ __forceinline__ uint64_t& at(int i) const { return base[(i + (i >> 4)) * S]; }
+    int64_t* base;
+    __device__ __forceinline__ int64_t& at(int i) const { return base[(i + (i >> 4)) * S]; }
 };
 
-// Registers in phase A layout -> shared memory -> registers in phase B layout.
-template <int L, int A, int B, class Lay>
-__device__ __forceinline__ void exchange(uint64_t (&x)[Geo<L>::E], int t, const Lay& lay) {
+// Registers in phase A layout -> shared memory -> registers in phase B
+// layout.  CLEAN: no thread can still be reading the buffer (the first
+// exchange of a kernel), so the leading barrier is left out.
+template <int L, int A, int B, bool CLEAN, class Lay>
+__device__ __forceinline__ void exchange(int64_t (&x)[Geo<L>::E], int t, const Lay& lay) {
+    if constexpr (!CLEAN) __syncthreads();
 #pragma unroll
     for (int e = 0; e < Geo<L>::E; ++e) lay.at(eidx<L, A>(t, e)) = x[e];
     __syncthreads();
 #pragma unroll
     for (int e = 0; e < Geo<L>::E; ++e) x[e] = lay.at(eidx<L, B>(t, e));
-    __syncthreads();
 }
 
 // All forward phases: registers start in phase 0 layout, end in the last.
-template <int L, bool FOLD, int P = 0, class Lay>
-__device__ __forceinline__ void forward_all(uint64_t (&x)[Geo<L>::E], int t,
-                                            const ulonglong2* __restrict__ tw, const Lay& lay) {
+// CLEAN: as for exchange, of the first one.
+template <int L, bool FOLD, bool CLEAN, int P = 0, class Lay>
+__device__ __forceinline__ void forward_all(int64_t (&x)[Geo<L>::E], int t,
+                                            const NttTw* __restrict__ tw, const Lay& lay) {
     if constexpr (P < Geo<L>::NPH) {
-        if constexpr (P > 0) exchange<L, P - 1, P>(x, t, lay);
+        if constexpr (P > 0) exchange<L, P - 1, P, CLEAN && P == 1>(x, t, lay);
         run_phase<L, P, false, FOLD>(x, t, tw);
-        forward_all<L, FOLD, P + 1>(x, t, tw, lay);
+        forward_all<L, FOLD, CLEAN, P + 1>(x, t, tw, lay);
     }
 }
 
 // All inverse phases: registers start in the last phase layout, end in phase 0.
-template <int L, bool FOLD, int P = Geo<L>::NPH - 1, class Lay>
-__device__ __forceinline__ void inverse_all(uint64_t (&x)[Geo<L>::E], int t,
-                                            const ulonglong2* __restrict__ twi, const Lay& lay) {
+template <int L, bool FOLD, bool CLEAN, int P = Geo<L>::NPH - 1, class Lay>
+__device__ __forceinline__ void inverse_all(int64_t (&x)[Geo<L>::E], int t,
+                                            const NttTw* __restrict__ twi, const Lay& lay) {
     if constexpr (P >= 0) {
-        if constexpr (P < Geo<L>::NPH - 1) exchange<L, P + 1, P>(x, t, lay);
+        if constexpr (P < Geo<L>::NPH - 1)
+            exchange<L, P + 1, P, CLEAN && P == Geo<L>::NPH - 2>(x, t, lay);
         run_phase<L, P, true, FOLD>(x, t, twi);
-        inverse_all<L, FOLD, P - 1>(x, t, twi, lay);
+        inverse_all<L, FOLD, CLEAN, P - 1>(x, t, twi, lay);
     }
 }
 
@@ -264,14 +273,22 @@ __device__ __forceinline__ void inverse_all(uint64_t (&x)[Geo<L>::E], int t,
 // Columns per CTA of the column passes.  Adjacent columns ride on adjacent
 // lanes: 128-byte row segments up to n1 = 512, then 64, 32 and 16 bytes so
 // that the CTA stays at 512 threads.  The column kernels are register-capped
-// for two CTAs per SM (a few spilled words at n1 >= 512), so one CTA's loads
-// overlap the other's butterflies; measured faster than one uncapped CTA.  (n2 >= n1 = 2^L, so C never exceeds
-// the row length.)
+// for 1024 threads per SM (64 registers), so one CTA's loads overlap another's
+// butterflies.  A launch with too few tiles for the chip takes the narrower
+// tiles of col_C_min (col_width).  (n2 >= n1 = 2^L, so C never exceeds the row
+// length.)
 __host__ __device__ constexpr int col_C(int L) {
     return L <= 3 ? (1 << L) : (L <= 9 ? 16 : (L == 10 ? 8 : (L == 11 ? 4 : 2)));
 }
-template <int L>
-__host__ __device__ constexpr int col_threads() { return Geo<L>::T * col_C(L); }
+__host__ __device__ constexpr int col_C_min(int L) {
+    return L >= 6 && L <= 10 ? 4 : col_C(L);
+}
+template <int L, int C>
+__host__ __device__ constexpr int col_threads() { return Geo<L>::T * C; }
+template <int L, int C>
+__host__ __device__ constexpr int col_min_ctas() {
+    return col_threads<L, C>() >= 64 ? 1024 / col_threads<L, C>() : 16;
+}
 // Transforms per CTA of the row passes (n1 >= 2^(L-1) rows exist).
 template <int L>
 __host__ __device__ constexpr int row_V() {
@@ -280,215 +297,257 @@ __host__ __device__ constexpr int row_V() {
 }
 template <int L>
 __host__ __device__ constexpr int row_threads() { return Geo<L>::T * row_V<L>(); }
+// CTAs per SM the row kernels are compiled for: 768 threads (85 registers).
+// 1024 threads (64 registers) are 2 % faster at 16 x 2^20 and 10 % slower
+// where a pass is one short wave (2^13 .. 2^18).
+template <int L>
+__host__ __device__ constexpr int row_min_ctas() {
+    return row_threads<L>() >= 64 ? 768 / row_threads<L>() + (row_threads<L>() > 768) : 12;
+}
+
+// Up to three transforms of one length and batch in one launch: transform z
+// takes src[z] (plus add[z] when set) to dst[z].
+struct FwdIn {
+    const uint64_t* src[3] = {nullptr, nullptr, nullptr};
+    const uint64_t* add[3] = {nullptr, nullptr, nullptr};
+    uint64_t* dst[3] = {nullptr, nullptr, nullptr};
+};
+template <class T>
+__device__ __forceinline__ T pick(T const (&v)[3], int z) {
+    return z == 0 ? v[0] : (z == 1 ? v[1] : v[2]);
+}
 
 // ---- pass bodies ---------------------------------------------------------------
 // Shared by the per-length kernels (one length, batch in gridDim.y) and the
 // mixed-length kernels (a job table names each CTA's polynomial and tile).
-// Pointers arrive already offset to the polynomial's first word.
+// Pointers arrive already offset to the polynomial's first word.  Buffers
+// between the passes of one transform hold signed lazy values.
+
+// Any 64-bit word (plus another) as a residue in [0, p] up to 3d.
+__device__ __forceinline__ int64_t load_raw(const uint64_t* src, const uint64_t* add, size_t i) {
+    int64_t v = fold_raw(src[i]);
+    if (add) v = fold(v + fold_raw(add[i]) - kPs);
+    return v;
+}
 
 // Column pass, forward, for columns [tile*C, tile*C + C).  src may equal
-// dst (every CTA loads its columns before its first store).  REDUCE maps
-// arbitrary 64-bit inputs into [0, p) first; otherwise inputs must be below
-// 4p.  Outputs in [0, 4p), without the four-step twiddle: the row pass
-// applies it together with its own first root.  L2 >= 0 fixes log2(n2) at
-// compile time (element offsets become immediates); -1 takes l2.
-template <int L, int C, bool REDUCE, int L2 = -1>
-__device__ __forceinline__ void col_fwd_body(const uint64_t* src, uint64_t* dst, int l2,
-                                             size_t tile, const ulonglong2* __restrict__ tw,
-                                             uint64_t* sm) {
+// dst (every CTA loads its columns before its first store).  Inputs are any
+// 64-bit words.  Outputs within 1.6p, without the four-step twiddle: the row pass applies it together with its own first root.  L2
+// fixes log2(n2) at compile time (element offsets become immediates).
+template <int L, int C, int L2>
+__device__ __forceinline__ void col_fwd_body(const uint64_t* src, const uint64_t* add,
+                                             uint64_t* dst, size_t tile,
+                                             const NttTw* __restrict__ tw, int64_t* sm) {
     constexpr int E = Geo<L>::E, LP = last_phase(L);
     const int t = threadIdx.x / C, c = threadIdx.x % C;
-    const size_t n2 = size_t{1} << (L2 >= 0 ? L2 : l2);
+    constexpr size_t n2 = size_t{1} << L2;
     const size_t col = tile * C + c;
-    uint64_t x[E];
+    int64_t x[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const uint64_t v = src[col + eidx<L, 0>(t, e) * n2];
-        x[e] = REDUCE ? reduce_p(v) : v;
-    }
-    forward_all<L, false>(x, t, tw, SmemLay<C>{sm + c});
+    for (int e = 0; e < E; ++e) x[e] = load_raw(src, add, col + eidx<L, 0>(t, e) * n2);
+    forward_all<L, false, true>(x, t, tw, SmemLay<C>{sm + c});
 #pragma unroll
-    for (int e = 0; e < E; ++e) dst[col + eidx<L, LP>(t, e) * n2] = x[e];
+    for (int e = 0; e < E; ++e)
+        dst[col + eidx<L, LP>(t, e) * n2] = static_cast<uint64_t>(x[e]);
 }
 
-// Column pass, inverse, in place (output in natural coefficient order, in
-// [0, p)).  L2 as in col_fwd_body.
-template <int L, int C, int L2 = -1>
-__device__ __forceinline__ void col_inv_body(uint64_t* d, int l2, size_t tile,
-                                             const ulonglong2* __restrict__ twi, uint64_t* sm) {
+// Column pass, inverse, in place: inputs in [-e p, (1 + e)p], output in
+// natural coefficient order, in [0, p).  L2 as in col_fwd_body.
+template <int L, int C, int L2>
+__device__ __forceinline__ void col_inv_body(uint64_t* d, size_t tile,
+                                             const NttTw* __restrict__ twi, int64_t* sm) {
     constexpr int E = Geo<L>::E, LP = last_phase(L);
     const int t = threadIdx.x / C, c = threadIdx.x % C;
-    const size_t n2 = size_t{1} << (L2 >= 0 ? L2 : l2);
+    constexpr size_t n2 = size_t{1} << L2;
     const size_t col = tile * C + c;
-    uint64_t x[E];
+    int64_t x[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) x[e] = d[col + eidx<L, LP>(t, e) * n2];
-    inverse_all<L, false>(x, t, twi, SmemLay<C>{sm + c});
+    for (int e = 0; e < E; ++e)
+        x[e] = static_cast<int64_t>(d[col + eidx<L, LP>(t, e) * n2]);
+    inverse_all<L, false, true>(x, t, twi, SmemLay<C>{sm + c});
 #pragma unroll
-    for (int e = 0; e < E; ++e) d[col + eidx<L, 0>(t, e) * n2] = csub(x[e], kPm);
+    for (int e = 0; e < E; ++e) d[col + eidx<L, 0>(t, e) * n2] = canon(x[e]);
 }
 
-// Row pass, forward, in place on rows [tile*V, tile*V + V) (each thread
-// reads and writes the same set of positions): the four-step twiddle with
-// the row transform's first root folded in (Wf, per element), then the row
-// transform; outputs in [0, p) in the permuted order.
-template <int L, int V>
-__device__ __forceinline__ void row_fwd_body(uint64_t* d, size_t tile,
-                                             const ulonglong2* __restrict__ tw,
-                                             const ulonglong2* __restrict__ Wf, uint64_t* sm) {
-    constexpr int E = Geo<L>::E, T = Geo<L>::T, LP = last_phase(L);
-    const int t = threadIdx.x % T, v = threadIdx.x / T;
-    const size_t base = (tile * V + v) * Geo<L>::n;
-    uint64_t* row = d + base;
-    uint64_t x[E];
+// Row pass, forward, of one row (thread t of its T): the four-step twiddle
+// with the row transform's first root folded in (Wf, the row's first entry),
+// then the row transform; outputs in the permuted order, in [0, p) (CANON) or
+// within 1.6p.  src may equal dst (a row's threads load it
+// before the first barrier or read and write the same positions).  DIRECT:
+// the row is a whole polynomial of any 64-bit words (n1 = 1), untwisted.
+template <int L, bool DIRECT, bool CANON>
+__device__ __forceinline__ void row_fwd_body(const uint64_t* src, const uint64_t* add,
+                                             uint64_t* dst, int t, bool valid,
+                                             const NttTw* __restrict__ tw,
+                                             const NttTw* __restrict__ Wf, int64_t* sm) {
+    constexpr int E = Geo<L>::E, LP = last_phase(L);
+    int64_t x[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const int i = eidx<L, 0>(t, e);
-        x[e] = shoup_tw(row[i], Wf + base + i);
+        if constexpr (DIRECT) x[e] = valid ? load_raw(src, add, i) : 0;
+        else x[e] = mul_tw(static_cast<int64_t>(src[i]), ldtw(Wf + i));
     }
-    forward_all<L, true>(x, t, tw, SmemLay<1>{sm + v * Geo<L>::PAD});
+    forward_all<L, !DIRECT, true>(x, t, tw, SmemLay<1>{sm});
+    if (!valid) return;
 #pragma unroll
     for (int e = 0; e < E; ++e)
-        row[perm_pos<L>(eidx<L, LP>(t, e))] = csub(csub(x[e], k2P), kPm);
+        dst[perm_pos<L>(eidx<L, LP>(t, e))] =
+            CANON ? canon(fold(x[e])) : static_cast<uint64_t>(x[e]);
 }
 
-// Multiply-accumulate row pass on rows [tile*V, tile*V + V):
-//   out row = Wi (.) INTT( sum_q NTT(g_q row) (.) img_q row ),
-// g_q = g + q*N, img_q = img + q*N; img_q in the permuted evaluation order,
-// Montgomery-scaled so that the Montgomery product gives the plain one.
-// g rows come from the column pass (Wf, the forward twiddle, is applied
-// here as in row_fwd_body); Wif is the inverse twiddle with the inverse
-// row transform's last root folded in.  out is in [0, p) and may alias g
-// (a CTA reads all its rows before its first store).  ONE (Q == 1, a plain
-// product): the product stays in the transform's registers, with no
-// separate accumulator live across the forward phases.
-template <int L, int V, bool ONE>
-__device__ __forceinline__ void row_mac_body(const uint64_t* g, const uint64_t* __restrict__ img,
-                                             int Q, size_t N, size_t tile,
-                                             const ulonglong2* __restrict__ tw,
-                                             const ulonglong2* __restrict__ twi,
-                                             const ulonglong2* __restrict__ Wf,
-                                             const ulonglong2* __restrict__ Wif, uint64_t* out,
-                                             uint64_t* sm) {
+// Multiply-accumulate and inverse row pass of one row:
+//   out row = Wi (.) INTT( sum_q g_q row (.) img_q row ),
+// g_q = g + q*N, img_q = img + q*N transforms in the permuted evaluation
+// order (row_fwd_body's output, lazy or canonical); Wif is the inverse
+// twiddle with the inverse row transform's last root folded in.  Each thread
+// loads the permuted positions of its last-phase registers, so the inverse
+// starts where the forward ended.  out is in [-e p, (1 + e)p], or in [0, p)
+// (CANON), and may alias g (a row's threads read all of it before the first
+// store).  The forward transforms ran as a launch of their own: kept in this
+// kernel, Q of them in a row left the chip idle (16 % warps active, 151 us
+// of 262 at N = 2^20, Q = 10; 81 us at N = 2^16, Q = 6).
+template <int L, bool ONE, bool CANON>
+__device__ __forceinline__ void row_mac_inv_body(const uint64_t* g, const uint64_t* img, int Q,
+                                                 size_t N, int t, bool valid,
+                                                 const NttTw* __restrict__ twi,
+                                                 const NttTw* __restrict__ Wif, uint64_t* out,
+                                                 int64_t* sm) {
     constexpr int E = Geo<L>::E, T = Geo<L>::T, LP = last_phase(L);
-    const int t = threadIdx.x % T, v = threadIdx.x / T;
-    const size_t base = (tile * V + v) * Geo<L>::n;
-    const SmemLay<1> lay{sm + v * Geo<L>::PAD};
-    uint64_t acc[E];
-    if constexpr (ONE) {
+    int64_t x[E];
+    if (valid) {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            const size_t i = base + eidx<L, 0>(t, e);
-            acc[e] = shoup_tw(g[i], Wf + i);
+            const int i = perm_pos<L>(eidx<L, LP>(t, e));
+            x[e] = mul_var(static_cast<int64_t>(g[i]), static_cast<int64_t>(img[i]));
         }
-        forward_all<L, true>(acc, t, tw, lay);
+        if constexpr (!ONE) {
+            for (int q = 1; q < Q; ++q) {
+                g += N;
+                img += N;
 #pragma unroll
-        for (int e = 0; e < E; ++e)
-            acc[e] = mont_lazy(acc[e], __ldg(img + base + perm_pos<L>(eidx<L, LP>(t, e))));
+                for (int e = 0; e < E; ++e) {
+                    const int i = perm_pos<L>(eidx<L, LP>(t, e));
+                    x[e] = fold(x[e] - kPs +
+                                mul_var(static_cast<int64_t>(g[i]), static_cast<int64_t>(__ldg(img + i))));
+                }
+            }
+        }
     } else {
 #pragma unroll
-        for (int e = 0; e < E; ++e) acc[e] = 0;
-        for (int q = 0; q < Q; ++q) {
-            const uint64_t* gr = g + q * N + base;
-            const uint64_t* im = img + q * N + base;
-            uint64_t x[E];
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int i = eidx<L, 0>(t, e);
-                x[e] = shoup_tw(gr[i], Wf + base + i);
-            }
-            forward_all<L, true>(x, t, tw, lay);
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const uint64_t m = mont_lazy(x[e], __ldg(im + perm_pos<L>(eidx<L, LP>(t, e))));
-                acc[e] = csub(acc[e] + m, k2P);
-            }
-        }
+        for (int e = 0; e < E; ++e) x[e] = 0;
     }
-    inverse_all<L, true>(acc, t, twi, lay);
+    (void)T;
+    inverse_all<L, true, true>(x, t, twi, SmemLay<1>{sm});
+    if (!valid) return;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        const size_t i = base + eidx<L, 0>(t, e);
-        out[i] = csub(shoup_tw(acc[e], Wif + i), kPm);
+        const int i = eidx<L, 0>(t, e);
+        const int64_t v = mul_tw(x[e], ldtw(Wif + i));
+        out[i] = CANON ? canon(v) : static_cast<uint64_t>(v);
     }
 }
 
-// Pointwise product and inverse row pass on rows [tile*V, tile*V + V) of a
-// transform already in the permuted evaluation order (row_fwd_body's
-// output): out row = Wi (.) INTT( d row (.) img row ), in place, Wi given
-// as WiRf (the inverse twiddle times 2^64, which cancels the Montgomery
-// product's 2^-64, with the last root folded in).  Each thread loads the
-// permuted positions of its last-phase registers, so the inverse starts
-// where the fused forward would have ended.
-template <int L, int V>
-__device__ __forceinline__ void row_pmul_inv_body(uint64_t* d, const uint64_t* __restrict__ img,
-                                                  size_t tile, const ulonglong2* __restrict__ twi,
-                                                  const ulonglong2* __restrict__ WiRf,
-                                                  uint64_t* sm) {
-    constexpr int E = Geo<L>::E, T = Geo<L>::T, LP = last_phase(L);
-    const int t = threadIdx.x % T, v = threadIdx.x / T;
-    const size_t base = (tile * V + v) * Geo<L>::n;
-    uint64_t x[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const size_t i = base + perm_pos<L>(eidx<L, LP>(t, e));
-        x[e] = mont_lazy(d[i], __ldg(img + i));
-    }
-    inverse_all<L, true>(x, t, twi, SmemLay<1>{sm + v * Geo<L>::PAD});
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const size_t i = base + eidx<L, 0>(t, e);
-        d[i] = csub(shoup_tw(x[e], WiRf + i), kPm);
-    }
-}
-
-// ---- per-length kernels: grid = (tiles, batch) ---------------------------------
+// ---- per-length kernels: grid = (tiles, batch, transforms) ------------------------
 
 // The column kernels fix the row length: l2 = L + DL (l2 - l1 is 0 or 1).
-template <int L, bool REDUCE, int DL>
-__global__ void __launch_bounds__(col_threads<L>(), 2) col_fwd_kernel(
-    const uint64_t* src, uint64_t* dst, const ulonglong2* __restrict__ tw) {
-    extern __shared__ uint64_t sm[];
+template <int L, int C, int DL>
+__global__ void __launch_bounds__(col_threads<L, C>(), col_min_ctas<L, C>())
+    col_fwd_kernel(const FwdIn in, const NttTw* __restrict__ tw) {
+    extern __shared__ int64_t sm[];
     const size_t off = static_cast<size_t>(blockIdx.y) << (2 * L + DL);
-    col_fwd_body<L, col_C(L), REDUCE, L + DL>(src + off, dst + off, L + DL, blockIdx.x, tw, sm);
+    const int z = blockIdx.z;
+    const uint64_t* add = pick(in.add, z);
+    col_fwd_body<L, C, L + DL>(pick(in.src, z) + off, add ? add + off : nullptr,
+                               pick(in.dst, z) + off, blockIdx.x, tw, sm);
 }
 
-template <int L, int DL>
-__global__ void __launch_bounds__(col_threads<L>(), 2) col_inv_kernel(
-    uint64_t* d, const ulonglong2* __restrict__ twi) {
-    extern __shared__ uint64_t sm[];
-    col_inv_body<L, col_C(L), L + DL>(d + (static_cast<size_t>(blockIdx.y) << (2 * L + DL)),
-                                      L + DL, blockIdx.x, twi, sm);
+template <int L, int C, int DL>
+__global__ void __launch_bounds__(col_threads<L, C>(), col_min_ctas<L, C>())
+    col_inv_kernel(uint64_t* d, const NttTw* __restrict__ twi) {
+    extern __shared__ int64_t sm[];
+    col_inv_body<L, C, L + DL>(d + (static_cast<size_t>(blockIdx.y) << (2 * L + DL)), blockIdx.x,
+                               twi, sm);
 }
 
-template <int L>
-__global__ void __launch_bounds__(row_threads<L>()) row_fwd_kernel(
-    uint64_t* d, int l1, const ulonglong2* __restrict__ tw, const ulonglong2* __restrict__ Wf) {
-    extern __shared__ uint64_t sm[];
-    row_fwd_body<L, row_V<L>()>(d + (static_cast<size_t>(blockIdx.y) << (L + l1)), blockIdx.x,
-                                tw, Wf, sm);
+// The row of thread group v of this CTA.  DIRECT: rows are the batch's
+// polynomials, V per CTA, the last CTA ragged.
+struct RowAt {
+    size_t inst, base;   // polynomial of the batch; offset of the row in it
+    bool valid;
+};
+template <int L, bool DIRECT>
+__device__ __forceinline__ RowAt row_at(int batch) {
+    const int v = threadIdx.x / Geo<L>::T;
+    const size_t r = static_cast<size_t>(blockIdx.x) * row_V<L>() + v;
+    if constexpr (DIRECT) return RowAt{r, 0, r < static_cast<size_t>(batch)};
+    else return RowAt{blockIdx.y, r << L, true};
 }
 
-template <int L>
-__global__ void __launch_bounds__(row_threads<L>()) row_pmul_inv_kernel(
-    uint64_t* d, const uint64_t* __restrict__ img, int l1, const ulonglong2* __restrict__ twi,
-    const ulonglong2* __restrict__ WiRf) {
-    extern __shared__ uint64_t sm[];
-    const size_t off = static_cast<size_t>(blockIdx.y) << (L + l1);
-    row_pmul_inv_body<L, row_V<L>()>(d + off, img + off, blockIdx.x, twi, WiRf, sm);
+template <int L, bool DIRECT, bool CANON>
+__global__ void __launch_bounds__(row_threads<L>(), row_min_ctas<L>()) row_fwd_kernel(
+    const FwdIn in, int batch, int l1, const NttTw* __restrict__ tw,
+    const NttTw* __restrict__ Wf) {
+    extern __shared__ int64_t sm[];
+    const int t = threadIdx.x % Geo<L>::T, v = threadIdx.x / Geo<L>::T, z = blockIdx.z;
+    const RowAt r = row_at<L, DIRECT>(batch);
+    const size_t off = (r.inst << (L + l1)) + r.base;
+    const uint64_t* add = DIRECT ? pick(in.add, z) : nullptr;
+    row_fwd_body<L, DIRECT, CANON>(pick(in.src, z) + off, add ? add + off : nullptr,
+                                   pick(in.dst, z) + off, t, r.valid, tw, Wf + r.base,
+                                   sm + v * Geo<L>::PAD);
 }
 
 // Instance b reads g and img at b*Q*N and writes out at b*N.
-template <int L, bool ONE>
-__global__ void __launch_bounds__(row_threads<L>()) row_mac_inv_kernel(
-    const uint64_t* g, const uint64_t* __restrict__ img, int Q, int l1,
-    const ulonglong2* __restrict__ tw, const ulonglong2* __restrict__ twi,
-    const ulonglong2* __restrict__ Wf, const ulonglong2* __restrict__ Wif, uint64_t* out) {
-    extern __shared__ uint64_t sm[];
+template <int L, bool DIRECT, bool ONE>
+__global__ void __launch_bounds__(row_threads<L>(), row_min_ctas<L>()) row_mac_inv_kernel(
+    const uint64_t* g, const uint64_t* img, int Q, int batch, int l1,
+    const NttTw* __restrict__ twi, const NttTw* __restrict__ Wif, uint64_t* out) {
+    extern __shared__ int64_t sm[];
+    const int t = threadIdx.x % Geo<L>::T, v = threadIdx.x / Geo<L>::T;
+    const RowAt r = row_at<L, DIRECT>(batch);
     const size_t N = size_t{1} << (L + l1);
-    const size_t b = blockIdx.y;
-    row_mac_body<L, row_V<L>(), ONE>(g + b * Q * N, img + b * Q * N, Q, N, blockIdx.x, tw, twi,
-                                     Wf, Wif, out + b * N, sm);
+    const size_t gi = r.inst * Q * N + r.base;
+    row_mac_inv_body<L, ONE, DIRECT>(g + gi, img + gi, Q, N, t, r.valid, twi, Wif + r.base,
+                                     out + r.inst * N + r.base, sm + v * Geo<L>::PAD);
+}
+
+// A whole product of one-row polynomials (n1 = 1) in one launch: both forward
+// transforms, the pointwise product and the inverse in registers, V products
+// per CTA.  At N = 2^12 it takes 18.5 us, where the passes took 39 (six
+// launches on a handful of CTAs, 12 for a batch); it is bound by the
+// multiplier pipe of one SM (73.7 K butterflies at about 37 cycles a warp).  A
+// second half of the CTA for b's transform gained nothing (24.8 us).  c may
+// alias a or b.
+template <int L>
+__global__ void __launch_bounds__(row_threads<L>()) row_product_kernel(
+    uint64_t* c, const uint64_t* a, const uint64_t* b, int batch,
+    const NttTw* __restrict__ tw, const NttTw* __restrict__ twi,
+    const NttTw* __restrict__ Wif) {
+    extern __shared__ int64_t sm[];
+    constexpr int E = Geo<L>::E;
+    const int t = threadIdx.x % Geo<L>::T, v = threadIdx.x / Geo<L>::T;
+    const RowAt r = row_at<L, true>(batch);
+    const size_t off = r.inst << L;
+    const SmemLay<1> lay{sm + v * Geo<L>::PAD};
+    int64_t x[E], y[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const size_t i = off + eidx<L, 0>(t, e);
+        x[e] = r.valid ? fold_raw(a[i]) : 0;
+        y[e] = r.valid ? fold_raw(b[i]) : 0;
+    }
+    forward_all<L, false, true>(x, t, tw, lay);
+    forward_all<L, false, false>(y, t, tw, lay);
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = mul_var(x[e], y[e]);
+    inverse_all<L, true, false>(x, t, twi, lay);
+    if (!r.valid) return;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = eidx<L, 0>(t, e);
+        c[off + i] = canon(mul_tw(x[e], ldtw(Wif + i)));
+    }
 }
 
 // ---- mixed-length kernels --------------------------------------------------------
@@ -504,12 +563,12 @@ struct MixedPoly {
     const uint64_t* b;
     uint64_t* c;
     uint64_t* A;                 // NTT(a), scratch
-    const ulonglong2* tw1;
-    const ulonglong2* tw1i;
-    const ulonglong2* tw2;
-    const ulonglong2* tw2i;
-    const ulonglong2* Wf;
-    const ulonglong2* WiRf;
+    const NttTw* tw1;
+    const NttTw* tw1i;
+    const NttTw* tw2;
+    const NttTw* tw2i;
+    const NttTw* Wf;
+    const NttTw* Wif;
     int l1, l2;
 };
 struct MixedCta {
@@ -521,12 +580,31 @@ template <int L>
 __host__ __device__ constexpr int mixed_C() { return kMixedColThreads / Geo<L>::T; }
 template <int L>
 __host__ __device__ constexpr int mixed_V() { return kMixedRowThreads / Geo<L>::T; }
-static_assert(mixed_V<8>() == row_V<8>() && mixed_V<9>() == row_V<9>() &&
-              mixed_V<10>() == row_V<10>(), "row CTA shapes agree");
 constexpr size_t kMixedColSmem = sizeof(uint64_t) * Geo<10>::PAD * mixed_C<10>();
 constexpr size_t kMixedRowSmem = sizeof(uint64_t) * Geo<10>::PAD * mixed_V<10>();
 static_assert(sizeof(uint64_t) * Geo<8>::PAD * mixed_C<8>() == kMixedColSmem &&
               sizeof(uint64_t) * Geo<9>::PAD * mixed_C<9>() == kMixedColSmem, "col smem");
+
+// Row `tile * V + thread group` of a row CTA of the mixed shapes.
+template <int L>
+struct MixedRow {
+    int t = threadIdx.x % Geo<L>::T, v = threadIdx.x / Geo<L>::T;
+    size_t base;
+    __device__ __forceinline__ explicit MixedRow(uint32_t tile)
+        : base((static_cast<size_t>(tile) * mixed_V<L>() + threadIdx.x / Geo<L>::T) << L) {}
+    __device__ __forceinline__ void fwd(uint64_t* d, const NttTw* tw, const NttTw* Wf,
+                                        int64_t* sm) const {
+        row_fwd_body<L, false, false>(d + base, nullptr, d + base, t, true, tw, Wf + base,
+                                      sm + v * Geo<L>::PAD);
+    }
+    template <bool ONE>
+    __device__ __forceinline__ void mac_inv(const uint64_t* g, const uint64_t* img, int Q, size_t N,
+                                            const NttTw* twi, const NttTw* Wif, uint64_t* out,
+                                            int64_t* sm) const {
+        row_mac_inv_body<L, ONE, false>(g + base, img + base, Q, N, t, true, twi, Wif + base,
+                                        out + base, sm + v * Geo<L>::PAD);
+    }
+};
 
 #define PCGB_MIXED_SWITCH(LEN, CALL) \
     switch (LEN) {                    \
@@ -546,50 +624,51 @@ static_assert(sizeof(uint64_t) * Geo<8>::PAD * mixed_C<8>() == kMixedColSmem &&
         default: break;                                \
     }
 
-// which = 0: column pass of a into A; which = 1: column pass of b into c.
+// Column pass of a into A (which = 0) and of b into c (which = 1), which =
+// first + blockIdx.y.
 __global__ void __launch_bounds__(kMixedColThreads, 2) mixed_col_fwd_kernel(
-    const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas, int which) {
-    extern __shared__ uint64_t sm[];
+    const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas, int first) {
+    extern __shared__ int64_t sm[];
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
+    const bool which = first + blockIdx.y != 0;
     const uint64_t* src = which ? p.b : p.a;
     uint64_t* dst = which ? p.c : p.A;
 #define PCGB_CALL(LL, L2) \
-    col_fwd_body<LL, mixed_C<LL>(), true, L2>(src, dst, L2, j.tile, p.tw1, sm)
+    col_fwd_body<LL, mixed_C<LL>(), L2>(src, nullptr, dst, j.tile, p.tw1, sm)
     PCGB_MIXED_COL_SWITCH(p.l1, p.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
 
+// Row pass of A (blockIdx.y = 0) and c (1).
 __global__ void __launch_bounds__(kMixedRowThreads) mixed_row_fwd_kernel(
     const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas) {
-    extern __shared__ uint64_t sm[];
+    extern __shared__ int64_t sm[];
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
-#define PCGB_CALL(LL) row_fwd_body<LL, mixed_V<LL>()>(p.A, j.tile, p.tw2, p.Wf, sm)
+    uint64_t* d = blockIdx.y ? p.c : p.A;
+#define PCGB_CALL(LL) MixedRow<LL>(j.tile).fwd(d, p.tw2, p.Wf, sm)
     PCGB_MIXED_SWITCH(p.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
 
-// c = Wi*R (.) INTT( NTT_rows(c) (.) A ), in place on c.
-__global__ void __launch_bounds__(kMixedRowThreads) mixed_row_mac_kernel(
+// c = Wi (.) INTT( c (.) A ), in place on c.
+__global__ void __launch_bounds__(kMixedRowThreads) mixed_row_mul_kernel(
     const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas) {
-    extern __shared__ uint64_t sm[];
+    extern __shared__ int64_t sm[];
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
-    const size_t N = size_t{1} << (p.l1 + p.l2);
-#define PCGB_CALL(LL) \
-    row_mac_body<LL, mixed_V<LL>(), true>(p.c, p.A, 1, N, j.tile, p.tw2, p.tw2i, p.Wf, p.WiRf, \
-                                          p.c, sm)
+#define PCGB_CALL(LL) MixedRow<LL>(j.tile).template mac_inv<true>(p.c, p.A, 1, 0, p.tw2i, p.Wif, p.c, sm)
     PCGB_MIXED_SWITCH(p.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
 
 __global__ void __launch_bounds__(kMixedColThreads, 2) mixed_col_inv_kernel(
     const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas) {
-    extern __shared__ uint64_t sm[];
+    extern __shared__ int64_t sm[];
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
-#define PCGB_CALL(LL, L2) col_inv_body<LL, mixed_C<LL>(), L2>(p.c, L2, j.tile, p.tw1i, sm)
+#define PCGB_CALL(LL, L2) col_inv_body<LL, mixed_C<LL>(), L2>(p.c, j.tile, p.tw1i, sm)
     PCGB_MIXED_COL_SWITCH(p.l1, p.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
@@ -598,21 +677,21 @@ __global__ void __launch_bounds__(kMixedColThreads, 2) mixed_col_inv_kernel(
 
 // ---- multi-request multiply-accumulate ------------------------------------
 // The step-4 transforms of several expansions of different lengths
-// 2^14 .. 2^20 (sub-lengths 2^7 .. 2^10) in three launches: the column pass
-// of every request's Q g' buffers, the Q-way multiply-accumulate row pass
-// with its inverse, and the inverse column pass into each request's z.  The
-// CTA shapes are the mixed kernels' (512 column threads, 64 row threads,
-// the same shared memory at every sub-length down to 2^7).
+// 2^14 .. 2^20 (sub-lengths 2^7 .. 2^10) in four launches: the column and the
+// row pass of every request's Q g' buffers, the Q-way multiply-accumulate
+// with the inverse row pass, and the inverse column pass into each request's
+// z.  The CTA shapes are the mixed kernels' (512 column threads, 64 row
+// threads, the same shared memory at every sub-length down to 2^7).
 struct MacReq {
-    uint64_t* g;                 // Q*N words, column-transformed in place
-    const uint64_t* img;         // Q*N, Montgomery-scaled evaluation images
+    uint64_t* g;                 // Q*N words, transformed in place
+    const uint64_t* img;         // Q*N, evaluation images
     uint64_t* z;                 // N
-    const ulonglong2* tw1;
-    const ulonglong2* tw1i;
-    const ulonglong2* tw2;
-    const ulonglong2* tw2i;
-    const ulonglong2* Wf;
-    const ulonglong2* Wif;
+    const NttTw* tw1;
+    const NttTw* tw1i;
+    const NttTw* tw2;
+    const NttTw* tw2i;
+    const NttTw* Wf;
+    const NttTw* Wif;
     int Q, l1, l2;
 };
 struct MacCta {
@@ -645,45 +724,53 @@ static_assert(sizeof(uint64_t) * Geo<7>::PAD * mixed_C<7>() == kMixedColSmem &&
 
 __global__ void __launch_bounds__(kMixedColThreads, 2) mac_col_fwd_kernel(
     const MacReq* __restrict__ reqs, const MacCta* __restrict__ ctas) {
-    extern __shared__ uint64_t sm[];
+    extern __shared__ int64_t sm[];
     const MacCta j = ctas[blockIdx.x];
     const MacReq& r = reqs[j.req];
     uint64_t* d = r.g + (static_cast<size_t>(j.q) << (r.l1 + r.l2));
-#define PCGB_CALL(LL, L2) col_fwd_body<LL, mixed_C<LL>(), false, L2>(d, d, L2, j.tile, r.tw1, sm)
+#define PCGB_CALL(LL, L2) col_fwd_body<LL, mixed_C<LL>(), L2>(d, nullptr, d, j.tile, r.tw1, sm)
     PCGB_MAC_COL_SWITCH(r.l1, r.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
 
-__global__ void __launch_bounds__(kMixedRowThreads) mac_row_kernel(
+__global__ void __launch_bounds__(kMixedRowThreads) mac_row_fwd_kernel(
     const MacReq* __restrict__ reqs, const MacCta* __restrict__ ctas) {
-    extern __shared__ uint64_t sm[];
+    extern __shared__ int64_t sm[];
+    const MacCta j = ctas[blockIdx.x];
+    const MacReq& r = reqs[j.req];
+    uint64_t* d = r.g + (static_cast<size_t>(j.q) << (r.l1 + r.l2));
+#define PCGB_CALL(LL) MixedRow<LL>(j.tile).fwd(d, r.tw2, r.Wf, sm)
+    PCGB_MAC_SWITCH(r.l2, PCGB_CALL)
+#undef PCGB_CALL
+}
+
+__global__ void __launch_bounds__(kMixedRowThreads) mac_row_inv_kernel(
+    const MacReq* __restrict__ reqs, const MacCta* __restrict__ ctas) {
+    extern __shared__ int64_t sm[];
     const MacCta j = ctas[blockIdx.x];
     const MacReq& r = reqs[j.req];
     const size_t N = size_t{1} << (r.l1 + r.l2);
 #define PCGB_CALL(LL) \
-    row_mac_body<LL, mixed_V<LL>(), false>(r.g, r.img, r.Q, N, j.tile, r.tw2, r.tw2i, r.Wf, r.Wif, \
-                                           r.z, sm)
+    MixedRow<LL>(j.tile).template mac_inv<false>(r.g, r.img, r.Q, N, r.tw2i, r.Wif, r.z, sm)
     PCGB_MAC_SWITCH(r.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
 
 __global__ void __launch_bounds__(kMixedColThreads, 2) mac_col_inv_kernel(
     const MacReq* __restrict__ reqs, const MacCta* __restrict__ ctas) {
-    extern __shared__ uint64_t sm[];
+    extern __shared__ int64_t sm[];
     const MacCta j = ctas[blockIdx.x];
     const MacReq& r = reqs[j.req];
-#define PCGB_CALL(LL, L2) col_inv_body<LL, mixed_C<LL>(), L2>(r.z, L2, j.tile, r.tw1i, sm)
+#define PCGB_CALL(LL, L2) col_inv_body<LL, mixed_C<LL>(), L2>(r.z, j.tile, r.tw1i, sm)
     PCGB_MAC_COL_SWITCH(r.l1, r.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
 #undef PCGB_MAC_SWITCH
 #undef PCGB_MAC_COL_SWITCH
 
-// Shoup pair (v, floor(v * 2^64 / p)) of v < p given in Montgomery form
-// vR = v * 2^64 mod p: the quotient is (v * 2^64 - vR) / p, an exact
-// division, so it equals vR * (-p^-1) mod 2^64.
-__device__ __forceinline__ ulonglong2 shoup_pair_from_mont(uint64_t vR) {
-    return make_ulonglong2(mont_mul(vR, 1), vR * kPNegInv);
+// The table entry of v given in Montgomery form (v * 2^64); c32 = 2^32 mod p.
+__device__ __forceinline__ NttTw tw_from_mont(uint64_t vR) {
+    return ntt_tw(mont_mul(vR, 1), mont_mul(vR, uint64_t{1} << 32));
 }
 
 // Twiddle tables, element k*n2 + j2 with e = j2*(2*brev(k)+1-n1) mod 2N:
@@ -692,7 +779,7 @@ __device__ __forceinline__ ulonglong2 shoup_pair_from_mont(uint64_t vR) {
 // w0 / w0i being the single root of the row transform's first forward /
 // last inverse stage (that stage then only adds and subtracts).
 // powR[b] = psi^(2^b) * R mod p; w0R, w0iR are w0, w0i times R.
-__global__ void twiddle_kernel(ulonglong2* Wf, ulonglong2* Wif, int l1, int l2,
+__global__ void twiddle_kernel(NttTw* Wf, NttTw* Wif, int l1, int l2,
                                const uint64_t* __restrict__ powR, uint64_t oneR, uint64_t ninvR,
                                uint64_t w0R, uint64_t w0iR) {
     const size_t N = static_cast<size_t>(1) << (l1 + l2);
@@ -716,29 +803,8 @@ __global__ void twiddle_kernel(ulonglong2* Wf, ulonglong2* Wif, int l1, int l2,
         a = mont_mul(a, w0R);
         b = mont_mul(b, w0iR);
     }
-    Wf[idx] = shoup_pair_from_mont(a);
-    Wif[idx] = shoup_pair_from_mont(b);
-}
-
-// dst = src * 2^64 mod p, Shoup pairs; r2 = 2^128 mod p.
-__global__ void scale_r_kernel(ulonglong2* dst, const ulonglong2* __restrict__ src, size_t n,
-                               uint64_t r2) {
-    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint64_t vR = mont_mul(src[i].x, r2);      // v * R: the new value
-    dst[i] = shoup_pair_from_mont(mont_mul(vR, r2));  // from its Montgomery form
-}
-
-// Pointwise products, one word per thread.
-//   mode 0: c = a*b*R^-1          (Montgomery product)
-//   mode 1: c = a*b               (plain product; r2 = R^2 mod p)
-__global__ void pointwise_kernel(uint64_t* c, const uint64_t* a, const uint64_t* b, size_t n,
-                                 int mode, uint64_t r2) {
-    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint64_t v = mont_mul(a[i], b[i]);
-    if (mode == 1) v = mont_mul(v, r2);
-    c[i] = v;
+    Wf[idx] = tw_from_mont(a);
+    Wif[idx] = tw_from_mont(b);
 }
 
 __global__ void reduce_kernel(uint64_t* d, const uint64_t* s, size_t n) {
@@ -771,43 +837,50 @@ uint64_t primitive_root_host() {
 // Roots of a length-2^logn negacyclic transform with psi_n a primitive
 // 2n-th root: stage s, group i uses psi_n^brev_logn(2^s + i) (Longa-Naehrig
 // table), stored at the phase-permuted slot 2^s + (i % 2^q) * 2^s0 + i / 2^q.
-ulonglong2* upload_root_table(uint64_t psi_n, int logn) {
+NttTw* upload_root_table(uint64_t psi_n, int logn) {
     const int n = 1 << logn;
     std::vector<uint64_t> pw(n);
     uint64_t a = 1;
     for (int k = 0; k < n; ++k) { pw[k] = a; a = mul_p_host(a, psi_n); }
-    std::vector<ulonglong2> tab(n > 1 ? n : 2, make_ulonglong2(0, 0));
+    std::vector<NttTw> tab(n > 1 ? n : 2, NttTw{0, 0, 0, 0});
     for (int s = 0; s < logn; ++s) {
         const int s0 = 4 * (s / 4), q = s - s0;
         for (int i = 0; i < (1 << s); ++i) {
             const uint64_t v = pw[brev_host(static_cast<uint32_t>((1 << s) + i), logn)];
             const int slot = (1 << s) + ((i & ((1 << q) - 1)) << s0) + (i >> q);
-            tab[slot] = make_ulonglong2(v, shoup_q_host(v));
+            tab[slot] = ntt_tw_host(v);
         }
     }
-    ulonglong2* d = nullptr;
-    PCGB_CK(cudaMalloc(&d, sizeof(ulonglong2) * tab.size()));
-    upload_blocking(d, tab.data(), sizeof(ulonglong2) * tab.size());
+    NttTw* d = nullptr;
+    PCGB_CK(cudaMalloc(&d, sizeof(NttTw) * tab.size()));
+    upload_blocking(d, tab.data(), sizeof(NttTw) * tab.size());
     return d;
 }
+
+// Lengths up to 2^12 are one row (l1 = 0): a row CTA holds the whole
+// polynomial, so there are no column passes.  At 2^13 one CTA takes 55 us for a
+// product, the column and row passes 24.7.
+constexpr int kDirectLogN = 12;
 
 NttPlan* build_plan(int logN) {
     auto* pl = new NttPlan();
     pl->logN = logN;
     pl->N = static_cast<size_t>(1) << logN;
-    pl->l1 = logN / 2;
+    pl->l1 = logN <= kDirectLogN ? 0 : logN / 2;
     pl->l2 = logN - pl->l1;
     pl->n1 = 1 << pl->l1;
     pl->n2 = 1 << pl->l2;
     const uint64_t g = primitive_root_host();
     const uint64_t psi = pow_p_host(g, (kPm - 1) / (2 * pl->N));
     const uint64_t psi_inv = pow_p_host(psi, kPm - 2);
-    pl->tw1 = upload_root_table(pow_p_host(psi, pl->n2), pl->l1);
-    pl->tw1i = upload_root_table(pow_p_host(psi_inv, pl->n2), pl->l1);
+    if (!pl->direct()) {
+        pl->tw1 = upload_root_table(pow_p_host(psi, pl->n2), pl->l1);
+        pl->tw1i = upload_root_table(pow_p_host(psi_inv, pl->n2), pl->l1);
+    }
     pl->tw2 = upload_root_table(pow_p_host(psi, pl->n1), pl->l2);
     pl->tw2i = upload_root_table(pow_p_host(psi_inv, pl->n1), pl->l2);
-    PCGB_CK(cudaMalloc(&pl->Wf, sizeof(ulonglong2) * pl->N));
-    PCGB_CK(cudaMalloc(&pl->Wif, sizeof(ulonglong2) * pl->N));
+    PCGB_CK(cudaMalloc(&pl->Wf, sizeof(NttTw) * pl->N));
+    PCGB_CK(cudaMalloc(&pl->Wif, sizeof(NttTw) * pl->N));
     const uint64_t R = r_mod_p();
     std::vector<uint64_t> powR(logN + 2);
     uint64_t pb = psi;
@@ -827,8 +900,8 @@ NttPlan* build_plan(int logN) {
     return pl;
 }
 
-template <int L>
-constexpr size_t col_smem() { return Geo<L>::NPH > 1 ? sizeof(uint64_t) * Geo<L>::PAD * col_C(L) : 0; }
+template <int L, int C>
+constexpr size_t col_smem() { return Geo<L>::NPH > 1 ? sizeof(uint64_t) * Geo<L>::PAD * C : 0; }
 template <int L>
 constexpr size_t row_smem() { return Geo<L>::NPH > 1 ? sizeof(uint64_t) * Geo<L>::PAD * row_V<L>() : 0; }
 
@@ -857,73 +930,110 @@ struct OptinOnce {
 };
 OptinOnce g_optin;
 
+// Column tile width for a launch over `work` = columns x batch: the widest
+// one that still gives every SM its 1024 threads, else the narrowest.
+template <int L, int C = col_C(L), class F>
+void col_width(size_t work, F&& f) {
+    if constexpr (C > col_C_min(L)) {
+        const size_t want = static_cast<size_t>(sm_count()) * (1024 / col_threads<L, C>());
+        if (work / C < want) {
+            col_width<L, C / 2>(work, f);
+            return;
+        }
+    }
+    f(std::integral_constant<int, C>{});
+}
+
 template <int L>
-void col_fwd_l(const NttPlan& pl, const uint64_t* src, uint64_t* dst, int batch, bool reduce,
-               cudaStream_t st) {
-    constexpr size_t sm = col_smem<L>();
-    const dim3 grid(pl.n2 / col_C(L), batch);
-    auto go = [&](auto kernel) {
-        g_optin(kernel, sm);
-        kernel<<<grid, col_threads<L>(), sm, st>>>(src, dst, pl.tw1);
-    };
-    const bool odd = pl.l2 != L;
-    if (reduce) odd ? go(col_fwd_kernel<L, true, 1>) : go(col_fwd_kernel<L, true, 0>);
-    else odd ? go(col_fwd_kernel<L, false, 1>) : go(col_fwd_kernel<L, false, 0>);
+void col_fwd_l(const NttPlan& pl, const FwdIn& in, int count, int batch, cudaStream_t st) {
+    col_width<L>(static_cast<size_t>(pl.n2) * batch * count, [&](auto CC) {
+        constexpr int C = decltype(CC)::value;
+        constexpr size_t sm = col_smem<L, C>();
+        auto go = [&](auto kernel) {
+            g_optin(kernel, sm);
+            kernel<<<dim3(pl.n2 / C, batch, count), col_threads<L, C>(), sm, st>>>(in, pl.tw1);
+        };
+        pl.l2 != L ? go(col_fwd_kernel<L, C, 1>) : go(col_fwd_kernel<L, C, 0>);
+    });
     PCGB_POST_LAUNCH();
 }
 
 template <int L>
 void col_inv_l(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
-    constexpr size_t sm = col_smem<L>();
+    col_width<L>(static_cast<size_t>(pl.n2) * batch, [&](auto CC) {
+        constexpr int C = decltype(CC)::value;
+        constexpr size_t sm = col_smem<L, C>();
+        auto go = [&](auto kernel) {
+            g_optin(kernel, sm);
+            kernel<<<dim3(pl.n2 / C, batch), col_threads<L, C>(), sm, st>>>(d, pl.tw1i);
+        };
+        pl.l2 != L ? go(col_inv_kernel<L, C, 1>) : go(col_inv_kernel<L, C, 0>);
+    });
+    PCGB_POST_LAUNCH();
+}
+
+// Grid of a row pass: V rows of one polynomial per CTA, or (direct plans) V
+// polynomials of the batch.
+template <int L>
+dim3 row_grid(const NttPlan& pl, int batch, int count) {
+    if (pl.direct()) return dim3((batch + row_V<L>() - 1) / row_V<L>(), 1, count);
+    return dim3(pl.n1 / row_V<L>(), batch, count);
+}
+
+template <int L>
+void row_fwd_l(const NttPlan& pl, const FwdIn& in, int count, int batch, bool canonical,
+               cudaStream_t st) {
+    constexpr size_t sm = row_smem<L>();
     auto go = [&](auto kernel) {
         g_optin(kernel, sm);
-        kernel<<<dim3(pl.n2 / col_C(L), batch), col_threads<L>(), sm, st>>>(d, pl.tw1i);
+        kernel<<<row_grid<L>(pl, batch, count), row_threads<L>(), sm, st>>>(in, batch, pl.l1,
+                                                                           pl.tw2, pl.Wf);
     };
-    pl.l2 != L ? go(col_inv_kernel<L, 1>) : go(col_inv_kernel<L, 0>);
-    PCGB_POST_LAUNCH();
-}
-
-template <int L>
-void row_fwd_l(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
-    constexpr size_t sm = row_smem<L>();
-    g_optin(row_fwd_kernel<L>, sm);
-    row_fwd_kernel<L><<<dim3(pl.n1 / row_V<L>(), batch), row_threads<L>(), sm, st>>>(d, pl.l1,
-                                                                                    pl.tw2, pl.Wf);
-    PCGB_POST_LAUNCH();
-}
-
-template <int L>
-void row_pmul_inv_l(const NttPlan& pl, uint64_t* d, const uint64_t* img, int batch,
-                    const ulonglong2* WiRf, cudaStream_t st) {
-    constexpr size_t sm = row_smem<L>();
-    g_optin(row_pmul_inv_kernel<L>, sm);
-    row_pmul_inv_kernel<L><<<dim3(pl.n1 / row_V<L>(), batch), row_threads<L>(), sm, st>>>(
-        d, img, pl.l1, pl.tw2i, WiRf);
-    PCGB_POST_LAUNCH();
-}
-
-template <int L>
-void row_mac_l(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
-               const ulonglong2* Wif, uint64_t* out, cudaStream_t st) {
-    constexpr size_t sm = row_smem<L>();
-    const dim3 grid(pl.n1 / row_V<L>(), batch);
-    if (Q == 1) {
-        g_optin(row_mac_inv_kernel<L, true>, sm);
-        row_mac_inv_kernel<L, true><<<grid, row_threads<L>(), sm, st>>>(g, img, Q, pl.l1, pl.tw2,
-                                                                        pl.tw2i, pl.Wf, Wif, out);
-    } else {
-        g_optin(row_mac_inv_kernel<L, false>, sm);
-        row_mac_inv_kernel<L, false><<<grid, row_threads<L>(), sm, st>>>(g, img, Q, pl.l1, pl.tw2,
-                                                                         pl.tw2i, pl.Wf, Wif, out);
+    if constexpr (L >= 7) {   // rows of 2^13 .. 2^24
+        if (!pl.direct()) {
+            canonical ? go(row_fwd_kernel<L, false, true>) : go(row_fwd_kernel<L, false, false>);
+            PCGB_POST_LAUNCH();
+            return;
+        }
     }
+    canonical ? go(row_fwd_kernel<L, true, true>) : go(row_fwd_kernel<L, true, false>);
     PCGB_POST_LAUNCH();
 }
 
-// Runtime sub-length -> template instance (2^0 .. 2^12).
+template <int L>
+void row_mac_inv_l(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
+                   uint64_t* out, cudaStream_t st) {
+    constexpr size_t sm = row_smem<L>();
+    auto go = [&](auto kernel) {
+        g_optin(kernel, sm);
+        kernel<<<row_grid<L>(pl, batch, 1), row_threads<L>(), sm, st>>>(g, img, Q, batch, pl.l1,
+                                                                       pl.tw2i, pl.Wif, out);
+    };
+    if constexpr (L >= 7) {
+        if (!pl.direct()) {
+            Q == 1 ? go(row_mac_inv_kernel<L, false, true>) : go(row_mac_inv_kernel<L, false, false>);
+            PCGB_POST_LAUNCH();
+            return;
+        }
+    }
+    Q == 1 ? go(row_mac_inv_kernel<L, true, true>) : go(row_mac_inv_kernel<L, true, false>);
+    PCGB_POST_LAUNCH();
+}
+
+template <int L>
+void row_product_l(const NttPlan& pl, uint64_t* c, const uint64_t* a, const uint64_t* b, int batch,
+                   cudaStream_t st) {
+    constexpr size_t sm = row_smem<L>();
+    g_optin(row_product_kernel<L>, sm);
+    row_product_kernel<L><<<row_grid<L>(pl, batch, 1), row_threads<L>(), sm, st>>>(
+        c, a, b, batch, pl.tw2, pl.tw2i, pl.Wif);
+    PCGB_POST_LAUNCH();
+}
+
+// Runtime row length -> template instance (2^1 .. 2^12).
 template <class F>
 void by_len(int L, F&& f) {
     switch (L) {
-        case 0: f(std::integral_constant<int, 0>{}); break;
         case 1: f(std::integral_constant<int, 1>{}); break;
         case 2: f(std::integral_constant<int, 2>{}); break;
         case 3: f(std::integral_constant<int, 3>{}); break;
@@ -939,38 +1049,69 @@ void by_len(int L, F&& f) {
         default: fail(PCGB_EINVAL, "NTT sub-length out of range");
     }
 }
+// Column sub-lengths: 2^6 .. 2^12 (logN 13 .. 24).
+template <class F>
+void by_col_len(int L, F&& f) {
+    switch (L) {
+        case 6: f(std::integral_constant<int, 6>{}); break;
+        case 7: f(std::integral_constant<int, 7>{}); break;
+        case 8: f(std::integral_constant<int, 8>{}); break;
+        case 9: f(std::integral_constant<int, 9>{}); break;
+        case 10: f(std::integral_constant<int, 10>{}); break;
+        case 11: f(std::integral_constant<int, 11>{}); break;
+        case 12: f(std::integral_constant<int, 12>{}); break;
+        default: fail(PCGB_EINVAL, "NTT sub-length out of range");
+    }
+}
 
-void col_fwd(const NttPlan& pl, const uint64_t* src, uint64_t* dst, int batch, bool reduce,
-             cudaStream_t st) {
-    by_len(pl.l1, [&](auto L) { col_fwd_l<decltype(L)::value>(pl, src, dst, batch, reduce, st); });
+void col_fwd(const NttPlan& pl, const FwdIn& in, int count, int batch, cudaStream_t st) {
+    by_col_len(pl.l1, [&](auto L) { col_fwd_l<decltype(L)::value>(pl, in, count, batch, st); });
 }
 void col_inv(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
-    by_len(pl.l1, [&](auto L) { col_inv_l<decltype(L)::value>(pl, d, batch, st); });
+    by_col_len(pl.l1, [&](auto L) { col_inv_l<decltype(L)::value>(pl, d, batch, st); });
 }
-void row_fwd(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
-    by_len(pl.l2, [&](auto L) { row_fwd_l<decltype(L)::value>(pl, d, batch, st); });
-}
-void row_pmul_inv(const NttPlan& pl, uint64_t* d, const uint64_t* img, int batch,
-                  const ulonglong2* WiRf, cudaStream_t st) {
+void row_fwd(const NttPlan& pl, const FwdIn& in, int count, int batch, bool canonical,
+             cudaStream_t st) {
     by_len(pl.l2,
-           [&](auto L) { row_pmul_inv_l<decltype(L)::value>(pl, d, img, batch, WiRf, st); });
+           [&](auto L) { row_fwd_l<decltype(L)::value>(pl, in, count, batch, canonical, st); });
 }
-void row_mac(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
-             const ulonglong2* Wif, uint64_t* out, cudaStream_t st) {
+void row_mac_inv(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
+                 uint64_t* out, cudaStream_t st) {
     by_len(pl.l2,
-           [&](auto L) { row_mac_l<decltype(L)::value>(pl, g, img, Q, batch, Wif, out, st); });
+           [&](auto L) { row_mac_inv_l<decltype(L)::value>(pl, g, img, Q, batch, out, st); });
 }
 
-const ulonglong2* wi_times_r(NttPlan& pl, cudaStream_t st) {
-    std::lock_guard<std::mutex> lk(pl.mu);
-    if (!pl.WiRf) {
-        PCGB_CK(cudaMalloc(&pl.WiRf, sizeof(ulonglong2) * pl.N));
-        scale_r_kernel<<<static_cast<unsigned>((pl.N + 255) / 256), 256, 0, st>>>(
-            pl.WiRf, pl.Wif, pl.N, r2_mod_p());
-        PCGB_POST_LAUNCH();
-        PCGB_CK(cudaStreamSynchronize(st));
+// Forward transforms of `count` batches, any 64-bit inputs: the column pass
+// from src (plus add) to dst and the row pass in place, or the single row
+// pass of a direct plan.
+void forward(const NttPlan& pl, const FwdIn& in, int count, int batch, bool canonical,
+             cudaStream_t st) {
+    if (pl.direct()) {
+        row_fwd(pl, in, count, batch, canonical, st);
+        return;
     }
-    return pl.WiRf;
+    col_fwd(pl, in, count, batch, st);
+    FwdIn rows;
+    for (int z = 0; z < count; ++z) rows.src[z] = rows.dst[z] = in.dst[z];
+    row_fwd(pl, rows, count, batch, canonical, st);
+}
+
+FwdIn fwd_one(const uint64_t* src, uint64_t* dst) {
+    FwdIn in;
+    in.src[0] = src;
+    in.dst[0] = dst;
+    return in;
+}
+FwdIn fwd_two(const uint64_t* s0, uint64_t* d0, const uint64_t* s1, uint64_t* d1) {
+    FwdIn in;
+    in.src[0] = s0; in.dst[0] = d0;
+    in.src[1] = s1; in.dst[1] = d1;
+    return in;
+}
+
+bool overlap(const uint64_t* a, size_t na, const uint64_t* b, size_t nb) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb * sizeof(uint64_t) && y < x + na * sizeof(uint64_t);
 }
 
 }  // namespace
@@ -987,10 +1128,15 @@ const NttPlan& ntt_plan(int logN) {
     return *slot;
 }
 
-void ntt_forward_from(const NttPlan& pl, const uint64_t* src, uint64_t* dst, int batch,
-                      bool reduce, cudaStream_t st) {
-    col_fwd(pl, src, dst, batch, reduce, st);
-    row_fwd(pl, dst, batch, st);
+void ntt_forward3(const NttPlan& pl, const uint64_t* const (&src)[3],
+                  const uint64_t* const (&add)[3], uint64_t* const (&dst)[3], cudaStream_t st) {
+    FwdIn in;
+    for (int z = 0; z < 3; ++z) {
+        in.src[z] = src[z];
+        in.add[z] = add[z];
+        in.dst[z] = dst[z];
+    }
+    forward(pl, in, 3, 1, true, st);
 }
 
 void ntt_log_sizes(const NttPlan& pl, int* l1, int* l2) {
@@ -999,8 +1145,7 @@ void ntt_log_sizes(const NttPlan& pl, int* l1, int* l2) {
 }
 
 void ntt_forward(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
-    col_fwd(pl, d, d, batch, false, st);
-    row_fwd(pl, d, batch, st);
+    forward(pl, fwd_one(d, d), 1, batch, true, st);
 }
 
 // Per device: a second stream and two events for the two-half schedule of
@@ -1018,53 +1163,55 @@ HalfFork& half_fork() {
     return f[dev];
 }
 
+bool poly_mul_needs_scratch(const NttPlan& pl) { return !pl.direct(); }
+
 void poly_mul_device(const NttPlan& pl, uint64_t* c, const uint64_t* a, const uint64_t* b,
                      int batch, uint64_t* scratch, cudaStream_t st) {
-    const ulonglong2* wir = wi_times_r(const_cast<NttPlan&>(pl), st);
-    // A = NTT(a) in scratch; c = NTT(b); c = INTT(c (.) A): the forward row
-    // pass of c and the pointwise product + inverse row pass are separate
-    // launches (each needs about 70 registers a thread where the fused
-    // pass needs 96, so more CTAs fit on an SM).
-    // a is read before c is first written, so c may alias a or b.
-    // A batch of two or more runs as two halves on two streams, pass by
-    // pass: each pass kernel alone leaves the IMAD pipe a third idle (its
-    // barriers and its tail), and the other half's CTAs fill those slots
-    // (16 x 2^20: 0.882 -> 0.843 ms; four quarters gave 0.839).  Each half
-    // reads and writes only its own products, so aliasing holds per half.
-    if (batch >= 2) {
-        HalfFork& f = half_fork();
-        std::lock_guard<std::mutex> lk(f.mu);
-        if (!f.side) {
-            PCGB_CK(cudaEventCreateWithFlags(&f.fork, cudaEventDisableTiming));
-            PCGB_CK(cudaEventCreateWithFlags(&f.join, cudaEventDisableTiming));
-            PCGB_CK(cudaStreamCreateWithFlags(&f.side, cudaStreamNonBlocking));
-        }
-        const int h0 = batch / 2, h1 = batch - h0;
-        const size_t o = static_cast<size_t>(h0) * pl.N;
-        PCGB_CK(cudaEventRecord(f.fork, st));
-        PCGB_CK(cudaStreamWaitEvent(f.side, f.fork, 0));
-        col_fwd(pl, a, scratch, h0, true, st);
-        col_fwd(pl, a + o, scratch + o, h1, true, f.side);
-        row_fwd(pl, scratch, h0, st);
-        row_fwd(pl, scratch + o, h1, f.side);
-        col_fwd(pl, b, c, h0, true, st);
-        col_fwd(pl, b + o, c + o, h1, true, f.side);
-        row_fwd(pl, c, h0, st);
-        row_fwd(pl, c + o, h1, f.side);
-        row_pmul_inv(pl, c, scratch, h0, wir, st);
-        row_pmul_inv(pl, c + o, scratch + o, h1, wir, f.side);
-        col_inv(pl, c, h0, st);
-        col_inv(pl, c + o, h1, f.side);
-        PCGB_CK(cudaEventRecord(f.join, f.side));
-        PCGB_CK(cudaStreamWaitEvent(st, f.join, 0));
+    if (pl.direct()) {
+        by_len(pl.l2,
+               [&](auto L) { row_product_l<decltype(L)::value>(pl, c, a, b, batch, st); });
         return;
     }
-    col_fwd(pl, a, scratch, batch, true, st);
-    row_fwd(pl, scratch, batch, st);
-    col_fwd(pl, b, c, batch, true, st);
-    row_fwd(pl, c, batch, st);
-    row_pmul_inv(pl, c, scratch, batch, wir, st);
-    col_inv(pl, c, batch, st);
+    // A = NTT(a) in scratch and c = NTT(b) as one launch per pass, then
+    // c = INTT(c (.) A).  When c overlaps a, the column pass of a runs first.
+    auto product = [&](size_t first, int count, cudaStream_t s) {
+        uint64_t *A = scratch + first, *C = c + first;
+        const uint64_t *x = a + first, *y = b + first;
+        const size_t n = static_cast<size_t>(count) * pl.N;
+        if (overlap(C, n, x, n)) {
+            col_fwd(pl, fwd_one(x, A), 1, count, s);
+            col_fwd(pl, fwd_one(y, C), 1, count, s);
+        } else {
+            col_fwd(pl, fwd_two(x, A, y, C), 2, count, s);
+        }
+        row_fwd(pl, fwd_two(A, A, C, C), 2, count, false, s);
+        row_mac_inv(pl, C, A, 1, count, C, s);
+        col_inv(pl, C, count, s);
+    };
+    // A batch of 2^18 words or more runs as two halves on two streams: each
+    // pass alone leaves the multiplier pipe a third idle (barriers, loads,
+    // its tail), and the other half's CTAs fill those slots (16 x 2^20: 829
+    // -> 801 us, 2 x 2^18: 49.7 -> 42.9; at 4 x 2^16 no difference, below it
+    // the fork costs 1 us).  Each half reads and writes only its own
+    // products, so aliasing holds per half.
+    if (batch < 2 || static_cast<size_t>(batch) * pl.N < (size_t{1} << 18)) {
+        product(0, batch, st);
+        return;
+    }
+    HalfFork& f = half_fork();
+    std::lock_guard<std::mutex> lk(f.mu);
+    if (!f.side) {
+        PCGB_CK(cudaEventCreateWithFlags(&f.fork, cudaEventDisableTiming));
+        PCGB_CK(cudaEventCreateWithFlags(&f.join, cudaEventDisableTiming));
+        PCGB_CK(cudaStreamCreateWithFlags(&f.side, cudaStreamNonBlocking));
+    }
+    const int h0 = batch / 2;
+    PCGB_CK(cudaEventRecord(f.fork, st));
+    PCGB_CK(cudaStreamWaitEvent(f.side, f.fork, 0));
+    product(static_cast<size_t>(h0) * pl.N, batch - h0, f.side);
+    product(0, h0, st);
+    PCGB_CK(cudaEventRecord(f.join, f.side));
+    PCGB_CK(cudaStreamWaitEvent(st, f.join, 0));
 }
 
 bool poly_mul_mixed_ok(int logN) { return logN >= 2 * kMixedLmin && logN <= 2 * kMixedLmax; }
@@ -1079,6 +1226,25 @@ void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const*
         order[i] = i;
         scratch_words += size_t{1} << logN[i];
     }
+    // Both operands' column passes share a launch unless some output
+    // overlaps a first operand (which must then be read before).
+    bool alias = false;
+    {
+        std::vector<std::pair<uintptr_t, uintptr_t>> ra(count), rc(count);
+        for (int i = 0; i < count; ++i) {
+            const uintptr_t len = sizeof(uint64_t) << logN[i];
+            ra[i] = {reinterpret_cast<uintptr_t>(a[i]), reinterpret_cast<uintptr_t>(a[i]) + len};
+            rc[i] = {reinterpret_cast<uintptr_t>(c[i]), reinterpret_cast<uintptr_t>(c[i]) + len};
+        }
+        std::sort(ra.begin(), ra.end());
+        // Furthest end of the operands that start at or before each one.
+        std::vector<uintptr_t> end(count);
+        for (int i = 0; i < count; ++i) end[i] = i ? std::max(end[i - 1], ra[i].second) : ra[i].second;
+        for (const auto& r : rc) {
+            const auto it = std::lower_bound(ra.begin(), ra.end(), std::make_pair(r.second, uintptr_t{0}));
+            if (it != ra.begin() && end[it - ra.begin() - 1] > r.first) alias = true;
+        }
+    }
     // Longest products first, so the last CTAs of each pass are short ones.
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return logN[x] > logN[y]; });
     std::vector<MixedPoly> polys(count);
@@ -1087,11 +1253,11 @@ void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const*
     size_t off = 0;
     for (int k = 0; k < count; ++k) {
         const int i = order[k];
-        NttPlan& pl = const_cast<NttPlan&>(ntt_plan(logN[i]));
+        const NttPlan& pl = ntt_plan(logN[i]);
         MixedPoly& m = polys[k];
         m.a = a[i]; m.b = b[i]; m.c = c[i]; m.A = scratch + off;
         m.tw1 = pl.tw1; m.tw1i = pl.tw1i; m.tw2 = pl.tw2; m.tw2i = pl.tw2i;
-        m.Wf = pl.Wf; m.WiRf = wi_times_r(pl, st);
+        m.Wf = pl.Wf; m.Wif = pl.Wif;
         m.l1 = pl.l1; m.l2 = pl.l2;
         off += pl.N;
         int C = 0, V = 0;
@@ -1121,14 +1287,15 @@ void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const*
     g_optin(mixed_col_fwd_kernel, kMixedColSmem);
     g_optin(mixed_col_inv_kernel, kMixedColSmem);
     g_optin(mixed_row_fwd_kernel, kMixedRowSmem);
-    g_optin(mixed_row_mac_kernel, kMixedRowSmem);
-    mixed_col_fwd_kernel<<<n_col, kMixedColThreads, kMixedColSmem, st>>>(d_polys, d_col, 0);
+    g_optin(mixed_row_mul_kernel, kMixedRowSmem);
+    for (int first = 0; first < (alias ? 2 : 1); ++first) {
+        mixed_col_fwd_kernel<<<dim3(n_col, alias ? 1 : 2), kMixedColThreads, kMixedColSmem, st>>>(
+            d_polys, d_col, first);
+        PCGB_POST_LAUNCH();
+    }
+    mixed_row_fwd_kernel<<<dim3(n_row, 2), kMixedRowThreads, kMixedRowSmem, st>>>(d_polys, d_row);
     PCGB_POST_LAUNCH();
-    mixed_row_fwd_kernel<<<n_row, kMixedRowThreads, kMixedRowSmem, st>>>(d_polys, d_row);
-    PCGB_POST_LAUNCH();
-    mixed_col_fwd_kernel<<<n_col, kMixedColThreads, kMixedColSmem, st>>>(d_polys, d_col, 1);
-    PCGB_POST_LAUNCH();
-    mixed_row_mac_kernel<<<n_row, kMixedRowThreads, kMixedRowSmem, st>>>(d_polys, d_row);
+    mixed_row_mul_kernel<<<n_row, kMixedRowThreads, kMixedRowSmem, st>>>(d_polys, d_row);
     PCGB_POST_LAUNCH();
     mixed_col_inv_kernel<<<n_col, kMixedColThreads, kMixedColSmem, st>>>(d_polys, d_col);
     PCGB_POST_LAUNCH();
@@ -1138,9 +1305,9 @@ void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const*
 
 void ntt_mac_inverse(const NttPlan& pl, uint64_t* g, const uint64_t* img, int Q, uint64_t* acc,
                      cudaStream_t st) {
-    col_fwd(pl, g, g, Q, false, st);
-    row_mac(pl, g, img, Q, 1, pl.Wif, acc, st);
-    col_inv(pl, acc, 1, st);
+    forward(pl, fwd_one(g, g), 1, Q, false, st);
+    row_mac_inv(pl, g, img, Q, 1, acc, st);
+    if (!pl.direct()) col_inv(pl, acc, 1, st);
 }
 
 bool ntt_mac_multi_ok(int logN) { return logN >= 2 * kMacLmin && logN <= 2 * kMixedLmax; }
@@ -1159,7 +1326,7 @@ void ntt_mac_inverse_multi(int count, uint64_t* const* g, const uint64_t* const*
         return (static_cast<uint64_t>(Q[x]) << logN[x]) > (static_cast<uint64_t>(Q[y]) << logN[y]);
     });
     std::vector<MacReq> reqs(count);
-    std::vector<MacCta> colf, row, coli;
+    std::vector<MacCta> colf, rowf, row, coli;
     for (int k = 0; k < count; ++k) {
         const int i = order[k];
         const NttPlan& pl = ntt_plan(logN[i]);
@@ -1178,44 +1345,43 @@ void ntt_mac_inverse_multi(int count, uint64_t* const* g, const uint64_t* const*
                 V = mixed_V<decltype(L)::value>();
         });
         const uint32_t kk = static_cast<uint32_t>(k);
-        for (uint32_t q = 0; q < static_cast<uint32_t>(m.Q); ++q)
-            for (uint32_t tl = 0; tl < static_cast<uint32_t>(pl.n2 / C); ++tl) colf.push_back({kk, q, tl});
-        for (uint32_t tl = 0; tl < static_cast<uint32_t>(pl.n1 / V); ++tl) row.push_back({kk, 0, tl});
-        for (uint32_t tl = 0; tl < static_cast<uint32_t>(pl.n2 / C); ++tl) coli.push_back({kk, 0, tl});
+        const uint32_t nc = static_cast<uint32_t>(pl.n2 / C), nr = static_cast<uint32_t>(pl.n1 / V);
+        for (uint32_t q = 0; q < static_cast<uint32_t>(m.Q); ++q) {
+            for (uint32_t tl = 0; tl < nc; ++tl) colf.push_back({kk, q, tl});
+            for (uint32_t tl = 0; tl < nr; ++tl) rowf.push_back({kk, q, tl});
+        }
+        for (uint32_t tl = 0; tl < nr; ++tl) row.push_back({kk, 0, tl});
+        for (uint32_t tl = 0; tl < nc; ++tl) coli.push_back({kk, 0, tl});
     }
-    const size_t b_req = sizeof(MacReq) * reqs.size();
-    const size_t o_colf = (b_req + 255) & ~size_t{255};
-    const size_t o_row = (o_colf + sizeof(MacCta) * colf.size() + 255) & ~size_t{255};
-    const size_t o_coli = (o_row + sizeof(MacCta) * row.size() + 255) & ~size_t{255};
-    const size_t total = o_coli + sizeof(MacCta) * coli.size();
+    // All tables in one copy: the requests, then the four CTA lists.
+    const std::vector<MacCta>* lists[4] = {&colf, &rowf, &row, &coli};
+    size_t o[4], total = sizeof(MacReq) * reqs.size();
+    for (int i = 0; i < 4; ++i) {
+        o[i] = (total + 255) & ~size_t{255};
+        total = o[i] + sizeof(MacCta) * lists[i]->size();
+    }
     std::vector<char> host(total);
-    std::memcpy(host.data(), reqs.data(), b_req);
-    std::memcpy(host.data() + o_colf, colf.data(), sizeof(MacCta) * colf.size());
-    std::memcpy(host.data() + o_row, row.data(), sizeof(MacCta) * row.size());
-    std::memcpy(host.data() + o_coli, coli.data(), sizeof(MacCta) * coli.size());
+    std::memcpy(host.data(), reqs.data(), sizeof(MacReq) * reqs.size());
+    for (int i = 0; i < 4; ++i)
+        std::memcpy(host.data() + o[i], lists[i]->data(), sizeof(MacCta) * lists[i]->size());
     char* tab = static_cast<char*>(pool_alloc(total, st));
     PCGB_CK(cudaMemcpyAsync(tab, host.data(), total, cudaMemcpyHostToDevice, st));
     const MacReq* d_req = reinterpret_cast<const MacReq*>(tab);
+    auto ctas = [&](int i) { return reinterpret_cast<const MacCta*>(tab + o[i]); };
+    auto grid = [&](int i) { return static_cast<unsigned>(lists[i]->size()); };
     g_optin(mac_col_fwd_kernel, kMixedColSmem);
-    g_optin(mac_row_kernel, kMixedRowSmem);
+    g_optin(mac_row_fwd_kernel, kMixedRowSmem);
+    g_optin(mac_row_inv_kernel, kMixedRowSmem);
     g_optin(mac_col_inv_kernel, kMixedColSmem);
-    mac_col_fwd_kernel<<<static_cast<unsigned>(colf.size()), kMixedColThreads, kMixedColSmem, st>>>(
-        d_req, reinterpret_cast<const MacCta*>(tab + o_colf));
+    mac_col_fwd_kernel<<<grid(0), kMixedColThreads, kMixedColSmem, st>>>(d_req, ctas(0));
     PCGB_POST_LAUNCH();
-    mac_row_kernel<<<static_cast<unsigned>(row.size()), kMixedRowThreads, kMixedRowSmem, st>>>(
-        d_req, reinterpret_cast<const MacCta*>(tab + o_row));
+    mac_row_fwd_kernel<<<grid(1), kMixedRowThreads, kMixedRowSmem, st>>>(d_req, ctas(1));
     PCGB_POST_LAUNCH();
-    mac_col_inv_kernel<<<static_cast<unsigned>(coli.size()), kMixedColThreads, kMixedColSmem, st>>>(
-        d_req, reinterpret_cast<const MacCta*>(tab + o_coli));
+    mac_row_inv_kernel<<<grid(2), kMixedRowThreads, kMixedRowSmem, st>>>(d_req, ctas(2));
+    PCGB_POST_LAUNCH();
+    mac_col_inv_kernel<<<grid(3), kMixedColThreads, kMixedColSmem, st>>>(d_req, ctas(3));
     PCGB_POST_LAUNCH();
     PCGB_CK(cudaFreeAsync(tab, st));
-}
-
-void pointwise_mul(uint64_t* c, const uint64_t* a, const uint64_t* b, size_t count, int mode,
-                   cudaStream_t st) {
-    pointwise_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, st>>>(c, a, b, count,
-                                                                               mode, r2_mod_p());
-    PCGB_POST_LAUNCH();
 }
 
 void reduce_mod_p(uint64_t* d, const uint64_t* s, size_t count, cudaStream_t st) {

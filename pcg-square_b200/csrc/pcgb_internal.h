@@ -279,37 +279,35 @@ void aes_tree_round_keys_host(const uint8_t master[16], int nk, uint8_t* rks);
 // ---- NTT (ntt.cu) --------------------------------------------------------
 struct NttPlan;
 const NttPlan& ntt_plan(int logN);   // resident per (device, logN)
-// In-place forward transform of `batch` length-N polys into the internal
-// evaluation layout (coefficients must be < p).
+// In-place forward transform of `batch` length-N polys of any 64-bit words
+// into the internal evaluation layout, values in [0, p).
 void ntt_forward(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st);
-// dst = forward transform of src (batch polys, contiguous); reduce maps any
-// uint64 input into [0, p) first, else inputs must be below 4p.
-void ntt_forward_from(const NttPlan& pl, const uint64_t* src, uint64_t* dst, int batch,
-                      bool reduce, cudaStream_t st);
+// Three forward transforms in one launch per pass: dst[z] = NTT(src[z] +
+// add[z]), add[z] null for none; inputs any uint64, outputs in [0, p).
+void ntt_forward3(const NttPlan& pl, const uint64_t* const (&src)[3],
+                  const uint64_t* const (&add)[3], uint64_t* const (&dst)[3], cudaStream_t st);
 void ntt_log_sizes(const NttPlan& pl, int* l1, int* l2);   // see ntt_layout.cuh
 // c = a * b mod (X^N+1) for `batch` polys; c may alias a or b; inputs any
-// uint64 (reduced mod p first).  scratch: batch*N words.
+// uint64 (reduced mod p first).  scratch: batch*N words when
+// poly_mul_needs_scratch, else unused.
+bool poly_mul_needs_scratch(const NttPlan& pl);
 void poly_mul_device(const NttPlan& pl, uint64_t* c, const uint64_t* a, const uint64_t* b,
                      int batch, uint64_t* scratch, cudaStream_t st);
 // c[i] = a[i] * b[i] mod (X^N_i + 1) for polynomials of different lengths
-// N_i = 2^logN[i] in 2^16 .. 2^20, five launches for the whole batch; c[i]
-// may alias a[i] or b[i]; inputs any uint64.
+// N_i = 2^logN[i] in 2^16 .. 2^20, four launches for the whole batch (five
+// when some c overlaps some a); c[i] may alias a[i] or b[i]; inputs any uint64.
 bool poly_mul_mixed_ok(int logN);
 void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const* a,
                            const uint64_t* const* b, const int* logN, cudaStream_t st);
 // acc = INTT( sum_q img[q] (.) NTT(g[q]) ); g is consumed (transformed in
-// place); img in Montgomery-scaled evaluation layout.
+// place); img in the evaluation layout, values in [0, p).
 void ntt_mac_inverse(const NttPlan& pl, uint64_t* g, const uint64_t* img, int Q, uint64_t* acc,
                      cudaStream_t st);
 // The same for `count` requests of different lengths N_i = 2^logN[i] in
-// 2^14 .. 2^20 (Q[i] buffers each), three launches for all of them.
+// 2^14 .. 2^20 (Q[i] buffers each), four launches for all of them.
 bool ntt_mac_multi_ok(int logN);
 void ntt_mac_inverse_multi(int count, uint64_t* const* g, const uint64_t* const* img, const int* Q,
                            uint64_t* const* z, const int* logN, cudaStream_t st);
-// Pointwise c[i] = a[i]*b[i]*R mod p over `count` words (R = 2^64): turns
-// an evaluation vector into its Montgomery-scaled form when b = R^2 scaled.
-void pointwise_mul(uint64_t* c, const uint64_t* a, const uint64_t* b, size_t count, int mode,
-                   cudaStream_t st);
 void reduce_mod_p(uint64_t* d, const uint64_t* s, size_t count, cudaStream_t st);
 
 // ---- triples and relation checks (triples.cu) ----------------------------

@@ -107,11 +107,8 @@ void triples_device(int N, int party, const uint64_t* x1, const uint64_t* z1, co
     ntt_log_sizes(pl, &l1, &l2);
     const size_t n = static_cast<size_t>(N);
     uint64_t* T = static_cast<uint64_t*>(pool_alloc(3 * n * sizeof(uint64_t), st));  // A | B | S
-    add_reduce_kernel<<<grid_for(n), kTpb, 0, st>>>(T + 2 * n, z1, z2, n);
-    PCGB_POST_LAUNCH();
-    ntt_forward_from(pl, party == 0 ? x1 : x2, T, 1, true, st);
-    ntt_forward_from(pl, party == 0 ? x2 : x1, T + n, 1, true, st);
-    ntt_forward_from(pl, T + 2 * n, T + 2 * n, 1, false, st);
+    ntt_forward3(pl, {party == 0 ? x1 : x2, party == 0 ? x2 : x1, z1}, {nullptr, nullptr, z2},
+                 {T, T + n, T + 2 * n}, st);
     triple_slots_kernel<<<grid_for(n), kTpb, 0, st>>>(T, T + n, T + 2 * n, n, l1, l2, r2_mod_p(),
                                                       a, b, c);
     PCGB_POST_LAUNCH();
@@ -125,11 +122,7 @@ void verify_ole_device(int N, const uint64_t* x0, const uint64_t* z0, const uint
     const size_t n = static_cast<size_t>(N);
     uint64_t* T = static_cast<uint64_t*>(pool_alloc(3 * n * sizeof(uint64_t), st));  // X0 | X1 | Z
     PCGB_CK(cudaMemsetAsync(bad, 0, sizeof(unsigned long long), st));
-    add_reduce_kernel<<<grid_for(n), kTpb, 0, st>>>(T + 2 * n, z0, z1, n);
-    PCGB_POST_LAUNCH();
-    ntt_forward_from(pl, x0, T, 1, true, st);
-    ntt_forward_from(pl, x1, T + n, 1, true, st);
-    ntt_forward_from(pl, T + 2 * n, T + 2 * n, 1, false, st);
+    ntt_forward3(pl, {x0, x1, z0}, {nullptr, nullptr, z1}, {T, T + n, T + 2 * n}, st);
     ole_check_kernel<<<check_grid(n), kTpb, 0, st>>>(T, T + n, T + 2 * n, n, r2_mod_p(), bad);
     PCGB_POST_LAUNCH();
     PCGB_CK(cudaFreeAsync(T, st));

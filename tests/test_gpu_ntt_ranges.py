@@ -1,0 +1,52 @@
+"""Products at the ends of the lazy value ranges: every length around the
+one-row / four-step border and the two-stream schedule, inputs of the largest
+and smallest residues and of unreduced words, outputs aliasing operands."""
+import numpy as np
+import pytest
+
+import oracle_lib as O
+from gpu_helpers import dev
+
+pytestmark = pytest.mark.gpu
+P = O.P
+
+
+def operand(kind, n, seed):
+    if kind == "top":
+        return np.full(n, P - 1, np.uint64)
+    if kind == "wrap":                       # unreduced: 2^64 - 1 - small
+        return np.uint64(2**64 - 1) - np.arange(n, dtype=np.uint64) % np.uint64(7)
+    if kind == "step":                       # 0 and p - 1 in blocks, half-p edges
+        v = np.where(np.arange(n) & 8, P - 1, 0).astype(np.uint64)
+        v[::5] = P // 2
+        v[::7] = P // 2 + 1
+        return v
+    return np.random.default_rng(seed).integers(0, 2**64 - 1, n, dtype=np.uint64)
+
+
+@pytest.mark.parametrize("lg,batch", [(1, 5), (2, 3), (3, 3), (4, 9), (5, 17), (6, 65), (8, 7),
+                                      (11, 3), (12, 3), (13, 1), (13, 33), (14, 3), (15, 2),
+                                      (17, 2)])
+@pytest.mark.parametrize("lhs,rhs", [("top", "top"), ("wrap", "step"), ("step", "any"),
+                                     ("any", "wrap")])
+def test_product_ranges(pcg, lg, batch, lhs, rhs):
+    n = batch << lg
+    a, b = operand(lhs, n, 1000 + lg), operand(rhs, n, 2000 + lg)
+    want = O.poly_mul(a, b, 1 << lg)
+    d_a, d_b, d_c = dev(pcg, a), dev(pcg, b), dev(pcg, np.zeros(n, np.uint64))
+    pcg.poly_mul_device(d_c.ptr, d_a.ptr, d_b.ptr, batch, 1 << lg)
+    assert (d_c.download(np.uint64, n) == want).all()
+    pcg.poly_mul_device(d_a.ptr, d_a.ptr, d_b.ptr, batch, 1 << lg)      # c = a
+    assert (d_a.download(np.uint64, n) == want).all()
+    d_a = dev(pcg, a)
+    pcg.poly_mul_device(d_b.ptr, d_a.ptr, d_b.ptr, batch, 1 << lg)      # c = b
+    assert (d_b.download(np.uint64, n) == want).all()
+
+
+def test_square_in_place(pcg):
+    """a, b and c the same buffer, in both plan forms."""
+    for lg in (7, 13):
+        a = operand("any", 1 << lg, lg)
+        d = dev(pcg, a)
+        pcg.poly_mul_device(d.ptr, d.ptr, d.ptr, 1, 1 << lg)
+        assert (d.download(np.uint64, 1 << lg) == O.poly_mul(a, a, 1 << lg)).all()
