@@ -1,5 +1,5 @@
 // Negacyclic NTT over F_p for N = 2^logN (1 <= logN <= 24): one row up to
-// 2^12 (N = n2, n1 = 1, a single CTA per transform), four-step above.
+// 2^9 (N = n2, n1 = 1, a single CTA per transform), four-step above.
 //
 // N = n1 * n2 with n1 = 2^floor(logN/2), n2 = 2^ceil(logN/2); coefficient j
 // sits at row j / n2, column j % n2.  With psi a primitive 2N-th root:
@@ -81,6 +81,11 @@ struct NttPlan {
     // (inverse) root folded into the upper half of each row
     NttTw* Wf = nullptr;     // forward twiddle
     NttTw* Wif = nullptr;    // inverse twiddle * N^-1
+    // The same three tables of the one-row form (tw2, tw2i, Wif themselves when
+    // l1 = 0), up to kOneRowLogN: whole products in one launch
+    NttTw* one_tw = nullptr;
+    NttTw* one_twi = nullptr;
+    NttTw* one_Wi = nullptr;
     bool direct() const { return l1 == 0; }   // one row: no column passes
 };
 
@@ -281,7 +286,7 @@ __host__ __device__ constexpr int col_C(int L) {
     return L <= 3 ? (1 << L) : (L <= 9 ? 16 : (L == 10 ? 8 : (L == 11 ? 4 : 2)));
 }
 __host__ __device__ constexpr int col_C_min(int L) {
-    return L >= 6 && L <= 10 ? 4 : col_C(L);
+    return L >= 5 && L <= 10 ? 4 : col_C(L);
 }
 template <int L, int C>
 __host__ __device__ constexpr int col_threads() { return Geo<L>::T * C; }
@@ -371,13 +376,16 @@ __device__ __forceinline__ void col_inv_body(uint64_t* d, size_t tile,
 
 // Row pass, forward, of one row (thread t of its T): the four-step twiddle
 // with the row transform's first root folded in (Wf, the row's first entry),
-// then the row transform; outputs in the permuted order, in [0, p) (CANON) or
-// within 1.6p.  src may equal dst (a row's threads load it
+// then the row transform; outputs in the permuted order: in [0, p) (kRowCanon),
+// within 1.6p (kRowLazy), or times img (kRowTimes: any residues within 1.7p, at
+// the same positions), in [-0.17p, 1.17p].  src may equal dst (a row's threads load it
 // before the first barrier or read and write the same positions).  DIRECT:
 // the row is a whole polynomial of any 64-bit words (n1 = 1), untwisted.
-template <int L, bool DIRECT, bool CANON>
+enum RowOut { kRowLazy, kRowCanon, kRowTimes };
+template <int L, bool DIRECT, RowOut OUT>
 __device__ __forceinline__ void row_fwd_body(const uint64_t* src, const uint64_t* add,
-                                             uint64_t* dst, int t, bool valid,
+                                             const uint64_t* __restrict__ img, uint64_t* dst,
+                                             int t, bool valid,
                                              const NttTw* __restrict__ tw,
                                              const NttTw* __restrict__ Wf, int64_t* sm) {
     constexpr int E = Geo<L>::E, LP = last_phase(L);
@@ -391,53 +399,48 @@ __device__ __forceinline__ void row_fwd_body(const uint64_t* src, const uint64_t
     forward_all<L, !DIRECT, true>(x, t, tw, SmemLay<1>{sm});
     if (!valid) return;
 #pragma unroll
-    for (int e = 0; e < E; ++e)
-        dst[perm_pos<L>(eidx<L, LP>(t, e))] =
-            CANON ? canon(fold(x[e])) : static_cast<uint64_t>(x[e]);
+    for (int e = 0; e < E; ++e) {
+        const int i = perm_pos<L>(eidx<L, LP>(t, e));
+        if constexpr (OUT == kRowCanon) dst[i] = canon(fold(x[e]));
+        else if constexpr (OUT == kRowTimes)
+            dst[i] = static_cast<uint64_t>(mul_var(x[e], static_cast<int64_t>(__ldg(img + i))));
+        else dst[i] = static_cast<uint64_t>(x[e]);
+    }
 }
 
-// Multiply-accumulate and inverse row pass of one row:
-//   out row = Wi (.) INTT( sum_q g_q row (.) img_q row ),
-// g_q = g + q*N, img_q = img + q*N transforms in the permuted evaluation
-// order (row_fwd_body's output, lazy or canonical); Wif is the inverse
-// twiddle with the inverse row transform's last root folded in.  Each thread
-// loads the permuted positions of its last-phase registers, so the inverse
-// starts where the forward ended.  out is in [-e p, (1 + e)p], or in [0, p)
-// (CANON), and may alias g (a row's threads read all of it before the first
-// store).  The forward transforms ran as a launch of their own: kept in this
-// kernel, Q of them in a row left the chip idle (16 % warps active, 151 us
-// of 262 at N = 2^20, Q = 10; 81 us at N = 2^16, Q = 6).
-template <int L, bool ONE, bool CANON>
-__device__ __forceinline__ void row_mac_inv_body(const uint64_t* g, const uint64_t* img, int Q,
-                                                 size_t N, int t, bool valid,
-                                                 const NttTw* __restrict__ twi,
-                                                 const NttTw* __restrict__ Wif, uint64_t* out,
-                                                 int64_t* sm) {
-    constexpr int E = Geo<L>::E, T = Geo<L>::T, LP = last_phase(L);
+// Inverse row pass of one row, out row = Wi (.) INTT(y row), with
+//   y = g (.) img         (SUM false: two transforms within 1.7p), or
+//   y = sum_{q < Q} g_q   (SUM: g_q = g + q*N, products of kRowTimes),
+// in the permuted evaluation order; Wif is the inverse twiddle with the
+// inverse row transform's last root folded in.  Each thread loads the
+// permuted positions of its last-phase registers, so the inverse starts where
+// the forward ended.  out is in [-e p, (1 + e)p], or in [0, p) (CANON), and may
+// alias g (a row's threads read all of it before the first store).
+template <int L, bool SUM, bool CANON>
+__device__ __forceinline__ void row_inv_body(const uint64_t* g, const uint64_t* img, int Q,
+                                             size_t N, int t, bool valid,
+                                             const NttTw* __restrict__ twi,
+                                             const NttTw* __restrict__ Wif, uint64_t* out,
+                                             int64_t* sm) {
+    constexpr int E = Geo<L>::E, LP = last_phase(L);
     int64_t x[E];
-    if (valid) {
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int i = perm_pos<L>(eidx<L, LP>(t, e));
-            x[e] = mul_var(static_cast<int64_t>(g[i]), static_cast<int64_t>(img[i]));
-        }
-        if constexpr (!ONE) {
-            for (int q = 1; q < Q; ++q) {
-                g += N;
-                img += N;
+    for (int e = 0; e < E; ++e) {
+        const int i = perm_pos<L>(eidx<L, LP>(t, e));
+        x[e] = valid ? static_cast<int64_t>(g[i]) : 0;
+        if constexpr (!SUM)
+            x[e] = mul_var(x[e], valid ? static_cast<int64_t>(img[i]) : 0);
+    }
+    if constexpr (SUM) {
+        for (int q = 1; q < Q; ++q) {
+            g += N;
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int i = perm_pos<L>(eidx<L, LP>(t, e));
-                    x[e] = fold(x[e] - kPs +
-                                mul_var(static_cast<int64_t>(g[i]), static_cast<int64_t>(__ldg(img + i))));
-                }
+            for (int e = 0; e < E; ++e) {
+                const int64_t y = valid ? static_cast<int64_t>(g[perm_pos<L>(eidx<L, LP>(t, e))]) : 0;
+                x[e] = fold(x[e] + y - kPs);
             }
         }
-    } else {
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = 0;
     }
-    (void)T;
     inverse_all<L, true, true>(x, t, twi, SmemLay<1>{sm});
     if (!valid) return;
 #pragma unroll
@@ -484,23 +487,24 @@ __device__ __forceinline__ RowAt row_at(int batch) {
     else return RowAt{blockIdx.y, r << L, true};
 }
 
-template <int L, bool DIRECT, bool CANON>
+// img (kRowTimes): instance b's image at img + b*N.
+template <int L, bool DIRECT, RowOut OUT>
 __global__ void __launch_bounds__(row_threads<L>(), row_min_ctas<L>()) row_fwd_kernel(
-    const FwdIn in, int batch, int l1, const NttTw* __restrict__ tw,
-    const NttTw* __restrict__ Wf) {
+    const FwdIn in, const uint64_t* __restrict__ img, int batch, int l1,
+    const NttTw* __restrict__ tw, const NttTw* __restrict__ Wf) {
     extern __shared__ int64_t sm[];
     const int t = threadIdx.x % Geo<L>::T, v = threadIdx.x / Geo<L>::T, z = blockIdx.z;
     const RowAt r = row_at<L, DIRECT>(batch);
     const size_t off = (r.inst << (L + l1)) + r.base;
     const uint64_t* add = DIRECT ? pick(in.add, z) : nullptr;
-    row_fwd_body<L, DIRECT, CANON>(pick(in.src, z) + off, add ? add + off : nullptr,
-                                   pick(in.dst, z) + off, t, r.valid, tw, Wf + r.base,
-                                   sm + v * Geo<L>::PAD);
+    row_fwd_body<L, DIRECT, OUT>(pick(in.src, z) + off, add ? add + off : nullptr,
+                                 OUT == kRowTimes ? img + off : nullptr, pick(in.dst, z) + off, t,
+                                 r.valid, tw, Wf + r.base, sm + v * Geo<L>::PAD);
 }
 
-// Instance b reads g and img at b*Q*N and writes out at b*N.
-template <int L, bool DIRECT, bool ONE>
-__global__ void __launch_bounds__(row_threads<L>(), row_min_ctas<L>()) row_mac_inv_kernel(
+// Instance b reads g (and img) at b*Q*N and writes out at b*N; Q = 1 unless SUM.
+template <int L, bool DIRECT, bool SUM>
+__global__ void __launch_bounds__(row_threads<L>(), row_min_ctas<L>()) row_inv_kernel(
     const uint64_t* g, const uint64_t* img, int Q, int batch, int l1,
     const NttTw* __restrict__ twi, const NttTw* __restrict__ Wif, uint64_t* out) {
     extern __shared__ int64_t sm[];
@@ -508,8 +512,8 @@ __global__ void __launch_bounds__(row_threads<L>(), row_min_ctas<L>()) row_mac_i
     const RowAt r = row_at<L, DIRECT>(batch);
     const size_t N = size_t{1} << (L + l1);
     const size_t gi = r.inst * Q * N + r.base;
-    row_mac_inv_body<L, ONE, DIRECT>(g + gi, img + gi, Q, N, t, r.valid, twi, Wif + r.base,
-                                     out + r.inst * N + r.base, sm + v * Geo<L>::PAD);
+    row_inv_body<L, SUM, DIRECT>(g + gi, SUM ? nullptr : img + gi, Q, N, t, r.valid, twi,
+                                 Wif + r.base, out + r.inst * N + r.base, sm + v * Geo<L>::PAD);
 }
 
 // A whole product of one-row polynomials (n1 = 1) in one launch: both forward
@@ -592,17 +596,18 @@ struct MixedRow {
     size_t base;
     __device__ __forceinline__ explicit MixedRow(uint32_t tile)
         : base((static_cast<size_t>(tile) * mixed_V<L>() + threadIdx.x / Geo<L>::T) << L) {}
-    __device__ __forceinline__ void fwd(uint64_t* d, const NttTw* tw, const NttTw* Wf,
-                                        int64_t* sm) const {
-        row_fwd_body<L, false, false>(d + base, nullptr, d + base, t, true, tw, Wf + base,
-                                      sm + v * Geo<L>::PAD);
+    template <RowOut OUT>
+    __device__ __forceinline__ void fwd(uint64_t* d, const uint64_t* img, const NttTw* tw,
+                                        const NttTw* Wf, int64_t* sm) const {
+        row_fwd_body<L, false, OUT>(d + base, nullptr, img + base, d + base, t, true, tw, Wf + base,
+                                    sm + v * Geo<L>::PAD);
     }
-    template <bool ONE>
-    __device__ __forceinline__ void mac_inv(const uint64_t* g, const uint64_t* img, int Q, size_t N,
-                                            const NttTw* twi, const NttTw* Wif, uint64_t* out,
-                                            int64_t* sm) const {
-        row_mac_inv_body<L, ONE, false>(g + base, img + base, Q, N, t, true, twi, Wif + base,
-                                        out + base, sm + v * Geo<L>::PAD);
+    template <bool SUM>
+    __device__ __forceinline__ void inv(const uint64_t* g, const uint64_t* img, int Q, size_t N,
+                                        const NttTw* twi, const NttTw* Wif, uint64_t* out,
+                                        int64_t* sm) const {
+        row_inv_body<L, SUM, false>(g + base, SUM ? nullptr : img + base, Q, N, t, true, twi,
+                                    Wif + base, out + base, sm + v * Geo<L>::PAD);
     }
 };
 
@@ -647,7 +652,7 @@ __global__ void __launch_bounds__(kMixedRowThreads) mixed_row_fwd_kernel(
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
     uint64_t* d = blockIdx.y ? p.c : p.A;
-#define PCGB_CALL(LL) MixedRow<LL>(j.tile).fwd(d, p.tw2, p.Wf, sm)
+#define PCGB_CALL(LL) MixedRow<LL>(j.tile).template fwd<kRowLazy>(d, nullptr, p.tw2, p.Wf, sm)
     PCGB_MIXED_SWITCH(p.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
@@ -658,7 +663,8 @@ __global__ void __launch_bounds__(kMixedRowThreads) mixed_row_mul_kernel(
     extern __shared__ int64_t sm[];
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
-#define PCGB_CALL(LL) MixedRow<LL>(j.tile).template mac_inv<true>(p.c, p.A, 1, 0, p.tw2i, p.Wif, p.c, sm)
+#define PCGB_CALL(LL) \
+    MixedRow<LL>(j.tile).template inv<false>(p.c, p.A, 1, 0, p.tw2i, p.Wif, p.c, sm)
     PCGB_MIXED_SWITCH(p.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
@@ -677,10 +683,10 @@ __global__ void __launch_bounds__(kMixedColThreads, 2) mixed_col_inv_kernel(
 
 // ---- multi-request multiply-accumulate ------------------------------------
 // The step-4 transforms of several expansions of different lengths
-// 2^14 .. 2^20 (sub-lengths 2^7 .. 2^10) in four launches: the column and the
-// row pass of every request's Q g' buffers, the Q-way multiply-accumulate
-// with the inverse row pass, and the inverse column pass into each request's
-// z.  The CTA shapes are the mixed kernels' (512 column threads, 64 row
+// 2^14 .. 2^20 (sub-lengths 2^7 .. 2^10) in four launches: the column pass and
+// the row pass (times the image) of every request's Q g' buffers, the Q-way
+// sum with the inverse row pass, and the inverse column pass into each
+// request's z.  The CTA shapes are the mixed kernels' (512 column threads, 64 row
 // threads, the same shared memory at every sub-length down to 2^7).
 struct MacReq {
     uint64_t* g;                 // Q*N words, transformed in place
@@ -738,8 +744,9 @@ __global__ void __launch_bounds__(kMixedRowThreads) mac_row_fwd_kernel(
     extern __shared__ int64_t sm[];
     const MacCta j = ctas[blockIdx.x];
     const MacReq& r = reqs[j.req];
-    uint64_t* d = r.g + (static_cast<size_t>(j.q) << (r.l1 + r.l2));
-#define PCGB_CALL(LL) MixedRow<LL>(j.tile).fwd(d, r.tw2, r.Wf, sm)
+    const size_t off = static_cast<size_t>(j.q) << (r.l1 + r.l2);
+#define PCGB_CALL(LL) \
+    MixedRow<LL>(j.tile).template fwd<kRowTimes>(r.g + off, r.img + off, r.tw2, r.Wf, sm)
     PCGB_MAC_SWITCH(r.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
@@ -751,7 +758,7 @@ __global__ void __launch_bounds__(kMixedRowThreads) mac_row_inv_kernel(
     const MacReq& r = reqs[j.req];
     const size_t N = size_t{1} << (r.l1 + r.l2);
 #define PCGB_CALL(LL) \
-    MixedRow<LL>(j.tile).template mac_inv<false>(r.g, r.img, r.Q, N, r.tw2i, r.Wif, r.z, sm)
+    MixedRow<LL>(j.tile).template inv<true>(r.g, nullptr, r.Q, N, r.tw2i, r.Wif, r.z, sm)
     PCGB_MAC_SWITCH(r.l2, PCGB_CALL)
 #undef PCGB_CALL
 }
@@ -857,10 +864,13 @@ NttTw* upload_root_table(uint64_t psi_n, int logn) {
     return d;
 }
 
-// Lengths up to 2^12 are one row (l1 = 0): a row CTA holds the whole
-// polynomial, so there are no column passes.  At 2^13 one CTA takes 55 us for a
-// product, the column and row passes 24.7.
-constexpr int kDirectLogN = 12;
+// Transforms up to 2^9 are one row (l1 = 0): a row CTA holds the whole
+// polynomial, so there are no column passes.  Longer ones would keep a single
+// SM busy where the four-step passes spread over several (2^12, three
+// transforms: 18 us against 10).  A product is one launch instead of four
+// passes, so it stays one row up to 2^12: 18.5 us against about 22; at 2^13, 55
+// against 24.7.
+constexpr int kDirectLogN = 9, kOneRowLogN = 12;
 
 NttPlan* build_plan(int logN) {
     auto* pl = new NttPlan();
@@ -895,6 +905,19 @@ NttPlan* build_plan(int logN) {
     twiddle_kernel<<<static_cast<unsigned>((pl->N + 255) / 256), 256>>>(
         pl->Wf, pl->Wif, pl->l1, pl->l2, d_pow, R, ninvR, w0R, w0iR);
     PCGB_POST_LAUNCH();
+    if (pl->direct()) {
+        pl->one_tw = pl->tw2;
+        pl->one_twi = pl->tw2i;
+        pl->one_Wi = pl->Wif;
+    } else if (logN <= kOneRowLogN) {
+        pl->one_tw = upload_root_table(psi, logN);
+        pl->one_twi = upload_root_table(psi_inv, logN);
+        // (a forward twiddle table comes with it: N entries of ones and w0)
+        PCGB_CK(cudaMalloc(&pl->one_Wi, 2 * sizeof(NttTw) * pl->N));
+        twiddle_kernel<<<static_cast<unsigned>((pl->N + 255) / 256), 256>>>(
+            pl->one_Wi + pl->N, pl->one_Wi, 0, logN, d_pow, R, ninvR, w0R, w0iR);
+        PCGB_POST_LAUNCH();
+    }
     PCGB_CK(cudaDeviceSynchronize());
     cudaFree(d_pow);
     return pl;
@@ -981,42 +1004,44 @@ dim3 row_grid(const NttPlan& pl, int batch, int count) {
 }
 
 template <int L>
-void row_fwd_l(const NttPlan& pl, const FwdIn& in, int count, int batch, bool canonical,
-               cudaStream_t st) {
+void row_fwd_l(const NttPlan& pl, const FwdIn& in, const uint64_t* img, int count, int batch,
+               RowOut out, cudaStream_t st) {
     constexpr size_t sm = row_smem<L>();
     auto go = [&](auto kernel) {
         g_optin(kernel, sm);
-        kernel<<<row_grid<L>(pl, batch, count), row_threads<L>(), sm, st>>>(in, batch, pl.l1,
+        kernel<<<row_grid<L>(pl, batch, count), row_threads<L>(), sm, st>>>(in, img, batch, pl.l1,
                                                                            pl.tw2, pl.Wf);
     };
-    if constexpr (L >= 7) {   // rows of 2^13 .. 2^24
-        if (!pl.direct()) {
-            canonical ? go(row_fwd_kernel<L, false, true>) : go(row_fwd_kernel<L, false, false>);
-            PCGB_POST_LAUNCH();
-            return;
-        }
+    auto by_out = [&](auto D) {
+        constexpr bool d = decltype(D)::value;
+        if (out == kRowCanon) go(row_fwd_kernel<L, d, kRowCanon>);
+        else if (out == kRowTimes) go(row_fwd_kernel<L, d, kRowTimes>);
+        else if constexpr (!d) go(row_fwd_kernel<L, d, kRowLazy>);   // a product's operands
+    };
+    if constexpr (L <= kDirectLogN) {
+        if (pl.direct()) by_out(std::true_type{});
     }
-    canonical ? go(row_fwd_kernel<L, true, true>) : go(row_fwd_kernel<L, true, false>);
+    if constexpr (L > kDirectLogN / 2) {
+        if (!pl.direct()) by_out(std::false_type{});
+    }
     PCGB_POST_LAUNCH();
 }
 
 template <int L>
-void row_mac_inv_l(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
-                   uint64_t* out, cudaStream_t st) {
+void row_inv_l(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
+               uint64_t* out, cudaStream_t st) {
     constexpr size_t sm = row_smem<L>();
     auto go = [&](auto kernel) {
         g_optin(kernel, sm);
         kernel<<<row_grid<L>(pl, batch, 1), row_threads<L>(), sm, st>>>(g, img, Q, batch, pl.l1,
                                                                        pl.tw2i, pl.Wif, out);
     };
-    if constexpr (L >= 7) {
-        if (!pl.direct()) {
-            Q == 1 ? go(row_mac_inv_kernel<L, false, true>) : go(row_mac_inv_kernel<L, false, false>);
-            PCGB_POST_LAUNCH();
-            return;
-        }
+    if constexpr (L <= kDirectLogN) {
+        if (pl.direct()) go(row_inv_kernel<L, true, true>);   // products run as one launch
     }
-    Q == 1 ? go(row_mac_inv_kernel<L, true, true>) : go(row_mac_inv_kernel<L, true, false>);
+    if constexpr (L > kDirectLogN / 2) {
+        if (!pl.direct()) img ? go(row_inv_kernel<L, false, false>) : go(row_inv_kernel<L, false, true>);
+    }
     PCGB_POST_LAUNCH();
 }
 
@@ -1025,8 +1050,8 @@ void row_product_l(const NttPlan& pl, uint64_t* c, const uint64_t* a, const uint
                    cudaStream_t st) {
     constexpr size_t sm = row_smem<L>();
     g_optin(row_product_kernel<L>, sm);
-    row_product_kernel<L><<<row_grid<L>(pl, batch, 1), row_threads<L>(), sm, st>>>(
-        c, a, b, batch, pl.tw2, pl.tw2i, pl.Wif);
+    row_product_kernel<L><<<(batch + row_V<L>() - 1) / row_V<L>(), row_threads<L>(), sm, st>>>(
+        c, a, b, batch, pl.one_tw, pl.one_twi, pl.one_Wi);
     PCGB_POST_LAUNCH();
 }
 
@@ -1049,10 +1074,11 @@ void by_len(int L, F&& f) {
         default: fail(PCGB_EINVAL, "NTT sub-length out of range");
     }
 }
-// Column sub-lengths: 2^6 .. 2^12 (logN 13 .. 24).
+// Column sub-lengths: 2^5 .. 2^12 (logN 10 .. 24).
 template <class F>
 void by_col_len(int L, F&& f) {
     switch (L) {
+        case 5: f(std::integral_constant<int, 5>{}); break;
         case 6: f(std::integral_constant<int, 6>{}); break;
         case 7: f(std::integral_constant<int, 7>{}); break;
         case 8: f(std::integral_constant<int, 8>{}); break;
@@ -1070,30 +1096,30 @@ void col_fwd(const NttPlan& pl, const FwdIn& in, int count, int batch, cudaStrea
 void col_inv(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
     by_col_len(pl.l1, [&](auto L) { col_inv_l<decltype(L)::value>(pl, d, batch, st); });
 }
-void row_fwd(const NttPlan& pl, const FwdIn& in, int count, int batch, bool canonical,
-             cudaStream_t st) {
+void row_fwd(const NttPlan& pl, const FwdIn& in, const uint64_t* img, int count, int batch,
+             RowOut out, cudaStream_t st) {
     by_len(pl.l2,
-           [&](auto L) { row_fwd_l<decltype(L)::value>(pl, in, count, batch, canonical, st); });
+           [&](auto L) { row_fwd_l<decltype(L)::value>(pl, in, img, count, batch, out, st); });
 }
-void row_mac_inv(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
-                 uint64_t* out, cudaStream_t st) {
-    by_len(pl.l2,
-           [&](auto L) { row_mac_inv_l<decltype(L)::value>(pl, g, img, Q, batch, out, st); });
+// Sum of Q products (img null), or the product g (.) img.
+void row_inv(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
+             uint64_t* out, cudaStream_t st) {
+    by_len(pl.l2, [&](auto L) { row_inv_l<decltype(L)::value>(pl, g, img, Q, batch, out, st); });
 }
 
 // Forward transforms of `count` batches, any 64-bit inputs: the column pass
 // from src (plus add) to dst and the row pass in place, or the single row
-// pass of a direct plan.
-void forward(const NttPlan& pl, const FwdIn& in, int count, int batch, bool canonical,
-             cudaStream_t st) {
+// pass of a direct plan.  out and img as for row_fwd_body.
+void forward(const NttPlan& pl, const FwdIn& in, const uint64_t* img, int count, int batch,
+             RowOut out, cudaStream_t st) {
     if (pl.direct()) {
-        row_fwd(pl, in, count, batch, canonical, st);
+        row_fwd(pl, in, img, count, batch, out, st);
         return;
     }
     col_fwd(pl, in, count, batch, st);
     FwdIn rows;
     for (int z = 0; z < count; ++z) rows.src[z] = rows.dst[z] = in.dst[z];
-    row_fwd(pl, rows, count, batch, canonical, st);
+    row_fwd(pl, rows, img, count, batch, out, st);
 }
 
 FwdIn fwd_one(const uint64_t* src, uint64_t* dst) {
@@ -1136,7 +1162,7 @@ void ntt_forward3(const NttPlan& pl, const uint64_t* const (&src)[3],
         in.add[z] = add[z];
         in.dst[z] = dst[z];
     }
-    forward(pl, in, 3, 1, true, st);
+    forward(pl, in, nullptr, 3, 1, kRowCanon, st);
 }
 
 void ntt_log_sizes(const NttPlan& pl, int* l1, int* l2) {
@@ -1145,7 +1171,7 @@ void ntt_log_sizes(const NttPlan& pl, int* l1, int* l2) {
 }
 
 void ntt_forward(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
-    forward(pl, fwd_one(d, d), 1, batch, true, st);
+    forward(pl, fwd_one(d, d), nullptr, 1, batch, kRowCanon, st);
 }
 
 // Per device: a second stream and two events for the two-half schedule of
@@ -1163,12 +1189,12 @@ HalfFork& half_fork() {
     return f[dev];
 }
 
-bool poly_mul_needs_scratch(const NttPlan& pl) { return !pl.direct(); }
+bool poly_mul_needs_scratch(const NttPlan& pl) { return pl.one_tw == nullptr; }
 
 void poly_mul_device(const NttPlan& pl, uint64_t* c, const uint64_t* a, const uint64_t* b,
                      int batch, uint64_t* scratch, cudaStream_t st) {
-    if (pl.direct()) {
-        by_len(pl.l2,
+    if (pl.one_tw) {
+        by_len(pl.logN,
                [&](auto L) { row_product_l<decltype(L)::value>(pl, c, a, b, batch, st); });
         return;
     }
@@ -1184,8 +1210,8 @@ void poly_mul_device(const NttPlan& pl, uint64_t* c, const uint64_t* a, const ui
         } else {
             col_fwd(pl, fwd_two(x, A, y, C), 2, count, s);
         }
-        row_fwd(pl, fwd_two(A, A, C, C), 2, count, false, s);
-        row_mac_inv(pl, C, A, 1, count, C, s);
+        row_fwd(pl, fwd_two(A, A, C, C), nullptr, 2, count, kRowLazy, s);
+        row_inv(pl, C, A, 1, count, C, s);
         col_inv(pl, C, count, s);
     };
     // A batch of 2^18 words or more runs as two halves on two streams: each
@@ -1305,8 +1331,8 @@ void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const*
 
 void ntt_mac_inverse(const NttPlan& pl, uint64_t* g, const uint64_t* img, int Q, uint64_t* acc,
                      cudaStream_t st) {
-    forward(pl, fwd_one(g, g), 1, Q, false, st);
-    row_mac_inv(pl, g, img, Q, 1, acc, st);
+    forward(pl, fwd_one(g, g), img, 1, Q, kRowTimes, st);
+    row_inv(pl, g, nullptr, Q, 1, acc, st);
     if (!pl.direct()) col_inv(pl, acc, 1, st);
 }
 
