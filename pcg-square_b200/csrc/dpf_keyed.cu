@@ -14,6 +14,12 @@ namespace pcgb {
 std::vector<int> tops_stages(int K, int w, int to_level) {
     std::vector<int> b{0};
     int l = 0;
+    while (l < to_level && tops_bfs_ok(K, w, 0, l + 1) &&
+           ((static_cast<size_t>(K) << (w * l)) < kTopsStage2Threads ||
+            (w == 1 && to_level - l > kTopsFixedLevels)))
+        ++l;
+    const bool bfs = l > 0;
+    if (bfs) b.push_back(l);
     while (l < to_level) {
         if ((static_cast<size_t>(K) << (w * l)) >= kTopsStage2Threads) {
             b.push_back(to_level);
@@ -27,10 +33,12 @@ std::vector<int> tops_stages(int K, int w, int to_level) {
         b.push_back(l);
     }
     if (w == 1) {
-        // Split deeper stages into pieces of at most kTopsFixedLevels, the
+        // Split deeper depth-first stages into pieces of at most kTopsFixedLevels, the
         // last piece the full length: [7, 16) becomes [7, 8), [8, 16).
         std::vector<int> out{b[0]};
-        for (size_t i = 1; i < b.size(); ++i) {
+        size_t i = 1;
+        if (bfs) out.push_back(b[i++]);
+        for (; i < b.size(); ++i) {
             std::vector<int> cuts;
             for (int e = b[i]; e - out.back() > kTopsFixedLevels; e -= kTopsFixedLevels)
                 cuts.push_back(e - kTopsFixedLevels);
@@ -111,7 +119,6 @@ void keyed_tops_multi(int groups, const int* K, const int* n, const int* to_leve
     try {
         for (size_t s = 0; s < stages; ++s) {
             std::vector<TopsJob> jobs;
-            unsigned long long total = 0;
             for (int g = 0; g < groups; ++g) {
                 const Plan& P = plan[g];
                 if (K[g] == 0 || s + 1 >= P.b.size()) continue;
@@ -119,18 +126,18 @@ void keyed_tops_multi(int groups, const int* K, const int* n, const int* to_leve
                 J.src = s == 0 ? roots[g] : P.base + ((s - 1) % 2) * P.half;
                 J.dst = (s + 2 == P.b.size()) ? out[g] : P.base + (s % 2) * P.half;
                 J.cws = cws[g];
-                J.first = total;
+                J.first = 0;   // numbered per launch
+                J.G = 1;
                 J.K = K[g];
                 J.src_lvl = P.b[s];
                 J.nlev = P.b[s + 1] - P.b[s];
                 J.levels = P.levels;
-                total += static_cast<unsigned long long>(K[g]) << (w * P.b[s]);
                 jobs.push_back(J);
             }
             if (prg == PCGB_PRG_AES)
-                keyed_tops_multi_aes(w, jobs, d_jobs, total, aes_te_table_device(), d_rk, st);
+                keyed_tops_multi_aes(w, jobs, d_jobs, aes_te_table_device(), d_rk, st);
             else
-                keyed_tops_multi_chacha(w, jobs, d_jobs, total, st);
+                keyed_tops_multi_chacha(w, jobs, d_jobs, st);
         }
     } catch (...) {
         if (pool) cudaFreeAsync(pool, st);
@@ -256,6 +263,16 @@ void gather_plan_free(GatherPlan& gp) {
     gp.d_off = nullptr; gp.d_entries = nullptr; gp.d_qorder = nullptr; gp.d_qslot = nullptr;
 }
 
+// log2 of the CTAs that share a tile's key halves: one until the launch has
+// four waves of resident threads (1024 per SM at 64 registers) without, else
+// up to a cluster of 8, each keeping at least two of the 2t .. 4t halves.
+int leaf_lsplit(size_t threads, int t) {
+    const size_t want = static_cast<size_t>(sm_count()) * 1024 * 4;
+    int l = 0;
+    while (l < 3 && (threads << l) < want && (2 * t >> (l + 1)) >= 2) ++l;
+    return l;
+}
+
 void keyed_leaf_gather(const GatherPlan& gp, int party, int prg, const Blk* F, const Blk* cws,
                        const uint64_t* cw_out, const uint32_t* d_aes_rk, uint64_t* gq,
                        cudaStream_t st) {
@@ -265,11 +282,12 @@ void keyed_leaf_gather(const GatherPlan& gp, int party, int prg, const Blk* F, c
     int tpb = gp.tpb > 0 ? gp.tpb : 256;
     while (tpb > 1 && static_cast<size_t>(tpb) * gp.S > L.bin) tpb >>= 1;
     if (static_cast<size_t>(tpb) * gp.S > L.bin) fail(PCGB_EINVAL, "bin smaller than one tile");
-    L.tpb = tpb;
     if (gp.Qs == 0) return;   // a shard with no pairs
-    L.grid = dim3(static_cast<unsigned>(L.bin / (static_cast<size_t>(tpb) * gp.S)),
+    L.lsplit = leaf_lsplit(static_cast<size_t>(gp.Qs) * gp.N / gp.S, gp.t);
+    L.tpb = tpb;
+    L.grid = dim3(static_cast<unsigned>(L.bin / (static_cast<size_t>(tpb) * gp.S)) << L.lsplit,
                   static_cast<unsigned>(gp.t), static_cast<unsigned>(gp.Qs));
-    L.smem = static_cast<size_t>(tpb) * (gp.S + 1) * 2 * sizeof(uint64_t) +
+    L.smem = static_cast<size_t>(L.tpb) * (gp.S + 1) * 2 * sizeof(uint64_t) +
              (prg == PCGB_PRG_AES ? keyed_aes_smem_bytes_aes() : 0);
     L.st = st;
     L.F = F; L.cws = cws; L.cw_out = cw_out;

@@ -19,14 +19,13 @@ void keyed_deal_aes(int w, unsigned grid, size_t smem, uint64_t seed, int c, int
                        r2, st);
 }
 
-void keyed_tops_multi_aes(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
-                             unsigned long long total, const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
-    tops_multi_for_prg<kPrgAes>(w, jobs, d_jobs, total, te, rk, st);
+void keyed_tops_multi_aes(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs, const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
+    tops_multi_for_prg<kPrgAes>(w, jobs, d_jobs, te, rk, st);
 }
 
-void keyed_leaf_multi_aes(int w, int sl, const LeafJob* d_jobs, int njobs, unsigned ctas, int tpb,
+void keyed_leaf_multi_aes(int w, int sl, const LeafJob* jobs, int njobs, int lsplit, int tpb,
                           size_t smem, const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
-    leaf_multi_for_prg<kPrgAes>(w, sl, d_jobs, njobs, ctas, tpb, smem, te, rk, st);
+    leaf_multi_for_prg<kPrgAes>(w, sl, jobs, njobs, lsplit, tpb, smem, te, rk, st);
 }
 
 size_t keyed_aes_smem_bytes_aes() { return sizeof(AesSmem); }

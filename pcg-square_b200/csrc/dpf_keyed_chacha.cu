@@ -19,14 +19,13 @@ void keyed_deal_chacha(int w, unsigned grid, size_t smem, uint64_t seed, int c, 
                        r2, st);
 }
 
-void keyed_tops_multi_chacha(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
-                             unsigned long long total, cudaStream_t st) {
-    tops_multi_for_prg<kPrgChaCha>(w, jobs, d_jobs, total, nullptr, nullptr, st);
+void keyed_tops_multi_chacha(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs, cudaStream_t st) {
+    tops_multi_for_prg<kPrgChaCha>(w, jobs, d_jobs, nullptr, nullptr, st);
 }
 
-void keyed_leaf_multi_chacha(int w, int sl, const LeafJob* d_jobs, int njobs, unsigned ctas, int tpb,
+void keyed_leaf_multi_chacha(int w, int sl, const LeafJob* jobs, int njobs, int lsplit, int tpb,
                           size_t smem, const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
-    leaf_multi_for_prg<kPrgChaCha>(w, sl, d_jobs, njobs, ctas, tpb, smem, te, rk, st);
+    leaf_multi_for_prg<kPrgChaCha>(w, sl, jobs, njobs, lsplit, tpb, smem, te, rk, st);
 }
 
 void deal_multi_chacha_launch(int w, const DealJob* d_jobs, int njobs, unsigned ctas, uint64_t r2,

@@ -25,6 +25,8 @@
 
 #include "pcgb_internal.h"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -36,6 +38,8 @@
 
 namespace pcgb {
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int kPrgAes = PCGB_PRG_AES;
 constexpr int kPrgChaCha = PCGB_PRG_CHACHA8;
@@ -76,11 +80,13 @@ __device__ __forceinline__ void aes_node(const AesPrmt* a, int k, uint64_t lo, u
     aes_ccr_prmt(*a, k, lo, hi, olo, ohi);
 }
 
-// m children of `p` under the level CWs cw[0..nk) (global, broadcast).
-template <int W, int PRG, class A>
+// m children of `p` under the level CWs cw[0..nk) (broadcast; in global
+// memory, or SHARED).
+template <int W, int PRG, bool SHARED = false, class A>
 __device__ __forceinline__ void children(const Blk& p, const Blk* __restrict__ cw,
                                          const A* aes, Blk (&kids)[1 << W]) {
     constexpr int M = 1 << W, NK = M - 1;
+    auto ldcw = [&](int k) { return SHARED ? cw[k] : ldblk(cw + k); };
     const bool t = (p.lo & 1) != 0;
     uint64_t hxl = 0, hxh = 0, cfl = 0, cfh = 0;
     if constexpr (PRG == kPrgChaCha) {
@@ -94,7 +100,7 @@ __device__ __forceinline__ void children(const Blk& p, const Blk* __restrict__ c
                 if (k < NK) {
                     const uint64_t hl = o[4 * c] | (static_cast<uint64_t>(o[4 * c + 1]) << 32);
                     const uint64_t hh = o[4 * c + 2] | (static_cast<uint64_t>(o[4 * c + 3]) << 32);
-                    const Blk cv = ldblk(cw + k);
+                    const Blk cv = ldcw(k);
                     cfl ^= cv.lo; cfh ^= cv.hi;
                     hxl ^= hl; hxh ^= hh;
                     kids[k] = Blk{hl ^ (t ? cv.lo : 0), hh ^ (t ? cv.hi : 0)};
@@ -106,7 +112,7 @@ __device__ __forceinline__ void children(const Blk& p, const Blk* __restrict__ c
         for (int k = 0; k < NK; ++k) {
             uint64_t hl, hh;
             aes_node(aes, k, p.lo, p.hi, hl, hh);
-            const Blk cv = ldblk(cw + k);
+            const Blk cv = ldcw(k);
             cfl ^= cv.lo; cfh ^= cv.hi;
             hxl ^= hl; hxh ^= hh;
             kids[k] = Blk{hl ^ (t ? cv.lo : 0), hh ^ (t ? cv.hi : 0)};
@@ -136,6 +142,94 @@ __device__ __forceinline__ void hash_raw(const Blk& p, const A* aes, Blk (&h)[(1
 #pragma unroll 1
         for (int k = 0; k < NK; ++k) aes_node(aes, k, p.lo, p.hi, h[k].lo, h[k].hi);
     }
+}
+
+// ---------------------------------------------------------------------------
+// tops_bfs: the first stage, root -> level nlev of G keys by one CTA, breadth
+// first through shared memory: a thread per parent of the current level, so
+// the chain is nlev hashes, where the depth-first walk of a narrow stage is a
+// chain of m^nlev of them in a handful of CTAs (64 keys to level 9: 8 us
+// against 21 us in two launches; AES, 777 keys to level 10: 62 us against
+// 148).  Several keys share a CTA once there are enough of them for every SM,
+// so that the narrow levels fill their warps (4096 keys to level 7: 34 us with
+// one key per CTA).
+template <int W, int PRG>
+__device__ __forceinline__ void tops_bfs_body(const Blk* __restrict__ roots,
+                                              const Blk* __restrict__ cws, int keys, int levels,
+                                              int nlev, Blk* __restrict__ out, Blk* sm,
+                                              const AesSmem* aes) {
+    constexpr int M = 1 << W, NK = M - 1;
+    Blk* buf[2] = {sm, sm + (static_cast<size_t>(keys) << (W * (nlev - 1)))};
+    Blk* cw = buf[1] + (static_cast<size_t>(keys) << (W * (nlev - 1)));
+    const int ncw = nlev * NK;
+    for (int i = threadIdx.x; i < keys * ncw; i += blockDim.x)
+        cw[i] = ldblk(cws + static_cast<size_t>(i / ncw) * levels * NK + i % ncw);
+    for (int i = threadIdx.x; i < keys; i += blockDim.x) buf[0][i] = ldblk(roots + i);
+    __syncthreads();
+    for (int l = 0; l < nlev; ++l) {
+        Blk* dst = l + 1 == nlev ? out : buf[(l + 1) & 1];
+        for (int p = threadIdx.x; p < keys << (W * l); p += blockDim.x) {
+            Blk kids[M];
+            children<W, PRG, true>(buf[l & 1][p], cw + (p >> (W * l)) * ncw + l * NK, aes, kids);
+#pragma unroll
+            for (int k = 0; k < M; ++k) stblk(dst + p * M + k, kids[k]);
+        }
+        __syncthreads();
+    }
+}
+
+template <int W, int PRG>
+__global__ void __launch_bounds__(kTopsBfsThreads) tops_bfs_kernel(
+    const Blk* __restrict__ roots, int K, int G, int nlev, int levels, const Blk* __restrict__ cws,
+    const uint32_t* __restrict__ aes_te, const uint32_t* __restrict__ aes_rk,
+    Blk* __restrict__ dst) {
+    constexpr int NK = (1 << W) - 1;
+    extern __shared__ __align__(16) uint64_t tops_dsm[];
+    AesSmem& aes_s = *reinterpret_cast<AesSmem*>(tops_dsm);
+    Blk* sm = reinterpret_cast<Blk*>(PRG == kPrgAes ? static_cast<void*>(&aes_s + 1) : tops_dsm);
+    if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
+    const size_t key = static_cast<size_t>(blockIdx.x) * G;
+    tops_bfs_body<W, PRG>(roots + key, cws + key * levels * NK, min(G, K - static_cast<int>(key)),
+                          levels, nlev, dst + (key << (W * nlev)), sm, &aes_s);
+}
+
+// The same for several key groups: job j owns CTAs [first, first + ceil(K / G)).
+template <int W, int PRG>
+__global__ void __launch_bounds__(kTopsBfsThreads) tops_bfs_multi_kernel(
+    const TopsJob* __restrict__ jobs, int njobs, const uint32_t* __restrict__ aes_te,
+    const uint32_t* __restrict__ aes_rk) {
+    constexpr int NK = (1 << W) - 1;
+    extern __shared__ __align__(16) uint64_t tops_dsm[];
+    AesSmem& aes_s = *reinterpret_cast<AesSmem*>(tops_dsm);
+    Blk* sm = reinterpret_cast<Blk*>(PRG == kPrgAes ? static_cast<void*>(&aes_s + 1) : tops_dsm);
+    if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
+    int j = 0;
+    while (j + 1 < njobs && jobs[j + 1].first <= blockIdx.x) ++j;
+    const TopsJob J = jobs[j];
+    const size_t key = (blockIdx.x - J.first) * J.G;
+    tops_bfs_body<W, PRG>(J.src + key, J.cws + key * J.levels * NK,
+                          min(J.G, J.K - static_cast<int>(key)), J.levels, J.nlev,
+                          J.dst + (key << (W * J.nlev)), sm, &aes_s);
+}
+
+// Keys per CTA for `total` keys in the launch: up to 16 while two CTAs per SM
+// remain and a CTA's last level stays within 2048 nodes.
+inline int tops_bfs_group(int total, int w, int nlev) {
+    int g = 1;
+    while (g < 16 && total / (2 * g) >= 2 * sm_count() && (2 * g) << (w * nlev) <= 2048) g *= 2;
+    return g;
+}
+// CTA size: a thread per parent of the stage's last level, in whole warps.
+inline int tops_bfs_threads(int w, int nlev, int g) {
+    const int parents = g << (w * (nlev - 1));
+    return parents < 32 ? 32 : (parents < kTopsBfsThreads ? parents : kTopsBfsThreads);
+}
+// Two node buffers, the CWs, the AES tables: at most 32 KB + 8 KB + 35 KB.
+template <int PRG>
+size_t tops_bfs_smem(int w, int nlev, int g) {
+    const size_t nodes = (static_cast<size_t>(2 * g) << (w * (nlev - 1))) +
+                         static_cast<size_t>(g) * nlev * ((1 << w) - 1);
+    return nodes * sizeof(Blk) + (PRG == kPrgAes ? sizeof(AesSmem) : 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -312,6 +406,14 @@ __global__ void __launch_bounds__(128) expand_tops_multi_fixed_kernel(
 // table is filled once per CTA, not once per 128 threads).
 constexpr int kAesPrmtThreads = 1024;
 
+// First source node of this thread: consecutive warps of node numbers go to
+// different CTAs, so the last, partial stride of the grid is spread over all
+// SMs instead of filling some of them (777 keys x 2^14: 5.25 strides).
+__device__ __forceinline__ size_t prmt_first_id() {
+    return (static_cast<size_t>(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 +
+           (threadIdx.x & 31);
+}
+
 // TopsFixed1 for AES with the PRMT-addressed tables.
 template <int D, int LV = 0>
 struct TopsFixedAes {
@@ -345,8 +447,7 @@ __global__ void __launch_bounds__(kAesPrmtThreads) expand_tops_prmt_fixed_kernel
     __shared__ AesPrmtKeys keys;
     const AesPrmt A = aes_prmt_setup<1>(prmt_dsm, keys, aes_te, aes_rk);
     const size_t total = static_cast<size_t>(K) << src_lvl;
-    for (size_t id = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; id < total;
-         id += static_cast<size_t>(gridDim.x) * blockDim.x)
+    for (size_t id = prmt_first_id(); id < total; id += static_cast<size_t>(gridDim.x) * blockDim.x)
         TopsFixedAes<D>::run(ldblk(src + id), cws + (id >> src_lvl) * levels + src_lvl, &A,
                              dst + (id << D), 0);
 }
@@ -361,8 +462,7 @@ __global__ void __launch_bounds__(kAesPrmtThreads) expand_tops_prmt_kernel(
     __shared__ AesPrmtKeys keys;
     const AesPrmt A = aes_prmt_setup<NK>(prmt_dsm, keys, aes_te, aes_rk);
     const size_t total = static_cast<size_t>(K) << (W * src_lvl);
-    for (size_t id = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; id < total;
-         id += static_cast<size_t>(gridDim.x) * blockDim.x)
+    for (size_t id = prmt_first_id(); id < total; id += static_cast<size_t>(gridDim.x) * blockDim.x)
         tops_walk<W, kPrgAes>(src, id, src_lvl, nlev, levels, cws, &A, dst);
 }
 
@@ -374,9 +474,8 @@ __global__ void __launch_bounds__(kAesPrmtThreads) expand_tops_multi_prmt_kernel
     extern __shared__ __align__(16) unsigned char prmt_dsm[];
     __shared__ AesPrmtKeys keys;
     const AesPrmt A = aes_prmt_setup<NK>(prmt_dsm, keys, aes_te, aes_rk);
-    for (unsigned long long g = static_cast<unsigned long long>(blockIdx.x) * blockDim.x +
-                                threadIdx.x;
-         g < total; g += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
+    for (unsigned long long g = prmt_first_id(); g < total;
+         g += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
         int j = 0;
         while (j + 1 < njobs && jobs[j + 1].first <= g) ++j;
         const TopsJob J = jobs[j];
@@ -491,16 +590,24 @@ struct DfsM {
     }
 };
 
-// One CTA's tile of the fused leaf kernel: output bin r of launched pair
-// z, tile bx.  acc_s is the CTA's dynamic shared memory (blockDim.x rows of
-// S + 1 128-bit accumulators).
+// One CTA's share of a tile of the fused leaf kernel: output bin r of launched
+// pair z, tile bx.  The 2^lsplit CTAs of a cluster share the tile: each takes
+// every 2^lsplit-th key half, and their sums meet at write-out through
+// distributed shared memory.  A thread's chain is 2t or 4t key halves long, so
+// a small expansion alone would keep a few warps busy for tens of microseconds
+// (N = 2^12, c = 2, t = 4: 45 us in 24 CTAs; leaf_lsplit chooses).  The share
+// is chosen by CTA and not by thread so that the key, its correction words and
+// its sign stay uniform: with the groups inside a CTA the kernel of 8 leaves a
+// thread needs 89 registers instead of 64 and the headline stage runs 1 %
+// slower.  acc_s is the CTA's dynamic shared memory (blockDim.x rows of S + 1
+// 128-bit accumulators).
 template <int W, int SL, int PRG>
 __device__ __forceinline__ void leaf_gather_tile(
     const Blk* __restrict__ F, const Blk* __restrict__ cws, const uint64_t* __restrict__ cw_out,
     const uint32_t* __restrict__ off, const uint32_t* __restrict__ entries,
     const uint16_t* __restrict__ q_order, const uint16_t* __restrict__ q_slot, int t, int levels,
     int hl, size_t bin, int N, int party, uint64_t* __restrict__ gq, unsigned bx, int r, int z,
-    ulonglong2* acc_s, const AesSmem* aes_s) {
+    int lsplit, unsigned share, ulonglong2* acc_s, const AesSmem* aes_s) {
     constexpr int M = 1 << W, NK = M - 1;
     constexpr int S = 1 << (W * SL);
     constexpr int STRIDE = S + 1;  // padded accumulator rows: conflict-free
@@ -516,7 +623,7 @@ __device__ __forceinline__ void leaf_gather_tile(
     const uint32_t e0 = off[q * t + r], e1 = off[q * t + r + 1];
     LeafCtx c;
     c.acc = acc;
-    for (uint32_t e = e0; e < e1; ++e) {
+    for (uint32_t e = e0 + share; e < e1; e += 1u << lsplit) {
         const uint32_t ent = __ldg(entries + e);
         const size_t key = ent >> 2;
         const size_t half = (ent >> 1) & 1;
@@ -527,55 +634,95 @@ __device__ __forceinline__ void leaf_gather_tile(
         if constexpr (W == 1) Dfs1<SL, PRG>::run(node, kcw, aes_s, 0, c);
         else DfsM<W, SL, PRG>::run(node, kcw, aes_s, 0, c);
     }
-    __syncthreads();
-    // Coalesced write-out of the CTA's tile.
+    // Coalesced write-out of the tile.
     uint64_t* dst = gq + static_cast<size_t>(slot) * N + static_cast<size_t>(r) * bin +
                     static_cast<size_t>(bx) * tile;
-    for (size_t e = threadIdx.x; e < tile; e += blockDim.x)
-        dst[e] = acc_mod_p(acc_s[(e / S) * STRIDE + (e % S)]);
+    if (lsplit == 0) {
+        __syncthreads();
+        for (size_t e = threadIdx.x; e < tile; e += blockDim.x)
+            dst[e] = acc_mod_p(acc_s[(e / S) * STRIDE + (e % S)]);
+        return;
+    }
+    // Each CTA of the cluster sums and writes its part of the positions.
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const unsigned part = (static_cast<unsigned>(tile) + (1u << lsplit) - 1) >> lsplit;
+    const unsigned e_end = min(static_cast<unsigned>(tile), (share + 1) * part);
+#pragma unroll 1
+    for (unsigned e = share * part + threadIdx.x; e < e_end; e += blockDim.x) {
+        ulonglong2* at = acc_s + (e / S) * STRIDE + (e % S);
+        ulonglong2 v = make_ulonglong2(0, 0);
+#pragma unroll 1
+        for (unsigned k = 0; k < 1u << lsplit; ++k) {
+            const ulonglong2 b = *cluster.map_shared_rank(at, k);
+            v.x += b.x;
+            v.y += b.y + (v.x < b.x ? 1 : 0);
+        }
+        dst[e] = acc_mod_p(v);
+    }
+    cluster.sync();   // the others may still be reading this CTA's sums
 }
 
+// grid.x = tiles << lsplit, in clusters of 1 << lsplit.
 template <int W, int SL, int PRG>
 __global__ void __launch_bounds__(256) leaf_gather_kernel(
     const Blk* __restrict__ F, const Blk* __restrict__ cws, const uint64_t* __restrict__ cw_out,
     const uint32_t* __restrict__ off, const uint32_t* __restrict__ entries,
     const uint16_t* __restrict__ q_order, const uint16_t* __restrict__ q_slot, int t, int levels,
     int hl, size_t bin, int N,
-    int party, const uint32_t* __restrict__ aes_te, const uint32_t* __restrict__ aes_rk,
-    uint64_t* __restrict__ gq) {
+    int party, int lsplit, const uint32_t* __restrict__ aes_te,
+    const uint32_t* __restrict__ aes_rk, uint64_t* __restrict__ gq) {
     constexpr int NK = (1 << W) - 1, S = 1 << (W * SL);
     extern __shared__ __align__(16) ulonglong2 acc_s[];
     AesSmem& aes_s = *reinterpret_cast<AesSmem*>(acc_s + blockDim.x * (S + 1));
     if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
     leaf_gather_tile<W, SL, PRG>(F, cws, cw_out, off, entries, q_order, q_slot, t, levels, hl, bin,
-                                 N, party, gq, blockIdx.x, blockIdx.y, blockIdx.z, acc_s, &aes_s);
+                                 N, party, gq, blockIdx.x >> lsplit, blockIdx.y, blockIdx.z,
+                                 lsplit, blockIdx.x & ((1u << lsplit) - 1), acc_s, &aes_s);
 }
 
 // The fused leaf kernel over several expansions (one job each, same w, sl,
-// PRG and CTA size): CTA b belongs to the job whose CTA range holds b, and
-// runs that job's tile (bx, r, z) = its local index in x-fastest order.
+// PRG and CTA size): cluster b of 1 << lsplit CTAs belongs to the job whose
+// range holds b, and runs that job's tile (bx, r, z) = its local index in
+// x-fastest order.  The jobs are a kernel parameter, so their fields are
+// uniform (constant-bank) operands as in the single kernel: 64 registers,
+// where a table in global memory took 80 to 100.
 template <int W, int SL, int PRG>
 __global__ void __launch_bounds__(256) leaf_gather_multi_kernel(
-    const LeafJob* __restrict__ jobs, int njobs, const uint32_t* __restrict__ aes_te,
-    const uint32_t* __restrict__ aes_rk) {
+    const __grid_constant__ LeafJobTable tab, int njobs, int lsplit,
+    const uint32_t* __restrict__ aes_te, const uint32_t* __restrict__ aes_rk) {
     constexpr int NK = (1 << W) - 1, S = 1 << (W * SL);
     extern __shared__ __align__(16) ulonglong2 acc_s[];
     AesSmem& aes_s = *reinterpret_cast<AesSmem*>(acc_s + blockDim.x * (S + 1));
     if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
+    const unsigned b = blockIdx.x >> lsplit;
     int k = 0;
-    while (k + 1 < njobs && jobs[k + 1].first <= blockIdx.x) ++k;
-    const LeafJob& J = jobs[k];
-    const unsigned local = blockIdx.x - J.first;
+    while (k + 1 < njobs && tab.job[k + 1].first <= b) ++k;
+    const LeafJob& J = tab.job[k];
+    const unsigned local = b - J.first;
     const unsigned bx = local % J.gx, r = (local / J.gx) % J.gy, z = local / (J.gx * J.gy);
     leaf_gather_tile<W, SL, PRG>(J.F, J.cws, J.cw_out, J.off, J.entries, J.q_order, J.q_slot, J.t,
                                  J.levels, J.hl, J.bin, J.N, J.party, J.gq, bx,
-                                 static_cast<int>(r), static_cast<int>(z), acc_s, &aes_s);
+                                 static_cast<int>(r), static_cast<int>(z), lsplit,
+                                 blockIdx.x & ((1u << lsplit) - 1), acc_s, &aes_s);
 }
 
 template <int W, int PRG>
 void launch_tops(const Blk* src, int K, int src_lvl, int nlev, int levels, const Blk* cws,
                  const uint32_t* te, const uint32_t* rk, Blk* dst, cudaStream_t st) {
     if (nlev < 0 || nlev >= tops_max_depth<W>()) fail(PCGB_EINVAL, "keyed expansion deeper than the DFS stack");
+    if (tops_bfs_ok(K, W, src_lvl, nlev)) {
+        const int G = tops_bfs_group(K, W, nlev);
+        const size_t smem = tops_bfs_smem<PRG>(W, nlev, G);
+        if (smem > 48 * 1024)
+            PCGB_CK(cudaFuncSetAttribute(tops_bfs_kernel<W, PRG>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem)));
+        tops_bfs_kernel<W, PRG><<<(K + G - 1) / G, tops_bfs_threads(W, nlev, G), smem, st>>>(
+            src, K, G, nlev, levels, cws, te, rk, dst);
+        PCGB_POST_LAUNCH();
+        return;
+    }
     const size_t threads = static_cast<size_t>(K) << (W * src_lvl);
     if constexpr (PRG == kPrgAes) {
         // A stage with fewer threads than one wave of PRMT CTAs keeps the
@@ -747,12 +894,46 @@ void tops_for_prg(int K, int levels, int w, const Blk* roots, const Blk* cws, co
 }
 
 template <int W, int PRG>
-void tops_multi_launch(const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
-                       unsigned long long total, const uint32_t* te, const uint32_t* rk,
-                       cudaStream_t st) {
-    for (const TopsJob& J : jobs)
+void tops_multi_launch(const std::vector<TopsJob>& all, TopsJob* d_jobs, const uint32_t* te,
+                       const uint32_t* rk, cudaStream_t st) {
+    // The jobs of the stage that run breadth first, then the others, each
+    // with thread (or CTA) numbers of its own.
+    std::vector<TopsJob> first, jobs;
+    unsigned long long ctas = 0, total = 0;
+    int keys = 0, threads = 32;
+    size_t bfs_smem = 0;
+    for (const TopsJob& J : all)
+        if (tops_bfs_ok(J.K, W, J.src_lvl, J.nlev)) keys += J.K;
+    for (const TopsJob& J : all) {
         if (J.nlev < 0 || J.nlev >= tops_max_depth<W>())
             fail(PCGB_EINVAL, "keyed expansion deeper than the DFS stack");
+        if (tops_bfs_ok(J.K, W, J.src_lvl, J.nlev)) {
+            first.push_back(J);
+            TopsJob& F = first.back();
+            F.first = ctas;
+            F.G = tops_bfs_group(keys, W, J.nlev);
+            ctas += static_cast<unsigned long long>((J.K + F.G - 1) / F.G);
+            threads = std::max(threads, tops_bfs_threads(W, J.nlev, F.G));
+            bfs_smem = std::max(bfs_smem, tops_bfs_smem<PRG>(W, J.nlev, F.G));
+        } else {
+            jobs.push_back(J);
+            jobs.back().first = total;
+            total += static_cast<unsigned long long>(J.K) << (W * J.src_lvl);
+        }
+    }
+    if (!first.empty()) {
+        PCGB_CK(cudaMemcpyAsync(d_jobs, first.data(), first.size() * sizeof(TopsJob),
+                                cudaMemcpyHostToDevice, st));
+        if (bfs_smem > 48 * 1024)
+            PCGB_CK(cudaFuncSetAttribute(tops_bfs_multi_kernel<W, PRG>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(bfs_smem)));
+        tops_bfs_multi_kernel<W, PRG><<<static_cast<unsigned>(ctas), threads, bfs_smem, st>>>(
+            d_jobs, static_cast<int>(first.size()), te, rk);
+        PCGB_POST_LAUNCH();
+        d_jobs += first.size();
+        if (jobs.empty()) return;
+    }
     const int TPB = 128;
     const unsigned long long cap = static_cast<unsigned long long>(sm_count()) * 8;  // persistent
     if constexpr (PRG == kPrgChaCha && W == 1) {
@@ -818,47 +999,69 @@ void tops_multi_launch(const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
 
 template <int PRG>
 void tops_multi_for_prg(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
-                        unsigned long long total, const uint32_t* te, const uint32_t* rk,
-                        cudaStream_t st) {
+                        const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
     switch (w) {
-        case 1: tops_multi_launch<1, PRG>(jobs, d_jobs, total, te, rk, st); break;
-        case 2: tops_multi_launch<2, PRG>(jobs, d_jobs, total, te, rk, st); break;
-        case 3: tops_multi_launch<3, PRG>(jobs, d_jobs, total, te, rk, st); break;
-        case 4: tops_multi_launch<4, PRG>(jobs, d_jobs, total, te, rk, st); break;
+        case 1: tops_multi_launch<1, PRG>(jobs, d_jobs, te, rk, st); break;
+        case 2: tops_multi_launch<2, PRG>(jobs, d_jobs, te, rk, st); break;
+        case 3: tops_multi_launch<3, PRG>(jobs, d_jobs, te, rk, st); break;
+        case 4: tops_multi_launch<4, PRG>(jobs, d_jobs, te, rk, st); break;
         default: fail(PCGB_EINVAL, "w must be in [1,4]");
     }
 }
 
-template <int W, int SL, int PRG>
-void leaf_one(const LeafLaunch& L) {
-    auto kern = leaf_gather_kernel<W, SL, PRG>;
-    if (L.smem > 48 * 1024)
-        PCGB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(L.smem)));
-    kern<<<L.grid, L.tpb, L.smem, L.st>>>(L.F, L.cws, L.cw_out, L.off, L.entries, L.q_order,
-                                         L.q_slot, L.t,
-                                         L.levels, L.hl, L.bin, L.N, L.party, L.te, L.rk, L.gq);
-    PCGB_POST_LAUNCH();
-}
-
-template <int W, int SL, int PRG>
-void leaf_multi_one(const LeafJob* d_jobs, int njobs, unsigned ctas, int tpb, size_t smem,
-                    const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
-    auto kern = leaf_gather_multi_kernel<W, SL, PRG>;
+// Launch in clusters of 1 << lsplit CTAs along x (a plain launch for lsplit = 0).
+template <class... P, class... A>
+void launch_split(void (*kern)(P...), dim3 grid, int tpb, size_t smem, int lsplit, cudaStream_t st,
+                  const A&... args) {
     if (smem > 48 * 1024)
         PCGB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
-    kern<<<ctas, tpb, smem, st>>>(d_jobs, njobs, te, rk);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(tpb));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1u << lsplit;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = lsplit > 0 ? 1 : 0;
+    PCGB_CK(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
     PCGB_POST_LAUNCH();
 }
 
+template <int W, int SL, int PRG>
+void leaf_one(const LeafLaunch& L) {
+    launch_split(leaf_gather_kernel<W, SL, PRG>, L.grid, L.tpb, L.smem, L.lsplit, L.st, L.F, L.cws,
+                 L.cw_out, L.off, L.entries, L.q_order, L.q_slot, L.t, L.levels, L.hl, L.bin, L.N,
+                 L.party, L.lsplit, L.te, L.rk, L.gq);
+}
+
+template <int W, int SL, int PRG>
+void leaf_multi_one(const LeafJob* jobs, int njobs, int lsplit, int tpb, size_t smem,
+                    const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
+    for (int at = 0; at < njobs; at += kLeafJobsMax) {
+        LeafJobTable tab;
+        const int n = std::min(njobs - at, kLeafJobsMax);
+        unsigned clusters = 0;
+        for (int i = 0; i < n; ++i) {
+            tab.job[i] = jobs[at + i];
+            tab.job[i].first = clusters;
+            clusters += tab.job[i].gx * tab.job[i].gy * tab.job[i].gz;
+        }
+        launch_split(leaf_gather_multi_kernel<W, SL, PRG>, dim3(clusters << lsplit), tpb, smem,
+                     lsplit, st, tab, n, lsplit, te, rk);
+    }
+}
+
 template <int PRG>
-void leaf_multi_for_prg(int w, int sl, const LeafJob* d_jobs, int njobs, unsigned ctas, int tpb,
-                        size_t smem, const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
+void leaf_multi_for_prg(int w, int sl, const LeafJob* jobs, int njobs, int lsplit, int tpb, size_t smem, const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
     switch (w * 8 + sl) {
 #define PCGB_LM(W_, SL_)                                                              \
     case W_ * 8 + SL_:                                                                \
-        leaf_multi_one<W_, SL_, PRG>(d_jobs, njobs, ctas, tpb, smem, te, rk, st); \
+        leaf_multi_one<W_, SL_, PRG>(jobs, njobs, lsplit, tpb, smem, te, rk, st); \
         break;
         PCGB_LM(1, 4) PCGB_LM(1, 3) PCGB_LM(1, 2) PCGB_LM(1, 1)
         PCGB_LM(2, 2) PCGB_LM(2, 1) PCGB_LM(3, 1) PCGB_LM(4, 1)

@@ -444,7 +444,7 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
     }
     std::vector<LeafJob> leaf(count);
     std::vector<XJob> xj(count);
-    unsigned leaf_ctas = 0, x_ctas = 0;
+    unsigned x_ctas = 0;
     size_t x_smem = 0;
     for (int i = 0; i < count; ++i) {
         const pcgb_expander* E = e[i];
@@ -456,8 +456,8 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
         L.t = E->t; L.levels = E->levels; L.hl = E->gp.hl; L.N = E->N; L.party = party[i];
         L.gx = static_cast<unsigned>(L.bin / (static_cast<size_t>(tpb) * S));
         L.gy = static_cast<unsigned>(E->t);
-        L.first = leaf_ctas;
-        leaf_ctas += L.gx * L.gy * static_cast<unsigned>(E->gp.Qs);
+        L.gz = static_cast<unsigned>(E->gp.Qs);
+        L.first = 0;   // numbered per launch
         XJob& X = xj[i];
         X.pos = pos[i]; X.val = val[i]; X.aR = E->d_aR; X.x = x[i];
         X.N = static_cast<size_t>(E->N); X.c = E->c; X.t = E->t; X.i0 = E->i0;
@@ -465,20 +465,19 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
         x_ctas += blocks_for(X.N, 256);
         x_smem = std::max(x_smem, sizeof(uint64_t) * 2 * static_cast<size_t>(E->c) * E->t);
     }
-    const size_t b_leaf = sizeof(LeafJob) * count;
-    const size_t o_x = (b_leaf + 255) & ~size_t{255};
-    const size_t total = o_x + sizeof(XJob) * count;
-    std::vector<char> host(total);
-    std::memcpy(host.data(), leaf.data(), b_leaf);
-    std::memcpy(host.data() + o_x, xj.data(), sizeof(XJob) * count);
-    char* tab = static_cast<char*>(pool_alloc(total, st));
-    PCGB_CK(cudaMemcpyAsync(tab, host.data(), total, cudaMemcpyHostToDevice, st));
+    char* tab = static_cast<char*>(pool_alloc(sizeof(XJob) * count, st));
+    PCGB_CK(cudaMemcpyAsync(tab, xj.data(), sizeof(XJob) * count, cudaMemcpyHostToDevice, st));
     // Stage 2: the fused leaf kernel over every expansion's tiles.
+    // A CTA of a t = 32 expansion runs 4 times as long as one of t = 8 (64 to
+    // 128 key halves a thread), and the launch waits for the last: clusters
+    // of up to 8 CTAs share a tile.
     const size_t leaf_smem = static_cast<size_t>(tpb) * (S + 1) * 2 * sizeof(uint64_t);
-    keyed_leaf_multi_chacha(w, sl, reinterpret_cast<const LeafJob*>(tab), count, leaf_ctas, tpb,
-                            leaf_smem, nullptr, nullptr, st);
+    int lsplit = 3;
+    for (int i = 0; i < count; ++i)
+        while (lsplit > 0 && (2 * e[i]->t >> lsplit) < 2) --lsplit;
+    keyed_leaf_multi_chacha(w, sl, leaf.data(), count, lsplit, tpb, leaf_smem, nullptr, nullptr, st);
     // Stage 3: the sparse x products.
-    x_multi_kernel<<<x_ctas, 256, x_smem, st>>>(reinterpret_cast<const XJob*>(tab + o_x), count);
+    x_multi_kernel<<<x_ctas, 256, x_smem, st>>>(reinterpret_cast<const XJob*>(tab), count);
     PCGB_POST_LAUNCH();
     // Stage 4: NTT multiply-accumulate and inverse, all lengths at once.
     std::vector<uint64_t*> g(count), zz(count);

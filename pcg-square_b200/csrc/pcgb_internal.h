@@ -78,6 +78,7 @@ struct TopsJob {
     const Blk* cws;             // the group's CWs [K][levels][m-1]
     unsigned long long first;   // first global thread index of this job
     int K, src_lvl, nlev, levels;
+    int G;                      // keys per CTA of the breadth-first stage
 };
 // Top-level walk of `groups` key groups of different domains (same w and
 // PRG), each to its own level to_level[g] into out[g]: one launch per stage
@@ -91,10 +92,8 @@ void keyed_tops_multi(int groups, const int* K, const int* n, const int* to_leve
 void keyed_full_eval_multi(int groups, const int* K, const int* n, int w, int prg,
                            const Blk* const* roots, const Blk* const* cws, const uint32_t* d_rk,
                            Blk* const* leaves, cudaStream_t st);
-void keyed_tops_multi_chacha(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
-                             unsigned long long total, cudaStream_t st);
-void keyed_tops_multi_aes(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
-                          unsigned long long total, const uint32_t* te, const uint32_t* rk,
+void keyed_tops_multi_chacha(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs, cudaStream_t st);
+void keyed_tops_multi_aes(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs, const uint32_t* te, const uint32_t* rk,
                           cudaStream_t st);
 void keyed_expand_tops(int K, int n, int w, int prg, const Blk* roots, const Blk* cws,
                        const uint32_t* d_aes_rk, int to_level, Blk* out, Blk* scratch,
@@ -103,16 +102,24 @@ void keyed_expand_tops(int K, int n, int w, int prg, const Blk* roots, const Blk
 // Contribution list of the gather form of the output-layer scatter: for
 // every merged (i<=j) pair q and output bin r, the key halves that land in
 // [r*bin, (r+1)*bin) of the folded g (see gather_plan in dpf_keyed.cu).
-// Keyed top-level expansion runs in stages.  Each stage gives every node of
-// its start level a thread that walks its subtree depth first down to the
-// next boundary; the thread count grows at most 32-fold per stage (so the
-// early, narrow stages do short walks) until K * m^l reaches this many
-// subtrees, and the final stage walks from there to the target level.
+// Keyed top-level expansion runs in stages.  The first is breadth first
+// (tops_bfs_kernel), until K * m^l reaches the thread count below (and, for w =
+// 1, one depth-first stage can take the rest) or a key has 2^10 nodes.  Each later stage gives every node of its start level a thread
+// that walks its subtree depth first down to the next boundary; the thread
+// count grows at most 32-fold per stage (so narrow stages do short walks)
+// until K * m^l reaches this many subtrees, and the final stage walks from
+// there to the target level.
 // 2^19 threads keep every SM busy and the final walks shallow.
 constexpr size_t kTopsStage2Threads = size_t{1} << 19;
 // w = 1 ChaCha8 stages of up to this many levels walk a depth fixed at
 // compile time (registers only); for w = 1 no stage is made deeper.
 constexpr int kTopsFixedLevels = 8;
+// The first stage runs breadth first to at most 2^10 nodes a key; with more
+// keys than this a thread per key fills the chip from the root.
+constexpr int kTopsBfsLog = 10, kTopsBfsThreads = 256, kTopsBfsKeys = 8192;
+inline bool tops_bfs_ok(int K, int w, int src_lvl, int nlev) {
+    return src_lvl == 0 && nlev > 0 && w * nlev <= kTopsBfsLog && K <= kTopsBfsKeys;
+}
 // Stage boundaries 0 = l_0 < l_1 < ... < l_s = to_level.
 std::vector<int> tops_stages(int K, int w, int to_level);
 
@@ -143,6 +150,7 @@ void gather_plan_free(GatherPlan& gp);
 struct LeafLaunch {
     dim3 grid;
     int tpb = 0;
+    int lsplit = 0;   // log2 of the CTAs (a cluster) that share a tile's key halves
     size_t smem = 0;
     cudaStream_t st = nullptr;
     const Blk* F = nullptr;
@@ -161,7 +169,7 @@ struct LeafLaunch {
 };
 
 // One expansion's part of a multi-expansion leaf launch: its LeafLaunch
-// fields plus its CTA range [first, first + gx*gy*gz) in the shared grid.
+// fields plus its range [first, first + gx*gy*gz) of the grid's clusters.
 struct LeafJob {
     const Blk* F;
     const Blk* cws;
@@ -173,8 +181,14 @@ struct LeafJob {
     uint64_t* gq;
     size_t bin;
     int t, levels, hl, N, party;
-    unsigned gx, gy, first;
+    unsigned gx, gy, gz, first;
 };
+// The jobs of one launch, a kernel parameter.
+constexpr int kLeafJobsMax = 32;
+struct LeafJobTable {
+    LeafJob job[kLeafJobsMax];
+};
+static_assert(sizeof(LeafJobTable) <= 4000, "kernel parameters are at most 4 KB");
 
 // One expansion's part of a multi-expansion dealer launch (ChaCha8).
 struct DealJob {
@@ -196,8 +210,7 @@ void deal_multi_chacha_launch(int w, const DealJob* d_jobs, int njobs, unsigned 
                            const uint32_t* te, const uint32_t* rk, int to_level, Blk* out,     \
                            Blk* scratch, cudaStream_t st);                                     \
     void keyed_leaf_##NAME(int w, int sl, const LeafLaunch& L);                                 \
-    void keyed_leaf_multi_##NAME(int w, int sl, const LeafJob* d_jobs, int njobs, unsigned ctas, \
-                                 int tpb, size_t smem, const uint32_t* te, const uint32_t* rk,  \
+    void keyed_leaf_multi_##NAME(int w, int sl, const LeafJob* jobs, int njobs, int lsplit, int tpb, size_t smem, const uint32_t* te, const uint32_t* rk,  \
                                  cudaStream_t st);                                              \
     void keyed_deal_##NAME(int w, unsigned grid, size_t smem, uint64_t seed, int c, int t,      \
                            int n, uint64_t bin, Blk* roots0, Blk* roots1, Blk* cws,            \
@@ -208,6 +221,7 @@ PCGB_KEYED_DECL(chacha)
 PCGB_KEYED_DECL(aes)
 #undef PCGB_KEYED_DECL
 
+int leaf_lsplit(size_t threads, int t);
 // Fused leaf kernel: frontier F (level hl) -> leaves -> out-hash -> convert
 // -> gather into the folded, pair-merged g' (Q buffers of N residues).
 void keyed_leaf_gather(const GatherPlan& gp, int party, int prg, const Blk* F, const Blk* cws,
