@@ -127,15 +127,32 @@ __global__ void __launch_bounds__(kTPB) hash_roots_kernel(const Blk* __restrict_
     cta_xor_reduce<NK>(h, my + static_cast<size_t>(b) * NK, red);
 }
 
+// Parents a thread expands: four once the launch keeps four waves of 8 CTAs
+// per SM that way, so that the CTA's set-up, XOR reduction and atomics are paid
+// once for 512 parents (2^23 parents, w = 1, ChaCha8: 275 -> 258 us, of which
+// the hashes need 223; with the output hashes of the fused last level, 2^22
+// parents, 144 -> 134.5).  One for w > 2, whose parents fill the registers, and
+// for a last level that only writes leaves (2^24 parents: 154 us, at HBM speed;
+// 161 with four).
+int parents_per_thread(size_t sz, int B, int w, bool hashes) {
+    int r = 1;
+    if (w > 2 || !hashes) return r;
+    while (r < 4 && sz >= static_cast<size_t>(2 * r) * kTPB &&
+           static_cast<size_t>(B) * sz / (2 * r * kTPB) >= static_cast<size_t>(sm_count()) * 32)
+        r *= 2;
+    return r;
+}
+
 // Expand level i (frontier size sz, hashes H) with CW = my ^ peer; write the
 // children to nxt; when hash_next, hash the children into Hn and reduce
-// their columns into my_next.  grid = (x, B); thread x*kTPB + t of an
-// instance expands its parent x*kTPB + t.
+// their columns into my_next.  grid = (x, B); CTA x of an instance expands its
+// parents [x*per*kTPB, (x+1)*per*kTPB), the next one's words loading while the
+// current one's children are hashed.
 template <int W, int PRG>
 __global__ void __launch_bounds__(kTPB) expand_level_kernel(
     const Blk* __restrict__ cur, const Blk* __restrict__ H, const Blk* __restrict__ my,
     const Blk* __restrict__ peer, Blk* __restrict__ nxt, Blk* __restrict__ Hn,
-    Blk* __restrict__ my_next, size_t sz, size_t D, size_t HS, int hash_next,
+    Blk* __restrict__ my_next, size_t sz, size_t D, size_t HS, int hash_next, int per,
     const uint32_t* te, const uint32_t* rk) {
     constexpr int M = 1 << W, NK = M - 1;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -155,14 +172,13 @@ __global__ void __launch_bounds__(kTPB) expand_level_kernel(
     Blk acc[NK];
 #pragma unroll
     for (int k = 0; k < NK; ++k) acc[k] = Blk{0, 0};
-    auto parent = [&](const size_t j) {
-        const Blk p = cur[static_cast<size_t>(b) * D + j];
+    auto parent = [&](const size_t j, const Blk& p, auto&& hash_of) {
         const bool t = (p.lo & 1) != 0;
         Blk kids[M];
         uint64_t xl = 0, xh = 0;
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
-            const Blk h = H[static_cast<size_t>(b) * HS + j * NK + k];
+            const Blk h = hash_of(k);
             xl ^= h.lo;
             xh ^= h.hi;
             kids[k] = Blk{h.lo ^ (t ? cw[k].lo : 0), h.hi ^ (t ? cw[k].hi : 0)};
@@ -196,8 +212,29 @@ __global__ void __launch_bounds__(kTPB) expand_level_kernel(
             }
         }
     };
-    const size_t j0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (j0 < sz) parent(j0);
+    size_t j = static_cast<size_t>(blockIdx.x) * per * blockDim.x + threadIdx.x;
+    if constexpr (W <= 2) {
+        Blk p{0, 0}, hs[NK];
+        auto load = [&](const size_t at) {
+            if (at >= sz) return;
+            p = cur[static_cast<size_t>(b) * D + at];
+#pragma unroll
+            for (int k = 0; k < NK; ++k) hs[k] = H[static_cast<size_t>(b) * HS + at * NK + k];
+        };
+        load(j);
+#pragma unroll 1
+        for (int i = 0; i < per && j < sz; ++i, j += blockDim.x) {
+            const Blk q = p;
+            Blk hq[NK];
+#pragma unroll
+            for (int k = 0; k < NK; ++k) hq[k] = hs[k];
+            if (i + 1 < per) load(j + blockDim.x);
+            parent(j, q, [&](int k) { return hq[k]; });
+        }
+    } else if (j < sz) {   // 7 or 15 hash words a parent: no registers to read ahead (per = 1)
+        parent(j, cur[static_cast<size_t>(b) * D + j],
+               [&](int k) { return H[static_cast<size_t>(b) * HS + j * NK + k]; });
+    }
     if (hash_next) cta_xor_reduce<NK>(acc, my_next + static_cast<size_t>(b) * NK, red);
 }
 
@@ -290,16 +327,17 @@ __global__ void __launch_bounds__(kPrmtTPB) expand_level_prmt_kernel(
 // (ChaCha8 out-hash, leaf_convert_cuda.cu's C and tau) into the converted
 // word conv[b*D + d] = C | tau << 63 and reduces C (mod p) and tau over the
 // CTA into partials[b*parts + x] and partials[(B + b)*parts + x].
-// grid = (parts, B), parts = ceil(sz / kTPB).
+// grid = (parts, B), parts = ceil(sz / (per * kTPB)); CTA x takes parents
+// [x*per*kTPB, (x+1)*per*kTPB).
 template <int W>
 __global__ void __launch_bounds__(kTPB) last_level_convert_kernel(
     const Blk* __restrict__ cur, const Blk* __restrict__ H, const Blk* __restrict__ my,
-    const Blk* __restrict__ peer, size_t sz, size_t D, size_t HS, uint64_t* __restrict__ conv,
-    uint64_t* __restrict__ partials) {
+    const Blk* __restrict__ peer, size_t sz, size_t D, size_t HS, int per,
+    uint64_t* __restrict__ conv, uint64_t* __restrict__ partials) {
     constexpr int M = 1 << W, NK = M - 1;
     __shared__ uint64_t sc[kTPB / 32], st[kTPB / 32];
     const int b = blockIdx.y, parts = gridDim.x;
-    const size_t j = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    size_t j = static_cast<size_t>(blockIdx.x) * per * blockDim.x + threadIdx.x;
     Blk cw[NK];
     Blk cwf{0, 0};
 #pragma unroll
@@ -310,20 +348,19 @@ __global__ void __launch_bounds__(kTPB) last_level_convert_kernel(
         cwf.hi ^= cw[k].hi;
     }
     uint64_t csum = 0, tsum = 0;
-    if (j < sz) {
-        const Blk p = cur[static_cast<size_t>(b) * D + j];
+    auto parent = [&](const size_t at, const Blk& p, auto&& hash_of) {
         const bool t = (p.lo & 1) != 0;
         Blk kids[M];
         uint64_t xl = 0, xh = 0;
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
-            const Blk h = H[static_cast<size_t>(b) * HS + j * NK + k];
+            const Blk h = hash_of(k);
             xl ^= h.lo;
             xh ^= h.hi;
             kids[k] = Blk{h.lo ^ (t ? cw[k].lo : 0), h.hi ^ (t ? cw[k].hi : 0)};
         }
         kids[NK] = Blk{xl ^ p.lo ^ (t ? cwf.lo : 0), xh ^ p.hi ^ (t ? cwf.hi : 0)};
-        uint64_t* dst = conv + static_cast<size_t>(b) * D + j * M;
+        uint64_t* dst = conv + static_cast<size_t>(b) * D + at * M;
 #pragma unroll
         for (int k = 0; k < M; ++k) {
             const uint64_t C = reduce_p(out_hash_lo64(kids[k].lo, kids[k].hi));
@@ -331,6 +368,28 @@ __global__ void __launch_bounds__(kTPB) last_level_convert_kernel(
             tsum += kids[k].lo & 1;
             dst[k] = C | (kids[k].lo << 63);
         }
+    };
+    if constexpr (W <= 2) {   // the next parent's words load while this one's are hashed
+        Blk p{0, 0}, hs[NK];
+        auto load = [&](const size_t at) {
+            if (at >= sz) return;
+            p = cur[static_cast<size_t>(b) * D + at];
+#pragma unroll
+            for (int k = 0; k < NK; ++k) hs[k] = H[static_cast<size_t>(b) * HS + at * NK + k];
+        };
+        load(j);
+#pragma unroll 1
+        for (int i = 0; i < per && j < sz; ++i, j += blockDim.x) {
+            const Blk q = p;
+            Blk hq[NK];
+#pragma unroll
+            for (int k = 0; k < NK; ++k) hq[k] = hs[k];
+            if (i + 1 < per) load(j + blockDim.x);
+            parent(j, q, [&](int k) { return hq[k]; });
+        }
+    } else if (j < sz) {   // per = 1
+        parent(j, cur[static_cast<size_t>(b) * D + j],
+               [&](int k) { return H[static_cast<size_t>(b) * HS + j * NK + k]; });
     }
 #pragma unroll
     for (int off = 16; off; off >>= 1) {
@@ -367,24 +426,26 @@ __global__ void convert_fold_kernel(const uint64_t* __restrict__ partials, int p
 struct ConvOut {
     uint64_t* conv;
     uint64_t* partials;
+    int per, parts;   // parents per thread, CTAs per instance
     pcgb_exchange_device_fn dex = nullptr;
     void* dex_user = nullptr;
 };
 
-// my[b][k] = dlt[b][level][k].
-__global__ void seed_kernel(Blk* my, const Blk* dlt, int B, int levels, int nk, int level) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * nk) return;
-    const int b = i / nk, k = i % nk;
-    my[i] = dlt[(static_cast<size_t>(b) * levels + level) * nk + k];
+// my[level][b][k] = dlt[b][level][k]: the share arrays of every level, seeded in
+// one launch; each level's hashes are XORed into its own.
+__global__ void seed_kernel(Blk* my, const Blk* dlt, int B, int levels, int nk) {
+    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= static_cast<size_t>(B) * levels * nk) return;
+    const size_t level = i / (static_cast<size_t>(B) * nk), r = i % (static_cast<size_t>(B) * nk);
+    my[i] = dlt[(r / nk * levels + level) * nk + r % nk];
 }
 
 struct Pool {
     Blk *cur = nullptr, *nxt = nullptr, *H = nullptr, *Hn = nullptr, *dlt = nullptr;
-    Blk *my = nullptr, *myn = nullptr, *peer = nullptr;
+    Blk *my = nullptr, *peer = nullptr;     // my: [levels][B][nk]
     uint32_t* rk = nullptr;
     Blk *h_my = nullptr, *h_peer = nullptr;   // pinned
-    size_t cap_front = 0, cap_h = 0, cap_dlt = 0, cap_cw = 0;
+    size_t cap_front = 0, cap_h = 0, cap_dlt = 0, cap_my = 0, cap_cw = 0;
     std::mutex mu;
 };
 
@@ -425,13 +486,14 @@ Blk* run_levels(Pool& pl, int B, int n, const Blk* roots, const Blk* dltsft,
                               static_cast<size_t>(B), cudaMemcpyHostToDevice, st));
     PCGB_CK(cudaMemcpyAsync(pl.dlt, dltsft, static_cast<size_t>(B) * levels * NK * sizeof(Blk),
                             cudaMemcpyHostToDevice, st));
-    const unsigned sgrid = static_cast<unsigned>((ncw + 255) / 256);
-    seed_kernel<<<sgrid, 256, 0, st>>>(pl.my, pl.dlt, B, levels, NK, 0);
+    seed_kernel<<<static_cast<unsigned>((ncw * levels + 255) / 256), 256, 0, st>>>(
+        pl.my, pl.dlt, B, levels, NK);
     PCGB_POST_LAUNCH();
     hash_roots_kernel<W, PRG><<<dim3(1, B), kTPB, smem, st>>>(pl.cur, D, pl.H, HS, pl.my, te, pl.rk);
     PCGB_POST_LAUNCH();
-    Blk *cur = pl.cur, *nxt = pl.nxt, *H = pl.H, *Hn = pl.Hn, *my = pl.my, *myn = pl.myn;
+    Blk *cur = pl.cur, *nxt = pl.nxt, *H = pl.H, *Hn = pl.Hn;
     for (int i = 0; i < levels; ++i) {
+        Blk *my = pl.my + ncw * i, *myn = my + ncw;   // this level's shares, the next one's
         if (conv && conv->dex) {
             // Shares stay on the device: the callback moves them (NCCL,
             // peer copies) after the level's reduction has finished.
@@ -453,22 +515,20 @@ Blk* run_levels(Pool& pl, int B, int n, const Blk* roots, const Blk* dltsft,
                                     st));
         }
         const int hash_next = (i + 1 < levels) ? 1 : 0;
-        if (hash_next) {
-            seed_kernel<<<sgrid, 256, 0, st>>>(myn, pl.dlt, B, levels, NK, i + 1);
-            PCGB_POST_LAUNCH();
-        }
         const size_t sz = static_cast<size_t>(1) << (W * i);
         if (!hash_next && conv) {
-            // One parent per thread: the grid the fold's `parts` assumes.
-            const dim3 cgrid(static_cast<unsigned>((sz + kTPB - 1) / kTPB), static_cast<unsigned>(B));
+            const dim3 cgrid(static_cast<unsigned>(conv->parts), static_cast<unsigned>(B));
             last_level_convert_kernel<W><<<cgrid, kTPB, 0, st>>>(cur, H, my, pl.peer, sz, D, HS,
-                                                                 conv->conv, conv->partials);
+                                                                 conv->per, conv->conv,
+                                                                 conv->partials);
             PCGB_POST_LAUNCH();
             return nullptr;
         }
         // The last level only writes leaves (no hashing): the plain kernel.
         const bool rep = PRG == PCGB_PRG_AES && sz >= kRepMinParents && hash_next;
-        const dim3 grid(static_cast<unsigned>((sz + kTPB - 1) / kTPB), static_cast<unsigned>(B));
+        const int per = parents_per_thread(sz, B, W, hash_next);
+        const size_t tile = static_cast<size_t>(per) * kTPB;
+        const dim3 grid(static_cast<unsigned>((sz + tile - 1) / tile), static_cast<unsigned>(B));
         if constexpr (PRG == PCGB_PRG_AES) {
             if (rep) {
                 PCGB_CK(cudaFuncSetAttribute(expand_level_prmt_kernel<W>,
@@ -481,16 +541,15 @@ Blk* run_levels(Pool& pl, int B, int n, const Blk* roots, const Blk* dltsft,
                     cur, H, my, pl.peer, nxt, Hn, myn, sz, D, HS, hash_next, B, te, pl.rk);
             } else {
                 expand_level_kernel<W, PRG><<<grid, kTPB, smem, st>>>(
-                    cur, H, my, pl.peer, nxt, Hn, myn, sz, D, HS, hash_next, te, pl.rk);
+                    cur, H, my, pl.peer, nxt, Hn, myn, sz, D, HS, hash_next, per, te, pl.rk);
             }
         } else {
             expand_level_kernel<W, PRG><<<grid, kTPB, smem, st>>>(
-                cur, H, my, pl.peer, nxt, Hn, myn, sz, D, HS, hash_next, te, pl.rk);
+                cur, H, my, pl.peer, nxt, Hn, myn, sz, D, HS, hash_next, per, te, pl.rk);
         }
         PCGB_POST_LAUNCH();
         std::swap(cur, nxt);
         std::swap(H, Hn);
-        std::swap(my, myn);
     }
     return cur;
 }
@@ -521,10 +580,9 @@ Blk* interactive_eval(int B, int n, int w, const Blk* roots, const Blk* dltsft, 
     grow_pair(pl.H, pl.Hn, pl.cap_h, static_cast<size_t>(B) * (D / m) * nk);
     grow(pl.dlt, pl.cap_dlt, static_cast<size_t>(B) * levels * nk);
     const size_t ncw = static_cast<size_t>(B) * nk;
+    grow(pl.my, pl.cap_my, ncw * levels);
     if (ncw > pl.cap_cw) {
-        size_t c1 = pl.cap_cw, c2 = pl.cap_cw, c3 = pl.cap_cw;
-        grow(pl.my, c1, ncw);
-        grow(pl.myn, c2, ncw);
+        size_t c3 = pl.cap_cw;
         grow(pl.peer, c3, ncw);
         if (pl.h_my) cudaFreeHost(pl.h_my);
         if (pl.h_peer) cudaFreeHost(pl.h_peer);
@@ -586,10 +644,12 @@ void dpf_interactive_convert_device(int B, int n, int w, const Blk* roots, const
     std::lock_guard<std::mutex> lk(pl.mu);
     cudaStream_t st = default_stream();
     const size_t last = static_cast<size_t>(1) << (n - w);   // parents at the last level
-    const int parts = static_cast<int>((last + kTPB - 1) / kTPB);
+    const int per = parents_per_thread(last, B, w, true);
+    const size_t tile = static_cast<size_t>(per) * kTPB;
+    const int parts = static_cast<int>((last + tile - 1) / tile);
     uint64_t* partials = static_cast<uint64_t*>(
         pool_alloc(2 * static_cast<size_t>(B) * parts * sizeof(uint64_t), st));
-    const ConvOut conv{d_conv, partials, dex, dex_user};
+    const ConvOut conv{d_conv, partials, per, parts, dex, dex_user};
     try {
         interactive_eval(B, n, w, roots, dltsft, rks, prg, ex, user, st, pl, &conv);
     } catch (...) {
