@@ -273,6 +273,7 @@ int pcgb_trim_pool(void) {
         cudaStream_t st = pcgb::default_stream();
         PCGB_CK(cudaStreamSynchronize(st));
         PCGB_CK(cudaMemPoolTrimTo(pcgb::library_pool(), 0));
+        pcgb::HostStage::trim();
     });
 }
 
@@ -511,8 +512,10 @@ int pcgb_poly_mul_u64(int variant, uint64_t* out, const uint64_t* a, const uint6
         uint64_t* d = nullptr;
         d = static_cast<uint64_t*>(pcgb::pool_alloc(5 * n * sizeof(uint64_t), st));
         uint64_t *da = d, *db = d + n, *dc = d + 2 * n, *scratch = d + 3 * n;
-        PCGB_CK(cudaMemcpyAsync(da, a, n * 8, cudaMemcpyHostToDevice, st));
-        PCGB_CK(cudaMemcpyAsync(db, b, n * 8, cudaMemcpyHostToDevice, st));
+        pcgb::HostStage io;
+        const void* in[2] = {a, b};
+        const size_t in_len[2] = {n * 8, n * 8};
+        io.upload(d, in, in_len, 2, st);   // db follows da
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         if (device_ms) {
             PCGB_CK(cudaEventCreate(&e0));
@@ -521,9 +524,9 @@ int pcgb_poly_mul_u64(int variant, uint64_t* out, const uint64_t* a, const uint6
         }
         pcgb::poly_mul_device(pl, dc, da, db, batch, scratch, st);
         if (device_ms) PCGB_CK(cudaEventRecord(e1, st));
-        PCGB_CK(cudaMemcpyAsync(out, dc, n * 8, cudaMemcpyDeviceToHost, st));
+        void* res[1] = {out};
+        io.download(res, in_len, 1, dc, st);
         PCGB_CK(cudaFreeAsync(d, st));
-        PCGB_CK(cudaStreamSynchronize(st));
         if (device_ms) {
             float ms = 0;
             PCGB_CK(cudaEventElapsedTime(&ms, e0, e1));

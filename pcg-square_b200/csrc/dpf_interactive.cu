@@ -492,6 +492,10 @@ Blk* run_levels(Pool& pl, int B, int n, const Blk* roots, const Blk* dltsft,
     hash_roots_kernel<W, PRG><<<dim3(1, B), kTPB, smem, st>>>(pl.cur, D, pl.H, HS, pl.my, te, pl.rk);
     PCGB_POST_LAUNCH();
     Blk *cur = pl.cur, *nxt = pl.nxt, *H = pl.H, *Hn = pl.Hn;
+    // Without an exchange the peer's shares are zero on every level, and no
+    // level waits for the host.
+    if (!ex && !(conv && conv->dex))
+        PCGB_CK(cudaMemsetAsync(pl.peer, 0, ncw * sizeof(Blk), st));
     for (int i = 0; i < levels; ++i) {
         Blk *my = pl.my + ncw * i, *myn = my + ncw;   // this level's shares, the next one's
         if (conv && conv->dex) {
@@ -501,16 +505,12 @@ Blk* run_levels(Pool& pl, int B, int n, const Blk* roots, const Blk* dltsft,
             if (conv->dex(reinterpret_cast<const pcgb_blk*>(my), reinterpret_cast<pcgb_blk*>(pl.peer),
                           ncw, conv->dex_user) != 0)
                 fail(PCGB_ECALLBACK, "dpf_gpu_batch_full_eval: device exchange callback failed");
-        } else {
+        } else if (ex) {
             PCGB_CK(cudaMemcpyAsync(pl.h_my, my, ncw * sizeof(Blk), cudaMemcpyDeviceToHost, st));
             PCGB_CK(cudaStreamSynchronize(st));
-            if (ex) {
-                if (ex(reinterpret_cast<const pcgb_blk*>(pl.h_my),
-                       reinterpret_cast<pcgb_blk*>(pl.h_peer), ncw, user) != 0)
-                    fail(PCGB_ECALLBACK, "dpf_gpu_batch_full_eval: exchange callback failed");
-            } else {
-                for (size_t k = 0; k < ncw; ++k) pl.h_peer[k] = Blk{0, 0};
-            }
+            if (ex(reinterpret_cast<const pcgb_blk*>(pl.h_my),
+                   reinterpret_cast<pcgb_blk*>(pl.h_peer), ncw, user) != 0)
+                fail(PCGB_ECALLBACK, "dpf_gpu_batch_full_eval: exchange callback failed");
             PCGB_CK(cudaMemcpyAsync(pl.peer, pl.h_peer, ncw * sizeof(Blk), cudaMemcpyHostToDevice,
                                     st));
         }
@@ -622,9 +622,12 @@ const Blk* dpf_interactive_device(int B, int n, int w, const Blk* roots, const B
     std::lock_guard<std::mutex> lk(pl.mu);
     cudaStream_t st = default_stream();
     Blk* leaves = interactive_eval(B, n, w, roots, dltsft, rks, prg, ex, user, st, pl);
-    if (host_out)
-        PCGB_CK(cudaMemcpyAsync(host_out, leaves, (static_cast<size_t>(B) << n) * sizeof(Blk),
-                                cudaMemcpyDeviceToHost, st));
+    if (host_out) {
+        HostStage io;
+        void* out[1] = {host_out};
+        const size_t out_len[1] = {(static_cast<size_t>(B) << n) * sizeof(Blk)};
+        io.download(out, out_len, 1, leaves, st);
+    }
     PCGB_CK(cudaStreamSynchronize(st));
     return leaves;
 }

@@ -854,15 +854,14 @@ void expand_host(pcgb_expander* e, int party, const Blk* roots, const Blk* cws,
     uint64_t* d_val = d_pos + ct;
     uint64_t* d_x = reinterpret_cast<uint64_t*>(d + in_bytes);
     uint64_t* d_z = d_x + NN;
-    PCGB_CK(cudaMemcpyAsync(d_roots, roots, b_roots, cudaMemcpyHostToDevice, st));
-    PCGB_CK(cudaMemcpyAsync(d_cws, cws, b_cws, cudaMemcpyHostToDevice, st));
-    PCGB_CK(cudaMemcpyAsync(d_cwo, cw_out, b_cwo, cudaMemcpyHostToDevice, st));
-    PCGB_CK(cudaMemcpyAsync(d_pos, pos, b_noise, cudaMemcpyHostToDevice, st));
-    PCGB_CK(cudaMemcpyAsync(d_val, val, b_noise, cudaMemcpyHostToDevice, st));
+    HostStage io;
+    const void* in[5] = {roots, cws, cw_out, pos, val};
+    const size_t in_len[5] = {b_roots, b_cws, b_cwo, b_noise, b_noise};
+    io.upload(d, in, in_len, 5, st);
     expand_device(e, party, d_roots, d_cws, d_cwo, d_pos, d_val, d_x, d_z, st);
-    PCGB_CK(cudaMemcpyAsync(x, d_x, b_out, cudaMemcpyDeviceToHost, st));
-    PCGB_CK(cudaMemcpyAsync(z, d_z, b_out, cudaMemcpyDeviceToHost, st));
-    PCGB_CK(cudaStreamSynchronize(st));
+    void* out[2] = {x, z};
+    const size_t out_len[2] = {b_out, b_out};
+    io.download(out, out_len, 2, d_x, st);   // z follows x
 }
 
 // Step 4 from externally computed output layers (the interactive two-party

@@ -384,9 +384,10 @@ void dpf_out_scatter_host(const Blk* d_leaves, int B, size_t D, int t, int party
     for (auto& v : cw) v %= kP;
     PCGB_CK(cudaMemcpyAsync(pl.cws, cw.data(), B * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     out_gather_launch(d_leaves, B, D, t, party, pl.cws, pl.g, static_cast<size_t>(N), st);
-    PCGB_CK(cudaMemcpyAsync(g_out, pl.g, static_cast<size_t>(N) * sizeof(uint64_t),
-                            cudaMemcpyDeviceToHost, st));
-    PCGB_CK(cudaStreamSynchronize(st));
+    HostStage io;
+    void* out[1] = {g_out};
+    const size_t out_len[1] = {static_cast<size_t>(N) * sizeof(uint64_t)};
+    io.download(out, out_len, 1, pl.g, st);
 }
 
 // Device-pointer form: CWs already on the device (values in [0, p)), g

@@ -54,6 +54,31 @@ inline cudaStream_t as_stream(void* s) {
 // Host-to-device copy that has landed when the call returns: a plain
 // cudaMemcpy from pageable memory may return before its DMA completes, and
 // work on the library's non-blocking streams is not ordered after it.
+// Host buffers to and from the device through a pinned buffer (host_stage.cpp).
+// One object per call: it holds the device's buffer until it goes out of scope
+// (another thread's call then copies directly).  `pieces` host ranges of len
+// bytes each make up one contiguous device range.  upload: the sources may be
+// reused on return.  download: waits for everything queued on the stream,
+// the pieces are complete on return; call it last.
+class HostStage {
+  public:
+    HostStage();
+    ~HostStage();
+    HostStage(const HostStage&) = delete;
+    HostStage& operator=(const HostStage&) = delete;
+    void upload(void* d_dst, const void* const* src, const size_t* len, int pieces,
+                cudaStream_t st);
+    void download(void* const* dst, const size_t* len, int pieces, const void* d_src,
+                  cudaStream_t st);
+    static void trim();   // frees the current device's buffer
+
+  private:
+    struct Impl;
+    Impl* im;
+    bool usable = false;
+    size_t used = 0;                  // bytes of the buffer that copies may still read
+    cudaStream_t pending = nullptr;   // their stream
+};
 void upload_blocking(void* d_dst, const void* src, size_t bytes);
 // Stream-ordered allocation from the library's own per-device pool, which
 // keeps freed memory mapped for the next request (release with
