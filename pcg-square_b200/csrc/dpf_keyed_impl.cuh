@@ -33,6 +33,7 @@
 
 #include "aes128.cuh"
 #include "chacha8.cuh"
+#include "chain.cuh"
 #include "field.cuh"
 #include "synth.h"
 
@@ -187,6 +188,7 @@ __global__ void __launch_bounds__(kTopsBfsThreads) tops_bfs_kernel(
     extern __shared__ __align__(16) uint64_t tops_dsm[];
     AesSmem& aes_s = *reinterpret_cast<AesSmem*>(tops_dsm);
     Blk* sm = reinterpret_cast<Blk*>(PRG == kPrgAes ? static_cast<void*>(&aes_s + 1) : tops_dsm);
+    chain_begin();
     if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
     const size_t key = static_cast<size_t>(blockIdx.x) * G;
     tops_bfs_body<W, PRG>(roots + key, cws + key * levels * NK, min(G, K - static_cast<int>(key)),
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(kTopsBfsThreads) tops_bfs_multi_kernel(
     extern __shared__ __align__(16) uint64_t tops_dsm[];
     AesSmem& aes_s = *reinterpret_cast<AesSmem*>(tops_dsm);
     Blk* sm = reinterpret_cast<Blk*>(PRG == kPrgAes ? static_cast<void*>(&aes_s + 1) : tops_dsm);
+    chain_begin();
     if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
     int j = 0;
     while (j + 1 < njobs && jobs[j + 1].first <= blockIdx.x) ++j;
@@ -247,7 +250,7 @@ __device__ __forceinline__ void tops_walk(const Blk* __restrict__ src, size_t id
     const Blk* kcw = cws + key * static_cast<size_t>(levels) * NK;
     const size_t fan = static_cast<size_t>(1) << (W * nlev);
     Blk* out = dst + key * (per_key_src * fan) + j * fan;
-    const Blk root = ldblk(src + id);
+    const Blk root = ld_chained(src + id);
     if (nlev == 0) { stblk(out, root); return; }
 
     // stack[d][k]: children at relative depth d+1; pos[d]: next child index.
@@ -289,6 +292,7 @@ __global__ void __launch_bounds__(128) expand_tops_kernel(
     constexpr int NK = (1 << W) - 1;
     extern __shared__ __align__(16) uint64_t tops_dsm[];
     AesSmem& aes_s = *reinterpret_cast<AesSmem*>(tops_dsm);
+    chain_begin();
     if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
     const size_t id = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (id >= (static_cast<size_t>(K) << (W * src_lvl))) return;
@@ -329,10 +333,11 @@ template <int D>
 __global__ void __launch_bounds__(128) expand_tops_fixed_kernel(
     const Blk* __restrict__ src, int K, int src_lvl, int levels, const Blk* __restrict__ cws,
     Blk* __restrict__ dst) {
+    chain_begin();
     const size_t id = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (id >= (static_cast<size_t>(K) << src_lvl)) return;
     const size_t key = id >> src_lvl;
-    TopsFixed1<D>::run(ldblk(src + id), cws + key * levels + src_lvl, dst + (id << D), 0);
+    TopsFixed1<D>::run(ld_chained(src + id), cws + key * levels + src_lvl, dst + (id << D), 0);
 }
 
 // One stage of several key groups of different domains in one persistent
@@ -346,6 +351,7 @@ __global__ void __launch_bounds__(128) expand_tops_multi_kernel(
     extern __shared__ __align__(16) uint64_t tops_dsm[];
     AesSmem& aes_s = *reinterpret_cast<AesSmem*>(tops_dsm);
     if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
+    chain_begin();
     for (unsigned long long g = static_cast<unsigned long long>(blockIdx.x) * blockDim.x +
                                 threadIdx.x;
          g < total; g += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
@@ -360,6 +366,7 @@ __global__ void __launch_bounds__(128) expand_tops_multi_kernel(
 template <int D>
 __global__ void __launch_bounds__(128) expand_tops_multi_depth_kernel(
     const TopsJob* __restrict__ jobs, int njobs, unsigned long long total) {
+    chain_begin();
     for (unsigned long long g = static_cast<unsigned long long>(blockIdx.x) * blockDim.x +
                                 threadIdx.x;
          g < total; g += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
@@ -367,7 +374,7 @@ __global__ void __launch_bounds__(128) expand_tops_multi_depth_kernel(
         while (j + 1 < njobs && jobs[j + 1].first <= g) ++j;
         const TopsJob J = jobs[j];
         const size_t id = g - J.first;
-        TopsFixed1<D>::run(ldblk(J.src + id), J.cws + (id >> J.src_lvl) * J.levels + J.src_lvl,
+        TopsFixed1<D>::run(ld_chained(J.src + id), J.cws + (id >> J.src_lvl) * J.levels + J.src_lvl,
                            J.dst + (id << D), 0);
     }
 }
@@ -377,6 +384,7 @@ __global__ void __launch_bounds__(128) expand_tops_multi_depth_kernel(
 // depth, a deeper one the run-time walk.
 __global__ void __launch_bounds__(128) expand_tops_multi_fixed_kernel(
     const TopsJob* __restrict__ jobs, int njobs, unsigned long long total) {
+    chain_begin();
     for (unsigned long long g = static_cast<unsigned long long>(blockIdx.x) * blockDim.x +
                                 threadIdx.x;
          g < total; g += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
@@ -388,7 +396,7 @@ __global__ void __launch_bounds__(128) expand_tops_multi_fixed_kernel(
         switch (J.nlev) {
 #define PCGB_TF(D)                                                          \
     case D:                                                                 \
-        TopsFixed1<D>::run(ldblk(J.src + id), kcw, J.dst + (id << D), 0); \
+        TopsFixed1<D>::run(ld_chained(J.src + id), kcw, J.dst + (id << D), 0); \
         break;
             PCGB_TF(1) PCGB_TF(2) PCGB_TF(3) PCGB_TF(4)
             PCGB_TF(5) PCGB_TF(6) PCGB_TF(7) PCGB_TF(8)
@@ -446,9 +454,10 @@ __global__ void __launch_bounds__(kAesPrmtThreads) expand_tops_prmt_fixed_kernel
     extern __shared__ __align__(16) unsigned char prmt_dsm[];
     __shared__ AesPrmtKeys keys;
     const AesPrmt A = aes_prmt_setup<1>(prmt_dsm, keys, aes_te, aes_rk);
+    chain_begin();
     const size_t total = static_cast<size_t>(K) << src_lvl;
     for (size_t id = prmt_first_id(); id < total; id += static_cast<size_t>(gridDim.x) * blockDim.x)
-        TopsFixedAes<D>::run(ldblk(src + id), cws + (id >> src_lvl) * levels + src_lvl, &A,
+        TopsFixedAes<D>::run(ld_chained(src + id), cws + (id >> src_lvl) * levels + src_lvl, &A,
                              dst + (id << D), 0);
 }
 
@@ -461,6 +470,7 @@ __global__ void __launch_bounds__(kAesPrmtThreads) expand_tops_prmt_kernel(
     extern __shared__ __align__(16) unsigned char prmt_dsm[];
     __shared__ AesPrmtKeys keys;
     const AesPrmt A = aes_prmt_setup<NK>(prmt_dsm, keys, aes_te, aes_rk);
+    chain_begin();
     const size_t total = static_cast<size_t>(K) << (W * src_lvl);
     for (size_t id = prmt_first_id(); id < total; id += static_cast<size_t>(gridDim.x) * blockDim.x)
         tops_walk<W, kPrgAes>(src, id, src_lvl, nlev, levels, cws, &A, dst);
@@ -474,6 +484,7 @@ __global__ void __launch_bounds__(kAesPrmtThreads) expand_tops_multi_prmt_kernel
     extern __shared__ __align__(16) unsigned char prmt_dsm[];
     __shared__ AesPrmtKeys keys;
     const AesPrmt A = aes_prmt_setup<NK>(prmt_dsm, keys, aes_te, aes_rk);
+    chain_begin();
     for (unsigned long long g = prmt_first_id(); g < total;
          g += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
         int j = 0;
@@ -629,7 +640,7 @@ __device__ __forceinline__ void leaf_gather_tile(
         const size_t half = (ent >> 1) & 1;
         c.neg = ((ent & 1) != 0) != (party != 0);
         c.cwo = __ldg(cw_out + key);
-        const Blk node = ldblk(F + key * per_key + (half * bin + o) / S);
+        const Blk node = ld_chained(F + key * per_key + (half * bin + o) / S);
         const Blk* kcw = cws + (key * levels + hl) * NK;
         if constexpr (W == 1) Dfs1<SL, PRG>::run(node, kcw, aes_s, 0, c);
         else DfsM<W, SL, PRG>::run(node, kcw, aes_s, 0, c);
@@ -676,6 +687,7 @@ __global__ void __launch_bounds__(256) leaf_gather_kernel(
     extern __shared__ __align__(16) ulonglong2 acc_s[];
     AesSmem& aes_s = *reinterpret_cast<AesSmem*>(acc_s + blockDim.x * (S + 1));
     if constexpr (PRG == kPrgAes) load_aes_smem(aes_s, aes_te, aes_rk, NK);
+    chain_begin();
     leaf_gather_tile<W, SL, PRG>(F, cws, cw_out, off, entries, q_order, q_slot, t, levels, hl, bin,
                                  N, party, gq, blockIdx.x >> lsplit, blockIdx.y, blockIdx.z,
                                  lsplit, blockIdx.x & ((1u << lsplit) - 1), acc_s, &aes_s);
@@ -701,6 +713,7 @@ __global__ void __launch_bounds__(256) leaf_gather_multi_kernel(
     const LeafJob& J = tab.job[k];
     const unsigned local = b - J.first;
     const unsigned bx = local % J.gx, r = (local / J.gx) % J.gy, z = local / (J.gx * J.gy);
+    chain_begin();
     leaf_gather_tile<W, SL, PRG>(J.F, J.cws, J.cw_out, J.off, J.entries, J.q_order, J.q_slot, J.t,
                                  J.levels, J.hl, J.bin, J.N, J.party, J.gq, bx,
                                  static_cast<int>(r), static_cast<int>(z), lsplit,
@@ -711,6 +724,7 @@ template <int W, int PRG>
 void launch_tops(const Blk* src, int K, int src_lvl, int nlev, int levels, const Blk* cws,
                  const uint32_t* te, const uint32_t* rk, Blk* dst, cudaStream_t st) {
     if (nlev < 0 || nlev >= tops_max_depth<W>()) fail(PCGB_EINVAL, "keyed expansion deeper than the DFS stack");
+    const bool chained = src_lvl > 0;   // level 0 is the first launch of a call
     if (tops_bfs_ok(K, W, src_lvl, nlev)) {
         const int G = tops_bfs_group(K, W, nlev);
         const size_t smem = tops_bfs_smem<PRG>(W, nlev, G);
@@ -736,26 +750,22 @@ void launch_tops(const Blk* src, int K, int src_lvl, int nlev, int levels, const
         PCGB_CK(cudaFuncSetAttribute(expand_tops_prmt_fixed_kernel<D>,                          \
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,               \
                                      static_cast<int>(kAesPrmtSmemBytes)));                     \
-        expand_tops_prmt_fixed_kernel<D><<<aes_prmt_grid(threads), kAesPrmtThreads,             \
-                                           kAesPrmtSmemBytes, st>>>(src, K, src_lvl, levels,    \
-                                                                    cws, te, rk, dst);          \
+        launch({aes_prmt_grid(threads), kAesPrmtThreads, kAesPrmtSmemBytes}, st,                \
+               expand_tops_prmt_fixed_kernel<D>, src, K, src_lvl, levels, cws, te, rk, dst);    \
         break;
                         PCGB_TF(1) PCGB_TF(2) PCGB_TF(3) PCGB_TF(4)
                         PCGB_TF(5) PCGB_TF(6) PCGB_TF(7) PCGB_TF(8)
 #undef PCGB_TF
                         default: break;
                     }
-                    PCGB_POST_LAUNCH();
                     return;
                 }
             }
             PCGB_CK(cudaFuncSetAttribute(expand_tops_prmt_kernel<W>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kAesPrmtSmemBytes)));
-            expand_tops_prmt_kernel<W><<<aes_prmt_grid(threads), kAesPrmtThreads,
-                                         kAesPrmtSmemBytes, st>>>(src, K, src_lvl, nlev, levels,
-                                                                  cws, te, rk, dst);
-            PCGB_POST_LAUNCH();
+            launch({aes_prmt_grid(threads), kAesPrmtThreads, kAesPrmtSmemBytes}, st,
+                   expand_tops_prmt_kernel<W>, src, K, src_lvl, nlev, levels, cws, te, rk, dst);
             return;
         }
     }
@@ -766,21 +776,20 @@ void launch_tops(const Blk* src, int K, int src_lvl, int nlev, int levels, const
             switch (nlev) {
 #define PCGB_TF(D)                                                                            \
     case D:                                                                                   \
-        expand_tops_fixed_kernel<D><<<grid, TPB, 0, st>>>(src, K, src_lvl, levels, cws, dst); \
+        launch({grid, TPB, 0, chained}, st, expand_tops_fixed_kernel<D>, src, K, src_lvl,     \
+               levels, cws, dst);                                                             \
         break;
                 PCGB_TF(1) PCGB_TF(2) PCGB_TF(3) PCGB_TF(4)
                 PCGB_TF(5) PCGB_TF(6) PCGB_TF(7) PCGB_TF(8)
 #undef PCGB_TF
                 default: break;
             }
-            PCGB_POST_LAUNCH();
             return;
         }
     }
     const size_t smem = PRG == kPrgAes ? sizeof(AesSmem) : 0;
-    expand_tops_kernel<W, PRG><<<grid, TPB, smem, st>>>(src, K, src_lvl, nlev, levels, cws, te,
-                                                        rk, dst);
-    PCGB_POST_LAUNCH();
+    launch({grid, TPB, smem, chained}, st, expand_tops_kernel<W, PRG>, src, K, src_lvl, nlev, levels,
+           cws, te, rk, dst);
 }
 
 template <int W, int PRG>
@@ -1009,27 +1018,14 @@ void tops_multi_for_prg(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs
     }
 }
 
-// Launch in clusters of 1 << lsplit CTAs along x (a plain launch for lsplit = 0).
+// After the top walk, in clusters of 1 << lsplit CTAs.
 template <class... P, class... A>
 void launch_split(void (*kern)(P...), dim3 grid, int tpb, size_t smem, int lsplit, cudaStream_t st,
                   const A&... args) {
     if (smem > 48 * 1024)
         PCGB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(static_cast<unsigned>(tpb));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 1u << lsplit;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = lsplit > 0 ? 1 : 0;
-    PCGB_CK(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
-    PCGB_POST_LAUNCH();
+    launch({grid, dim3(static_cast<unsigned>(tpb)), smem, true, 1u << lsplit}, st, kern, args...);
 }
 
 template <int W, int SL, int PRG>

@@ -22,6 +22,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "field.cuh"
 #include "synth.h"
 
@@ -88,7 +89,11 @@ __global__ void x_kernel(const uint64_t* __restrict__ pos, const uint64_t* __res
                          const uint64_t* __restrict__ aR, int c, int t, int i0, size_t N,
                          uint64_t* __restrict__ x) {
     extern __shared__ uint64_t nz[];
+    // x depends only on the call's inputs: it fills what the leaf kernel's last
+    // wave leaves free, and waits for it at the end.
+    chain_release();
     x_body(pos, val, aR, c, t, i0, N, x, blockIdx.x, nz);
+    chain_wait();
 }
 
 // x of several expansions in one launch: CTA b runs block b - first of the
@@ -104,10 +109,12 @@ struct XJob {
 };
 __global__ void x_multi_kernel(const XJob* __restrict__ jobs, int njobs) {
     extern __shared__ uint64_t nz[];
+    chain_release();   // as x_kernel
     int k = 0;
     while (k + 1 < njobs && jobs[k + 1].first <= blockIdx.x) ++k;
     const XJob& J = jobs[k];
     x_body(J.pos, J.val, J.aR, J.c, J.t, J.i0, J.N, J.x, blockIdx.x - J.first, nz);
+    chain_wait();
 }
 
 // Digests of several vectors in one launch: job k covers CTAs
@@ -140,6 +147,7 @@ __global__ void digest_multi_kernel(const DigestJob* __restrict__ jobs, unsigned
 // c*c per-block output-layer vectors g[(i*c + j)*N ..] (each in [0, p)).
 __global__ void pair_merge_kernel(const uint64_t* __restrict__ g, int c, size_t N,
                                   uint64_t* __restrict__ gq) {
+    chain_begin();
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int q = blockIdx.y;
     if (idx >= N) return;
@@ -387,8 +395,8 @@ void expand_device_ws(pcgb_expander* e, const Workspace& ws, int party, const Bl
     keyed_leaf_gather(e->gp, party, e->prg, ws.F, cws, cw_out, e->d_rk, ws.g, st);
     if (ev) PCGB_CK(cudaEventRecord(ev[2], st));
     const size_t sm = sizeof(uint64_t) * 2 * static_cast<size_t>(e->c) * e->t;
-    x_kernel<<<blocks_for(NN, 256), 256, sm, st>>>(pos, val, e->d_aR, e->c, e->t, e->i0, NN, x);
-    PCGB_POST_LAUNCH();
+    launch({blocks_for(NN, 256), 256, sm, true}, st, x_kernel, pos, val, e->d_aR, e->c, e->t, e->i0,
+           NN, x);
     if (ev) PCGB_CK(cudaEventRecord(ev[3], st));
     if (e->gp.Qs > 0) ntt_mac_inverse(*e->ntt, ws.g, e->d_img, e->gp.Qs, z, st);
     else PCGB_CK(cudaMemsetAsync(z, 0, sizeof(uint64_t) * NN, st));   // a shard with no pairs
@@ -477,8 +485,7 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
         while (lsplit > 0 && (2 * e[i]->t >> lsplit) < 2) --lsplit;
     keyed_leaf_multi_chacha(w, sl, leaf.data(), count, lsplit, tpb, leaf_smem, nullptr, nullptr, st);
     // Stage 3: the sparse x products.
-    x_multi_kernel<<<x_ctas, 256, x_smem, st>>>(reinterpret_cast<const XJob*>(tab), count);
-    PCGB_POST_LAUNCH();
+    launch({x_ctas, 256, x_smem, true}, st, x_multi_kernel, reinterpret_cast<const XJob*>(tab), count);
     // Stage 4: NTT multiply-accumulate and inverse, all lengths at once.
     std::vector<uint64_t*> g(count), zz(count);
     std::vector<const uint64_t*> img(count);
@@ -876,8 +883,8 @@ void expand_from_g_device(pcgb_expander* e, const uint64_t* g, const uint64_t* p
     pair_merge_kernel<<<dim3(blocks_for(NN, 256), e->Q), 256, 0, st>>>(g, e->c, NN, e->d_g);
     PCGB_POST_LAUNCH();
     const size_t sm = sizeof(uint64_t) * 2 * static_cast<size_t>(e->c) * e->t;
-    x_kernel<<<blocks_for(NN, 256), 256, sm, st>>>(pos, val, e->d_aR, e->c, e->t, e->i0, NN, x);
-    PCGB_POST_LAUNCH();
+    launch({blocks_for(NN, 256), 256, sm, true}, st, x_kernel, pos, val, e->d_aR, e->c, e->t, e->i0,
+           NN, x);
     ntt_mac_inverse(*e->ntt, e->d_g, e->d_img, e->Q, z, st);
 }
 

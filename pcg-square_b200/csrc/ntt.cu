@@ -64,6 +64,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "chain.cuh"
 #include "field.cuh"
 #include "ntt_arith.cuh"
 
@@ -458,6 +459,7 @@ template <int L, int C, int DL>
 __global__ void __launch_bounds__(col_threads<L, C>(), col_min_ctas<L, C>())
     col_fwd_kernel(const FwdIn in, const NttTw* __restrict__ tw) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const size_t off = static_cast<size_t>(blockIdx.y) << (2 * L + DL);
     const int z = blockIdx.z;
     const uint64_t* add = pick(in.add, z);
@@ -469,6 +471,7 @@ template <int L, int C, int DL>
 __global__ void __launch_bounds__(col_threads<L, C>(), col_min_ctas<L, C>())
     col_inv_kernel(uint64_t* d, const NttTw* __restrict__ twi) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     col_inv_body<L, C, L + DL>(d + (static_cast<size_t>(blockIdx.y) << (2 * L + DL)), blockIdx.x,
                                twi, sm);
 }
@@ -493,6 +496,7 @@ __global__ void __launch_bounds__(row_threads<L>(), row_min_ctas<L>()) row_fwd_k
     const FwdIn in, const uint64_t* __restrict__ img, int batch, int l1,
     const NttTw* __restrict__ tw, const NttTw* __restrict__ Wf) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const int t = threadIdx.x % Geo<L>::T, v = threadIdx.x / Geo<L>::T, z = blockIdx.z;
     const RowAt r = row_at<L, DIRECT>(batch);
     const size_t off = (r.inst << (L + l1)) + r.base;
@@ -508,6 +512,7 @@ __global__ void __launch_bounds__(row_threads<L>(), row_min_ctas<L>()) row_inv_k
     const uint64_t* g, const uint64_t* img, int Q, int batch, int l1,
     const NttTw* __restrict__ twi, const NttTw* __restrict__ Wif, uint64_t* out) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const int t = threadIdx.x % Geo<L>::T, v = threadIdx.x / Geo<L>::T;
     const RowAt r = row_at<L, DIRECT>(batch);
     const size_t N = size_t{1} << (L + l1);
@@ -634,6 +639,7 @@ struct MixedRow {
 __global__ void __launch_bounds__(kMixedColThreads, 2) mixed_col_fwd_kernel(
     const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas, int first) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
     const bool which = first + blockIdx.y != 0;
@@ -649,6 +655,7 @@ __global__ void __launch_bounds__(kMixedColThreads, 2) mixed_col_fwd_kernel(
 __global__ void __launch_bounds__(kMixedRowThreads) mixed_row_fwd_kernel(
     const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
     uint64_t* d = blockIdx.y ? p.c : p.A;
@@ -661,6 +668,7 @@ __global__ void __launch_bounds__(kMixedRowThreads) mixed_row_fwd_kernel(
 __global__ void __launch_bounds__(kMixedRowThreads) mixed_row_mul_kernel(
     const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
 #define PCGB_CALL(LL) \
@@ -672,6 +680,7 @@ __global__ void __launch_bounds__(kMixedRowThreads) mixed_row_mul_kernel(
 __global__ void __launch_bounds__(kMixedColThreads, 2) mixed_col_inv_kernel(
     const MixedPoly* __restrict__ polys, const MixedCta* __restrict__ ctas) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const MixedCta j = ctas[blockIdx.x];
     const MixedPoly& p = polys[j.poly];
 #define PCGB_CALL(LL, L2) col_inv_body<LL, mixed_C<LL>(), L2>(p.c, j.tile, p.tw1i, sm)
@@ -731,6 +740,7 @@ static_assert(sizeof(uint64_t) * Geo<7>::PAD * mixed_C<7>() == kMixedColSmem &&
 __global__ void __launch_bounds__(kMixedColThreads, 2) mac_col_fwd_kernel(
     const MacReq* __restrict__ reqs, const MacCta* __restrict__ ctas) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const MacCta j = ctas[blockIdx.x];
     const MacReq& r = reqs[j.req];
     uint64_t* d = r.g + (static_cast<size_t>(j.q) << (r.l1 + r.l2));
@@ -742,6 +752,7 @@ __global__ void __launch_bounds__(kMixedColThreads, 2) mac_col_fwd_kernel(
 __global__ void __launch_bounds__(kMixedRowThreads) mac_row_fwd_kernel(
     const MacReq* __restrict__ reqs, const MacCta* __restrict__ ctas) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const MacCta j = ctas[blockIdx.x];
     const MacReq& r = reqs[j.req];
     const size_t off = static_cast<size_t>(j.q) << (r.l1 + r.l2);
@@ -754,6 +765,7 @@ __global__ void __launch_bounds__(kMixedRowThreads) mac_row_fwd_kernel(
 __global__ void __launch_bounds__(kMixedRowThreads) mac_row_inv_kernel(
     const MacReq* __restrict__ reqs, const MacCta* __restrict__ ctas) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const MacCta j = ctas[blockIdx.x];
     const MacReq& r = reqs[j.req];
     const size_t N = size_t{1} << (r.l1 + r.l2);
@@ -766,6 +778,7 @@ __global__ void __launch_bounds__(kMixedRowThreads) mac_row_inv_kernel(
 __global__ void __launch_bounds__(kMixedColThreads, 2) mac_col_inv_kernel(
     const MacReq* __restrict__ reqs, const MacCta* __restrict__ ctas) {
     extern __shared__ int64_t sm[];
+    chain_begin();
     const MacCta j = ctas[blockIdx.x];
     const MacReq& r = reqs[j.req];
 #define PCGB_CALL(LL, L2) col_inv_body<LL, mixed_C<LL>(), L2>(r.z, j.tile, r.tw1i, sm)
@@ -968,17 +981,18 @@ void col_width(size_t work, F&& f) {
 }
 
 template <int L>
-void col_fwd_l(const NttPlan& pl, const FwdIn& in, int count, int batch, cudaStream_t st) {
+void col_fwd_l(const NttPlan& pl, const FwdIn& in, int count, int batch, bool chained,
+               cudaStream_t st) {
     col_width<L>(static_cast<size_t>(pl.n2) * batch * count, [&](auto CC) {
         constexpr int C = decltype(CC)::value;
         constexpr size_t sm = col_smem<L, C>();
         auto go = [&](auto kernel) {
             g_optin(kernel, sm);
-            kernel<<<dim3(pl.n2 / C, batch, count), col_threads<L, C>(), sm, st>>>(in, pl.tw1);
+            launch({dim3(pl.n2 / C, batch, count), col_threads<L, C>(), sm, chained}, st, kernel, in,
+                   pl.tw1);
         };
         pl.l2 != L ? go(col_fwd_kernel<L, C, 1>) : go(col_fwd_kernel<L, C, 0>);
     });
-    PCGB_POST_LAUNCH();
 }
 
 template <int L>
@@ -988,11 +1002,10 @@ void col_inv_l(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
         constexpr size_t sm = col_smem<L, C>();
         auto go = [&](auto kernel) {
             g_optin(kernel, sm);
-            kernel<<<dim3(pl.n2 / C, batch), col_threads<L, C>(), sm, st>>>(d, pl.tw1i);
+            launch({dim3(pl.n2 / C, batch), col_threads<L, C>(), sm, true}, st, kernel, d, pl.tw1i);
         };
         pl.l2 != L ? go(col_inv_kernel<L, C, 1>) : go(col_inv_kernel<L, C, 0>);
     });
-    PCGB_POST_LAUNCH();
 }
 
 // Grid of a row pass: V rows of one polynomial per CTA, or (direct plans) V
@@ -1005,12 +1018,12 @@ dim3 row_grid(const NttPlan& pl, int batch, int count) {
 
 template <int L>
 void row_fwd_l(const NttPlan& pl, const FwdIn& in, const uint64_t* img, int count, int batch,
-               RowOut out, cudaStream_t st) {
+               RowOut out, bool chained, cudaStream_t st) {
     constexpr size_t sm = row_smem<L>();
     auto go = [&](auto kernel) {
         g_optin(kernel, sm);
-        kernel<<<row_grid<L>(pl, batch, count), row_threads<L>(), sm, st>>>(in, img, batch, pl.l1,
-                                                                           pl.tw2, pl.Wf);
+        launch({row_grid<L>(pl, batch, count), row_threads<L>(), sm, chained}, st, kernel, in, img,
+               batch, pl.l1, pl.tw2, pl.Wf);
     };
     auto by_out = [&](auto D) {
         constexpr bool d = decltype(D)::value;
@@ -1024,7 +1037,6 @@ void row_fwd_l(const NttPlan& pl, const FwdIn& in, const uint64_t* img, int coun
     if constexpr (L > kDirectLogN / 2) {
         if (!pl.direct()) by_out(std::false_type{});
     }
-    PCGB_POST_LAUNCH();
 }
 
 template <int L>
@@ -1033,8 +1045,8 @@ void row_inv_l(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q,
     constexpr size_t sm = row_smem<L>();
     auto go = [&](auto kernel) {
         g_optin(kernel, sm);
-        kernel<<<row_grid<L>(pl, batch, 1), row_threads<L>(), sm, st>>>(g, img, Q, batch, pl.l1,
-                                                                       pl.tw2i, pl.Wif, out);
+        launch({row_grid<L>(pl, batch, 1), row_threads<L>(), sm, true}, st, kernel, g, img, Q, batch,
+               pl.l1, pl.tw2i, pl.Wif, out);
     };
     if constexpr (L <= kDirectLogN) {
         if (pl.direct()) go(row_inv_kernel<L, true, true>);   // products run as one launch
@@ -1042,7 +1054,6 @@ void row_inv_l(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q,
     if constexpr (L > kDirectLogN / 2) {
         if (!pl.direct()) img ? go(row_inv_kernel<L, false, false>) : go(row_inv_kernel<L, false, true>);
     }
-    PCGB_POST_LAUNCH();
 }
 
 template <int L>
@@ -1090,16 +1101,21 @@ void by_col_len(int L, F&& f) {
     }
 }
 
-void col_fwd(const NttPlan& pl, const FwdIn& in, int count, int batch, cudaStream_t st) {
-    by_col_len(pl.l1, [&](auto L) { col_fwd_l<decltype(L)::value>(pl, in, count, batch, st); });
+// chained: a kernel of the same call precedes this one on the stream
+// (chain.cuh).  The inverse passes always have one.
+void col_fwd(const NttPlan& pl, const FwdIn& in, int count, int batch, bool chained,
+             cudaStream_t st) {
+    by_col_len(pl.l1,
+               [&](auto L) { col_fwd_l<decltype(L)::value>(pl, in, count, batch, chained, st); });
 }
 void col_inv(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
     by_col_len(pl.l1, [&](auto L) { col_inv_l<decltype(L)::value>(pl, d, batch, st); });
 }
 void row_fwd(const NttPlan& pl, const FwdIn& in, const uint64_t* img, int count, int batch,
-             RowOut out, cudaStream_t st) {
-    by_len(pl.l2,
-           [&](auto L) { row_fwd_l<decltype(L)::value>(pl, in, img, count, batch, out, st); });
+             RowOut out, bool chained, cudaStream_t st) {
+    by_len(pl.l2, [&](auto L) {
+        row_fwd_l<decltype(L)::value>(pl, in, img, count, batch, out, chained, st);
+    });
 }
 // Sum of Q products (img null), or the product g (.) img.
 void row_inv(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, int batch,
@@ -1111,15 +1127,15 @@ void row_inv(const NttPlan& pl, const uint64_t* g, const uint64_t* img, int Q, i
 // from src (plus add) to dst and the row pass in place, or the single row
 // pass of a direct plan.  out and img as for row_fwd_body.
 void forward(const NttPlan& pl, const FwdIn& in, const uint64_t* img, int count, int batch,
-             RowOut out, cudaStream_t st) {
+             RowOut out, bool chained, cudaStream_t st) {
     if (pl.direct()) {
-        row_fwd(pl, in, img, count, batch, out, st);
+        row_fwd(pl, in, img, count, batch, out, chained, st);
         return;
     }
-    col_fwd(pl, in, count, batch, st);
+    col_fwd(pl, in, count, batch, chained, st);
     FwdIn rows;
     for (int z = 0; z < count; ++z) rows.src[z] = rows.dst[z] = in.dst[z];
-    row_fwd(pl, rows, img, count, batch, out, st);
+    row_fwd(pl, rows, img, count, batch, out, true, st);
 }
 
 FwdIn fwd_one(const uint64_t* src, uint64_t* dst) {
@@ -1162,7 +1178,7 @@ void ntt_forward3(const NttPlan& pl, const uint64_t* const (&src)[3],
         in.add[z] = add[z];
         in.dst[z] = dst[z];
     }
-    forward(pl, in, nullptr, 3, 1, kRowCanon, st);
+    forward(pl, in, nullptr, 3, 1, kRowCanon, false, st);
 }
 
 void ntt_log_sizes(const NttPlan& pl, int* l1, int* l2) {
@@ -1171,7 +1187,7 @@ void ntt_log_sizes(const NttPlan& pl, int* l1, int* l2) {
 }
 
 void ntt_forward(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
-    forward(pl, fwd_one(d, d), nullptr, 1, batch, kRowCanon, st);
+    forward(pl, fwd_one(d, d), nullptr, 1, batch, kRowCanon, false, st);
 }
 
 // Per device: a second stream and two events for the two-half schedule of
@@ -1205,12 +1221,12 @@ void poly_mul_device(const NttPlan& pl, uint64_t* c, const uint64_t* a, const ui
         const uint64_t *x = a + first, *y = b + first;
         const size_t n = static_cast<size_t>(count) * pl.N;
         if (overlap(C, n, x, n)) {
-            col_fwd(pl, fwd_one(x, A), 1, count, s);
-            col_fwd(pl, fwd_one(y, C), 1, count, s);
+            col_fwd(pl, fwd_one(x, A), 1, count, false, s);
+            col_fwd(pl, fwd_one(y, C), 1, count, true, s);
         } else {
-            col_fwd(pl, fwd_two(x, A, y, C), 2, count, s);
+            col_fwd(pl, fwd_two(x, A, y, C), 2, count, false, s);
         }
-        row_fwd(pl, fwd_two(A, A, C, C), nullptr, 2, count, kRowLazy, s);
+        row_fwd(pl, fwd_two(A, A, C, C), nullptr, 2, count, kRowLazy, true, s);
         row_inv(pl, C, A, 1, count, C, s);
         col_inv(pl, C, count, s);
     };
@@ -1315,23 +1331,20 @@ void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const*
     g_optin(mixed_row_fwd_kernel, kMixedRowSmem);
     g_optin(mixed_row_mul_kernel, kMixedRowSmem);
     for (int first = 0; first < (alias ? 2 : 1); ++first) {
-        mixed_col_fwd_kernel<<<dim3(n_col, alias ? 1 : 2), kMixedColThreads, kMixedColSmem, st>>>(
-            d_polys, d_col, first);
-        PCGB_POST_LAUNCH();
+        launch({dim3(n_col, alias ? 1 : 2), kMixedColThreads, kMixedColSmem, first > 0}, st,
+               mixed_col_fwd_kernel, d_polys, d_col, first);
     }
-    mixed_row_fwd_kernel<<<dim3(n_row, 2), kMixedRowThreads, kMixedRowSmem, st>>>(d_polys, d_row);
-    PCGB_POST_LAUNCH();
-    mixed_row_mul_kernel<<<n_row, kMixedRowThreads, kMixedRowSmem, st>>>(d_polys, d_row);
-    PCGB_POST_LAUNCH();
-    mixed_col_inv_kernel<<<n_col, kMixedColThreads, kMixedColSmem, st>>>(d_polys, d_col);
-    PCGB_POST_LAUNCH();
+    launch({dim3(n_row, 2), kMixedRowThreads, kMixedRowSmem, true}, st, mixed_row_fwd_kernel, d_polys,
+           d_row);
+    launch({n_row, kMixedRowThreads, kMixedRowSmem, true}, st, mixed_row_mul_kernel, d_polys, d_row);
+    launch({n_col, kMixedColThreads, kMixedColSmem, true}, st, mixed_col_inv_kernel, d_polys, d_col);
     PCGB_CK(cudaFreeAsync(tab, st));
     PCGB_CK(cudaFreeAsync(scratch, st));
 }
 
 void ntt_mac_inverse(const NttPlan& pl, uint64_t* g, const uint64_t* img, int Q, uint64_t* acc,
                      cudaStream_t st) {
-    forward(pl, fwd_one(g, g), img, 1, Q, kRowTimes, st);
+    forward(pl, fwd_one(g, g), img, 1, Q, kRowTimes, true, st);
     row_inv(pl, g, nullptr, Q, 1, acc, st);
     if (!pl.direct()) col_inv(pl, acc, 1, st);
 }
@@ -1399,14 +1412,10 @@ void ntt_mac_inverse_multi(int count, uint64_t* const* g, const uint64_t* const*
     g_optin(mac_row_fwd_kernel, kMixedRowSmem);
     g_optin(mac_row_inv_kernel, kMixedRowSmem);
     g_optin(mac_col_inv_kernel, kMixedColSmem);
-    mac_col_fwd_kernel<<<grid(0), kMixedColThreads, kMixedColSmem, st>>>(d_req, ctas(0));
-    PCGB_POST_LAUNCH();
-    mac_row_fwd_kernel<<<grid(1), kMixedRowThreads, kMixedRowSmem, st>>>(d_req, ctas(1));
-    PCGB_POST_LAUNCH();
-    mac_row_inv_kernel<<<grid(2), kMixedRowThreads, kMixedRowSmem, st>>>(d_req, ctas(2));
-    PCGB_POST_LAUNCH();
-    mac_col_inv_kernel<<<grid(3), kMixedColThreads, kMixedColSmem, st>>>(d_req, ctas(3));
-    PCGB_POST_LAUNCH();
+    launch({grid(0), kMixedColThreads, kMixedColSmem}, st, mac_col_fwd_kernel, d_req, ctas(0));
+    launch({grid(1), kMixedRowThreads, kMixedRowSmem, true}, st, mac_row_fwd_kernel, d_req, ctas(1));
+    launch({grid(2), kMixedRowThreads, kMixedRowSmem, true}, st, mac_row_inv_kernel, d_req, ctas(2));
+    launch({grid(3), kMixedColThreads, kMixedColSmem, true}, st, mac_col_inv_kernel, d_req, ctas(3));
     PCGB_CK(cudaFreeAsync(tab, st));
 }
 

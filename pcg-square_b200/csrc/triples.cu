@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <string>
 
+#include "chain.cuh"
 #include "field.cuh"
 #include "ntt_layout.cuh"
 
@@ -37,26 +38,27 @@ __global__ void add_reduce_kernel(uint64_t* d, const uint64_t* u, const uint64_t
 
 // Slot k of the outputs: a = A, b = B, c = A*B + S at the transform
 // position of slot k (A, B, S transformed, values in [0, p)).
-__global__ void triple_slots_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
-                                    const uint64_t* __restrict__ S, size_t n, int l1, int l2,
-                                    uint64_t r2, uint64_t* a, uint64_t* b, uint64_t* c) {
+__global__ void triple_slots_kernel(const uint64_t* A, const uint64_t* B, const uint64_t* S,
+                                    size_t n, int l1, int l2, uint64_t r2, uint64_t* a, uint64_t* b,
+                                    uint64_t* c) {
+    chain_begin();
     const size_t k = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const size_t s = ntt_slot_position(k, l1, l2);
-    const uint64_t x = __ldg(A + s), y = __ldg(B + s);
+    const uint64_t x = ld_chained(A + s), y = ld_chained(B + s), v = ld_chained(S + s);
     a[k] = x;
     b[k] = y;
-    c[k] = add_p(mont_mul(mont_mul(x, y), r2), __ldg(S + s));
+    c[k] = add_p(mont_mul(mont_mul(x, y), r2), v);
 }
 
 // Counts slots where X0*X1 != Z (all transformed, in [0, p)).
-__global__ void ole_check_kernel(const uint64_t* __restrict__ X0, const uint64_t* __restrict__ X1,
-                                 const uint64_t* __restrict__ Z, size_t n, uint64_t r2,
-                                 unsigned long long* bad) {
+__global__ void ole_check_kernel(const uint64_t* X0, const uint64_t* X1, const uint64_t* Z,
+                                 size_t n, uint64_t r2, unsigned long long* bad) {
+    chain_begin();
     unsigned long long mine = 0;
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<size_t>(gridDim.x) * blockDim.x)
-        mine += mont_mul(mont_mul(X0[i], X1[i]), r2) != Z[i];
+        mine += mont_mul(mont_mul(ld_chained(X0 + i), ld_chained(X1 + i)), r2) != ld_chained(Z + i);
     for (int o = 16; o; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
     if ((threadIdx.x & 31) == 0 && mine) atomicAdd(bad, mine);
 }
@@ -109,9 +111,8 @@ void triples_device(int N, int party, const uint64_t* x1, const uint64_t* z1, co
     uint64_t* T = static_cast<uint64_t*>(pool_alloc(3 * n * sizeof(uint64_t), st));  // A | B | S
     ntt_forward3(pl, {party == 0 ? x1 : x2, party == 0 ? x2 : x1, z1}, {nullptr, nullptr, z2},
                  {T, T + n, T + 2 * n}, st);
-    triple_slots_kernel<<<grid_for(n), kTpb, 0, st>>>(T, T + n, T + 2 * n, n, l1, l2, r2_mod_p(),
-                                                      a, b, c);
-    PCGB_POST_LAUNCH();
+    launch({grid_for(n), kTpb, 0, true}, st, triple_slots_kernel, T, T + n, T + 2 * n, n, l1, l2,
+           r2_mod_p(), a, b, c);
     PCGB_CK(cudaFreeAsync(T, st));
 }
 
@@ -123,8 +124,8 @@ void verify_ole_device(int N, const uint64_t* x0, const uint64_t* z0, const uint
     uint64_t* T = static_cast<uint64_t*>(pool_alloc(3 * n * sizeof(uint64_t), st));  // X0 | X1 | Z
     PCGB_CK(cudaMemsetAsync(bad, 0, sizeof(unsigned long long), st));
     ntt_forward3(pl, {x0, x1, z0}, {nullptr, nullptr, z1}, {T, T + n, T + 2 * n}, st);
-    ole_check_kernel<<<check_grid(n), kTpb, 0, st>>>(T, T + n, T + 2 * n, n, r2_mod_p(), bad);
-    PCGB_POST_LAUNCH();
+    launch({check_grid(n), kTpb, 0, true}, st, ole_check_kernel, T, T + n, T + 2 * n, n, r2_mod_p(),
+           bad);
     PCGB_CK(cudaFreeAsync(T, st));
 }
 
