@@ -22,6 +22,7 @@
 
 #include "aes128.cuh"
 #include "chacha8.cuh"
+#include "chain.cuh"
 #include "field.cuh"
 
 namespace pcgb {
@@ -186,8 +187,18 @@ __global__ void __launch_bounds__(kTPB) expand_level_kernel(
         kids[NK] = Blk{xl ^ p.lo ^ (t ? cwf.lo : 0), xh ^ p.hi ^ (t ? cwf.hi : 0)};
         Blk* dst = nxt + static_cast<size_t>(b) * D + j * M;
 #pragma unroll
-        for (int k = 0; k < M; ++k) dst[k] = kids[k];
+        for (int k = 0; k < M; k += 2) st_pair(dst + k, kids[k], kids[k + 1], true);
         if (hash_next) {
+            if constexpr (PRG == PCGB_PRG_CHACHA8 && W == 1) {
+                // Both children's blocks in flight, their hashes one store.
+                Blk h0[NK], h1[NK];
+                hash_node<W, PRG>(kids[0], a, h0);
+                hash_node<W, PRG>(kids[1], a, h1);
+                st_pair(Hn + static_cast<size_t>(b) * HS + j * M, h0[0], h1[0], true);
+                acc[0].lo ^= h0[0].lo ^ h1[0].lo;
+                acc[0].hi ^= h0[0].hi ^ h1[0].hi;
+                return;
+            }
             auto hash_child = [&](int k) {
                 Blk h[NK];
                 hash_node<W, PRG>(kids[k], a, h);
@@ -289,15 +300,14 @@ __global__ void __launch_bounds__(kPrmtTPB) expand_level_prmt_kernel(
             kids[NK] = Blk{xl ^ p.lo ^ (t ? cwf.lo : 0), xh ^ p.hi ^ (t ? cwf.hi : 0)};
             Blk* dst = nxt + b * D + j * M;
 #pragma unroll
-            for (int k = 0; k < M; ++k) dst[k] = kids[k];
+            for (int k = 0; k < M; k += 2) st_pair(dst + k, kids[k], kids[k + 1], true);
             if (hash_next) {
                 if constexpr (W == 1) {
                     // Both children's hashes in flight at once.
                     Blk h0, h1;
                     aes_ccr_prmt(A, 0, kids[0].lo, kids[0].hi, h0.lo, h0.hi);
                     aes_ccr_prmt(A, 0, kids[1].lo, kids[1].hi, h1.lo, h1.hi);
-                    Hn[b * HS + j * 2] = h0;
-                    Hn[b * HS + j * 2 + 1] = h1;
+                    st_pair(Hn + b * HS + j * 2, h0, h1, true);
                     acc[0].lo ^= h0.lo ^ h1.lo;
                     acc[0].hi ^= h0.hi ^ h1.hi;
                 } else {
@@ -440,6 +450,10 @@ __global__ void seed_kernel(Blk* my, const Blk* dlt, int B, int levels, int nk) 
     my[i] = dlt[(r / nk * levels + level) * nk + r % nk];
 }
 
+// The node and hash arrays are allocations of their own and an instance's part
+// of each has an even number of nodes wherever pairs are written (D = 2^n, and
+// HS = D / 2 >= 2 for w = 1 when there is a next level), so the kernels' pairs
+// are 32-byte aligned.
 struct Pool {
     Blk *cur = nullptr, *nxt = nullptr, *H = nullptr, *Hn = nullptr, *dlt = nullptr;
     Blk *my = nullptr, *peer = nullptr;     // my: [levels][B][nk]

@@ -252,6 +252,7 @@ __device__ __forceinline__ void tops_walk(const Blk* __restrict__ src, size_t id
     Blk* out = dst + key * (per_key_src * fan) + j * fan;
     const Blk root = ld_chained(src + id);
     if (nlev == 0) { stblk(out, root); return; }
+    const bool wide = pair_aligned(dst);   // every subtree starts at an even node
 
     // stack[d][k]: children at relative depth d+1; pos[d]: next child index.
     Blk stack[MAXD][M];
@@ -263,7 +264,8 @@ __device__ __forceinline__ void tops_walk(const Blk* __restrict__ src, size_t id
     while (d >= 0) {
         if (d == nlev - 1) {
 #pragma unroll
-            for (int k = 0; k < M; ++k) stblk(out + emitted + k, stack[d][k]);
+            for (int k = 0; k < M; k += 2)
+                st_pair(out + emitted + k, stack[d][k], stack[d][k + 1], wide);
             emitted += M;
             --d;
             if (d >= 0) ++pos[d];
@@ -427,18 +429,17 @@ template <int D, int LV = 0>
 struct TopsFixedAes {
     __device__ __forceinline__ static void run(const Blk& node, const Blk* __restrict__ cw,
                                                const AesPrmt* aes, Blk* __restrict__ out,
-                                               unsigned u) {
+                                               unsigned u, bool wide) {
         Blk k2[2];
         children<1, kPrgAes>(node, cw + LV, aes, k2);
         if constexpr (D == 1) {
-            stblk(out + u, k2[0]);
-            stblk(out + u + 1, k2[1]);
+            st_pair(out + u, k2[0], k2[1], wide);
         } else {
             Blk cur = k2[0];
             const Blk R = k2[1];
 #pragma unroll 1
             for (unsigned i = 0; i < 2; ++i) {
-                TopsFixedAes<D - 1, LV + 1>::run(cur, cw, aes, out, u + (i << (D - 1)));
+                TopsFixedAes<D - 1, LV + 1>::run(cur, cw, aes, out, u + (i << (D - 1)), wide);
                 cur = R;
             }
         }
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(kAesPrmtThreads) expand_tops_prmt_fixed_kernel
     const size_t total = static_cast<size_t>(K) << src_lvl;
     for (size_t id = prmt_first_id(); id < total; id += static_cast<size_t>(gridDim.x) * blockDim.x)
         TopsFixedAes<D>::run(ld_chained(src + id), cws + (id >> src_lvl) * levels + src_lvl, &A,
-                             dst + (id << D), 0);
+                             dst + (id << D), 0, pair_aligned(dst));
 }
 
 template <int W>

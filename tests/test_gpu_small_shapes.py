@@ -44,3 +44,25 @@ def test_breadth_first_walk(pcg, prg, K, n, w):
     d_r, d_c = dev(pcg, roots), dev(pcg, cws)
     pcg.dpf_keyed_full_eval_device(K, n, w, prg, d_r.ptr, d_c.ptr, out.ptr, round_keys=rks)
     assert (out.download(np.uint64, 2 * (K << n)) == want).all()
+
+
+@pytest.mark.parametrize("prg", [O.PRG_CHACHA8, O.PRG_AES])
+@pytest.mark.parametrize("K,n,w", [(300, 12, 1), (160, 12, 2), (5, 3, 1)])
+def test_leaves_at_a_16_byte_address(pcg, prg, K, n, w):
+    """A leaf buffer aligned to a node but not to a pair of them."""
+    nk = (1 << w) - 1
+    rng = np.random.default_rng(K + n)
+    roots = rng.integers(0, 2**64 - 1, (K, 2), dtype=np.uint64)
+    cws = rng.integers(0, 2**64 - 1, (K * (n // w) * nk, 2), dtype=np.uint64)
+    rks = O.aes_tree_round_keys(np.arange(16, dtype=np.uint8), nk) if prg == O.PRG_AES else None
+    out = pcg.DeviceBuffer((16 * K << n) + 32)
+    d_r, d_c = dev(pcg, roots), dev(pcg, cws)
+    words = []
+    for off in (0, 16):
+        pcg.dpf_keyed_full_eval_device(K, n, w, prg, d_r.ptr, d_c.ptr, out.ptr + off,
+                                       round_keys=rks)
+        pcg.synchronize()
+        words.append(out.download(np.uint64, (2 * K << n) + 2)[off // 8:][:2 * K << n])
+    assert (words[0] == words[1]).all()
+    few = O.dpf_keyed_full_eval(2, n, w, roots[:2], cws[:2 * (n // w) * nk], prg, rks).reshape(-1)
+    assert (words[1][:few.size] == few).all()
