@@ -263,13 +263,19 @@ void gather_plan_free(GatherPlan& gp) {
     gp.d_off = nullptr; gp.d_entries = nullptr; gp.d_qorder = nullptr; gp.d_qslot = nullptr;
 }
 
-// log2 of the CTAs that share a tile's key halves: one until the launch has
-// four waves of resident threads (1024 per SM at 64 registers) without, else
-// up to a cluster of 8, each keeping at least two of the 2t .. 4t halves.
-int leaf_lsplit(size_t threads, int t) {
-    const size_t want = static_cast<size_t>(sm_count()) * 1024 * 4;
+// log2 of the CTAs that share a tile's key halves.  `leaves` (all keys' leaves,
+// of every expansion in the launch) over S per thread and 1024 resident threads
+// per SM (64 registers) is the launch's length in key halves; a thread's chain
+// is up to 4t of them, and the launch waits for the last.  The chain is cut
+// until it is at most half the launch, in up to 8 parts that keep at least two
+// halves each.  Cutting costs: 20:4:16 + 18:2:8 (logN:c:t) in one launch 15.66 ms
+// whole, 16.38 in 8 parts, three of t <= 16 at 2^17 .. 2^18 2.59 against 2.63; it
+// pays where t is large for the work: six small requests up to t = 32 2.50 ->
+// 2.18 ms, two of 14:2:8 221 -> 131 us.
+int leaf_lsplit(double leaves, int S, int t) {
+    const double halves = leaves / S / (1024.0 * sm_count());
     int l = 0;
-    while (l < 3 && (threads << l) < want && (2 * t >> (l + 1)) >= 2) ++l;
+    while (l < 3 && (4 * t >> l) > halves / 2 && (2 * t >> (l + 1)) >= 2) ++l;
     return l;
 }
 
@@ -283,7 +289,7 @@ void keyed_leaf_gather(const GatherPlan& gp, int party, int prg, const Blk* F, c
     while (tpb > 1 && static_cast<size_t>(tpb) * gp.S > L.bin) tpb >>= 1;
     if (static_cast<size_t>(tpb) * gp.S > L.bin) fail(PCGB_EINVAL, "bin smaller than one tile");
     if (gp.Qs == 0) return;   // a shard with no pairs
-    L.lsplit = leaf_lsplit(static_cast<size_t>(gp.Qs) * gp.N / gp.S, gp.t);
+    L.lsplit = leaf_lsplit(gather_leaves(gp), gp.S, gp.t);
     L.tpb = tpb;
     L.grid = dim3(static_cast<unsigned>(L.bin / (static_cast<size_t>(tpb) * gp.S)) << L.lsplit,
                   static_cast<unsigned>(gp.t), static_cast<unsigned>(gp.Qs));

@@ -476,13 +476,15 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
     char* tab = static_cast<char*>(pool_alloc(sizeof(XJob) * count, st));
     PCGB_CK(cudaMemcpyAsync(tab, xj.data(), sizeof(XJob) * count, cudaMemcpyHostToDevice, st));
     // Stage 2: the fused leaf kernel over every expansion's tiles.
-    // A CTA of a t = 32 expansion runs 4 times as long as one of t = 8 (64 to
-    // 128 key halves a thread), and the launch waits for the last: clusters
-    // of up to 8 CTAs share a tile.
     const size_t leaf_smem = static_cast<size_t>(tpb) * (S + 1) * 2 * sizeof(uint64_t);
-    int lsplit = 3;
-    for (int i = 0; i < count; ++i)
+    double leaves = 0;
+    int t_max = 1, lsplit = 3;
+    for (int i = 0; i < count; ++i) {
+        leaves += gather_leaves(e[i]->gp);
+        t_max = std::max(t_max, e[i]->t);
         while (lsplit > 0 && (2 * e[i]->t >> lsplit) < 2) --lsplit;
+    }
+    lsplit = std::min(lsplit, leaf_lsplit(leaves, S, t_max));
     keyed_leaf_multi_chacha(w, sl, leaf.data(), count, lsplit, tpb, leaf_smem, nullptr, nullptr, st);
     // Stage 3: the sparse x products.
     launch({x_ctas, 256, x_smem, true}, st, x_multi_kernel, reinterpret_cast<const XJob*>(tab), count);

@@ -246,7 +246,14 @@ PCGB_KEYED_DECL(chacha)
 PCGB_KEYED_DECL(aes)
 #undef PCGB_KEYED_DECL
 
-int leaf_lsplit(size_t threads, int t);
+int leaf_lsplit(double leaves, int S, int t);
+// Leaves the gather of this shard hashes: every one of its blocks' keys'.
+inline double gather_leaves(const GatherPlan& gp) {
+    int blocks = 0;
+    for (int q : gp.shard_pairs)
+        blocks += gp.pair_ij[q] / gp.c == gp.pair_ij[q] % gp.c ? 1 : 2;
+    return 2.0 * blocks * gp.t * gp.N;   // t^2 keys of 2N/t leaves a block
+}
 // Fused leaf kernel: frontier F (level hl) -> leaves -> out-hash -> convert
 // -> gather into the folded, pair-merged g' (Q buffers of N residues).
 void keyed_leaf_gather(const GatherPlan& gp, int party, int prg, const Blk* F, const Blk* cws,
