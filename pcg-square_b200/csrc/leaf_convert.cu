@@ -124,7 +124,7 @@ __device__ __forceinline__ unsigned __int128 leaf_y(uint64_t w, uint64_t cw) {
 template <class In>
 __host__ __device__ constexpr int gather_ahead() { return sizeof(In) == 16 ? 1 : 8; }
 
-// Gather scatter: thread per output word p < N.  The instances b = kk*t + (s -
+// Gather scatter: thread per output word p, p0 <= p < p1.  The instances b = kk*t + (s -
 // kk) of one (fold, s) are t - 1 apart, so their leaves are walked with one
 // stride, gather_ahead of them loaded before they are used: 14.3 us for
 // converted words at N = 2^16, t = 16, where one load at a time took 20.8.  The
@@ -134,10 +134,11 @@ template <class In>
 __global__ void __launch_bounds__(kTPB, 4) out_gather_kernel(const In* __restrict__ leaves,
                                                           int B, size_t D, int t, int party,
                                                           const uint64_t* __restrict__ cws,
-                                                          uint64_t* __restrict__ g, size_t N) {
+                                                          uint64_t* __restrict__ g, size_t N,
+                                                          size_t p0, size_t p1) {
     constexpr int U = gather_ahead<In>();
-    const size_t p = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= N) return;
+    const size_t p = p0 + static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (p >= p1) return;
     const size_t bin = D >> 1;
     const int kk_max = (B - 1) / t;
     const long s_max = static_cast<long>(kk_max) + t - 1;
@@ -218,7 +219,12 @@ __global__ void beaver_close_kernel(int B, int party, const uint64_t* __restrict
     cw[b] = v;
 }
 
+constexpr int kGatherCtas = 4;   // resident per SM (the kernel's launch bound)
+constexpr int kParts = 16;       // pieces of dpf_out_scatter_g's result, at most
+
 struct ConvPool {
+    cudaStream_t copy = nullptr;
+    cudaEvent_t part[kParts] = {};
     uint64_t* partials = nullptr;
     uint64_t* sums = nullptr;
     uint64_t* cws = nullptr;
@@ -275,9 +281,11 @@ void out_sums_launch(const Blk* d_leaves, int B, size_t D, uint64_t* partials, u
 }
 
 void out_gather_launch(const Blk* d_leaves, int B, size_t D, int t, int party,
-                       const uint64_t* d_cws, uint64_t* d_g, size_t N, cudaStream_t st) {
-    out_gather_kernel<ulonglong2><<<static_cast<unsigned>((N + kTPB - 1) / kTPB), kTPB, 0, st>>>(
-        reinterpret_cast<const ulonglong2*>(d_leaves), B, D, t, party, d_cws, d_g, N);
+                       const uint64_t* d_cws, uint64_t* d_g, size_t N, size_t p0, size_t p1,
+                       cudaStream_t st) {
+    out_gather_kernel<ulonglong2>
+        <<<static_cast<unsigned>((p1 - p0 + kTPB - 1) / kTPB), kTPB, 0, st>>>(
+            reinterpret_cast<const ulonglong2*>(d_leaves), B, D, t, party, d_cws, d_g, N, p0, p1);
     PCGB_POST_LAUNCH();
 }
 
@@ -381,13 +389,42 @@ void dpf_out_scatter_host(const Blk* d_leaves, int B, size_t D, int t, int party
     grow(pl.cws, pl.cap_cw, static_cast<size_t>(B));
     grow(pl.g, pl.cap_g, static_cast<size_t>(N));
     std::vector<uint64_t> cw(CW, CW + B);
-    for (auto& v : cw) v %= kP;
+    for (auto& v : cw) v = reduce_p(v);
     PCGB_CK(cudaMemcpyAsync(pl.cws, cw.data(), B * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    out_gather_launch(d_leaves, B, D, t, party, pl.cws, pl.g, static_cast<size_t>(N), st);
-    HostStage io;
-    void* out[1] = {g_out};
-    const size_t out_len[1] = {static_cast<size_t>(N) * sizeof(uint64_t)};
-    io.download(out, out_len, 1, pl.g, st);
+    // From two waves of resident threads on, g is made in pieces of whole waves
+    // (no more partial waves than in one launch) and each piece crosses to the
+    // host while the next is hashed: at N = 2^20, t = 16 the 8 MB copy took as
+    // long as the kernel.
+    const size_t n = static_cast<size_t>(N);
+    const size_t wave = static_cast<size_t>(sm_count()) * kGatherCtas * kTPB;
+    if (n <= 2 * wave) {
+        out_gather_launch(d_leaves, B, D, t, party, pl.cws, pl.g, n, 0, n, st);
+        HostStage io;
+        void* out[1] = {g_out};
+        const size_t out_len[1] = {n * sizeof(uint64_t)};
+        io.download(out, out_len, 1, pl.g, st);
+        return;
+    }
+    if (!pl.copy) {
+        for (auto& e : pl.part)
+            if (!e) PCGB_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        PCGB_CK(cudaStreamCreateWithFlags(&pl.copy, cudaStreamNonBlocking));
+    }
+    const size_t waves = (n + wave - 1) / wave;
+    const size_t piece = wave * std::max<size_t>(2, (waves + kParts - 1) / kParts);
+    int parts = 0;
+    for (size_t p = 0; p < n; p += piece, ++parts) {
+        out_gather_launch(d_leaves, B, D, t, party, pl.cws, pl.g, n, p, std::min(n, p + piece), st);
+        PCGB_CK(cudaEventRecord(pl.part[parts], st));
+    }
+    for (int i = 0; i < parts; ++i) {
+        const size_t p = static_cast<size_t>(i) * piece;
+        PCGB_CK(cudaStreamWaitEvent(pl.copy, pl.part[i], 0));
+        PCGB_CK(cudaMemcpyAsync(g_out + p, pl.g + p, std::min(piece, n - p) * sizeof(uint64_t),
+                                cudaMemcpyDeviceToHost, pl.copy));
+    }
+    PCGB_CK(cudaStreamSynchronize(pl.copy));
+    PCGB_CK(cudaStreamSynchronize(st));
 }
 
 // Device-pointer form: CWs already on the device (values in [0, p)), g
@@ -402,7 +439,8 @@ void dpf_out_scatter_device(const Blk* d_leaves, int B, size_t D, int t, int par
     const size_t s_max = static_cast<size_t>((B - 1) / t) + t - 1;
     if ((s_max + 2) * bin > 2 * static_cast<size_t>(N))
         fail(PCGB_EINVAL, "dpf_out_scatter_g_device: N smaller than the instances' span");
-    out_gather_launch(d_leaves, B, D, t, party, d_cw, d_g, static_cast<size_t>(N), st);
+    out_gather_launch(d_leaves, B, D, t, party, d_cw, d_g, static_cast<size_t>(N), 0,
+                      static_cast<size_t>(N), st);
 }
 
 void dpf_out_convert_device(const Blk* d_leaves, int B, size_t D, uint64_t* d_conv,
@@ -432,7 +470,8 @@ void dpf_out_scatter_conv_device(const uint64_t* d_conv, int B, size_t D, int t,
     if ((s_max + 2) * bin > 2 * static_cast<size_t>(N))
         fail(PCGB_EINVAL, "dpf_out_scatter_g_conv_device: N smaller than the instances' span");
     out_gather_kernel<uint64_t><<<static_cast<unsigned>((N + kTPB - 1) / kTPB), kTPB, 0, st>>>(
-        d_conv, B, D, t, party, d_cw, d_g, static_cast<size_t>(N));
+        d_conv, B, D, t, party, d_cw, d_g, static_cast<size_t>(N), size_t{0},
+        static_cast<size_t>(N));
     PCGB_POST_LAUNCH();
 }
 

@@ -85,3 +85,23 @@ def test_interactive_levels_without_exchange(pcg):
         pcg.synchronize()
         assert (d_c2.download(np.uint64, B << n) == conv).all()
         assert (ref.download(np.uint64, 2 * B) == d_s.download(np.uint64, 2 * B)).all()
+
+
+@pytest.mark.parametrize("t,D,N", [(4, 1 << 17, 1 << 18), (8, 1 << 17, 1 << 19),
+                                   (5, 1 << 17, 700001), (4, 1 << 18, 6000000)])
+def test_scatter_in_pieces(pcg, t, D, N):
+    """g copied out piece by piece equals the device form's, past the fold and
+    in the zero tail of an N larger than the instances span."""
+    B = t * t
+    leaves = pcg.DeviceBuffer(16 * B * D)
+    rng = np.random.default_rng(t)
+    block = rng.integers(0, 2**64 - 1, 2 * D, dtype=np.uint64)
+    for b in range(B):
+        leaves.upload_at(np.roll(block, 2 * b), 16 * b * D)
+    CW = rng.integers(0, 2**64 - 1, B, dtype=np.uint64)
+    d_cw, d_g = pcg.to_device(CW % np.uint64(P)), pcg.DeviceBuffer(8 * N)
+    for party in (0, 1):
+        g = pcg.dpf_out_scatter_g(leaves.ptr, B, D, t, party, CW, N)
+        pcg.dpf_out_scatter_g_device(leaves.ptr, B, D, t, party, d_cw.ptr, d_g.ptr, N)
+        pcg.synchronize()
+        assert (g == d_g.download(np.uint64, N)).all()
