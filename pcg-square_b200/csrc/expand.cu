@@ -226,6 +226,14 @@ int ilog2(uint64_t v) {
 }  // namespace
 }  // namespace pcgb
 
+namespace pcgb {
+// A second stream and the events that tie it to a call's own.
+struct Fork {
+    cudaStream_t side = nullptr;
+    cudaEvent_t begin = nullptr, end = nullptr;
+};
+}  // namespace pcgb
+
 struct pcgb_expander {
     int dev = 0;
     int N = 0, c = 0, t = 0, w = 0, prg = 0, n = 0, levels = 0, nk = 0, K = 0, Q = 0;
@@ -250,6 +258,7 @@ struct pcgb_expander {
     std::array<const void*, 7> graph_key{};
     int graph_party = -1;
     cudaStream_t graph_stream = nullptr;
+    pcgb::Fork graph_fork;       // the x branch of the captured graph
     // host staging for pcgb_expand_host
     void* h_stage = nullptr;
     size_t h_stage_bytes = 0;
@@ -357,6 +366,9 @@ void expander_destroy(pcgb_expander* e) {
     if (e->async_compute) cudaEventDestroy(e->async_compute);
     for (auto& ev : e->prof_ev) cudaEventDestroy(ev);
     if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
+    if (e->graph_fork.begin) cudaEventDestroy(e->graph_fork.begin);
+    if (e->graph_fork.end) cudaEventDestroy(e->graph_fork.end);
+    if (e->graph_fork.side) cudaStreamDestroy(e->graph_fork.side);
     cudaSetDevice(cur);
     delete e;
 }
@@ -381,26 +393,46 @@ Workspace workspace_carve(const pcgb_expander* e, void* base) {
     return ws;
 }
 
-void expand_device_ws(pcgb_expander* e, const Workspace& ws, int party, const Blk* roots,
-                      const Blk* cws, const uint64_t* cw_out, const uint64_t* pos,
-                      const uint64_t* val, uint64_t* x, uint64_t* z, cudaStream_t st) {
+// fork (while a graph is captured): x becomes a branch of its own beside the
+// walk and the leaf kernel, which leave the multiplier pipe and the L2 idle (its
+// 0.14 ms of the headline's 15.06, 4 of the 39 us at N = 2^12).  Launched directly
+// it follows the leaf kernel and fills its last wave (x_kernel).
+static void expand_stages(pcgb_expander* e, const Workspace& ws, int party, const Blk* roots,
+                          const Blk* cws, const uint64_t* cw_out, const uint64_t* pos,
+                          const uint64_t* val, uint64_t* x, uint64_t* z, const Fork* fork,
+                          cudaStream_t st) {
     if (party != 0 && party != 1) fail(PCGB_EINVAL, "expand: party must be 0 or 1");
     if (!roots || !cws || !cw_out || !pos || !val || !x || !z) fail(PCGB_EINVAL, "expand: null pointer");
     const size_t NN = static_cast<size_t>(e->N);
     cudaEvent_t* ev = nullptr;
     if (e->prof_slots > 0 && e->prof_used < e->prof_slots) ev = &e->prof_ev[5 * e->prof_used++];
+    const size_t sm = sizeof(uint64_t) * 2 * static_cast<size_t>(e->c) * e->t;
+    if (fork) {
+        PCGB_CK(cudaEventRecord(fork->begin, st));
+        PCGB_CK(cudaStreamWaitEvent(fork->side, fork->begin, 0));
+        launch({blocks_for(NN, 256), 256, sm}, fork->side, x_kernel, pos, val, e->d_aR, e->c, e->t,
+               e->i0, NN, x);
+        PCGB_CK(cudaEventRecord(fork->end, fork->side));
+    }
     if (ev) PCGB_CK(cudaEventRecord(ev[0], st));
     keyed_expand_tops(e->K, e->n, e->w, e->prg, roots, cws, e->d_rk, e->gp.hl, ws.F, ws.tops, st);
     if (ev) PCGB_CK(cudaEventRecord(ev[1], st));
     keyed_leaf_gather(e->gp, party, e->prg, ws.F, cws, cw_out, e->d_rk, ws.g, st);
     if (ev) PCGB_CK(cudaEventRecord(ev[2], st));
-    const size_t sm = sizeof(uint64_t) * 2 * static_cast<size_t>(e->c) * e->t;
-    launch({blocks_for(NN, 256), 256, sm, true}, st, x_kernel, pos, val, e->d_aR, e->c, e->t, e->i0,
-           NN, x);
+    if (!fork)
+        launch({blocks_for(NN, 256), 256, sm, true}, st, x_kernel, pos, val, e->d_aR, e->c, e->t,
+               e->i0, NN, x);
     if (ev) PCGB_CK(cudaEventRecord(ev[3], st));
     if (e->gp.Qs > 0) ntt_mac_inverse(*e->ntt, ws.g, e->d_img, e->gp.Qs, z, st);
     else PCGB_CK(cudaMemsetAsync(z, 0, sizeof(uint64_t) * NN, st));   // a shard with no pairs
     if (ev) PCGB_CK(cudaEventRecord(ev[4], st));
+    if (fork) PCGB_CK(cudaStreamWaitEvent(st, fork->end, 0));
+}
+
+void expand_device_ws(pcgb_expander* e, const Workspace& ws, int party, const Blk* roots,
+                      const Blk* cws, const uint64_t* cw_out, const uint64_t* pos,
+                      const uint64_t* val, uint64_t* x, uint64_t* z, cudaStream_t st) {
+    expand_stages(e, ws, party, roots, cws, cw_out, pos, val, x, z, nullptr, st);
 }
 
 // Expansions of different shapes as one batch (ChaCha8, one w and one leaf
@@ -600,10 +632,14 @@ void expand_device(pcgb_expander* e, int party, const Blk* roots, const Blk* cws
         note_launches(e->graph_kernels);
         return;
     }
+    Fork& f = e->graph_fork;
+    if (!f.begin) PCGB_CK(cudaEventCreateWithFlags(&f.begin, cudaEventDisableTiming));
+    if (!f.end) PCGB_CK(cudaEventCreateWithFlags(&f.end, cudaEventDisableTiming));
+    if (!f.side) PCGB_CK(cudaStreamCreateWithFlags(&f.side, cudaStreamNonBlocking));
     cudaGraph_t graph = nullptr;
     PCGB_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     try {
-        expand_device_ws(e, ws, party, roots, cws, cw_out, pos, val, x, z, st);
+        expand_stages(e, ws, party, roots, cws, cw_out, pos, val, x, z, &f, st);
     } catch (...) {
         cudaStreamEndCapture(st, &graph);
         if (graph) cudaGraphDestroy(graph);
