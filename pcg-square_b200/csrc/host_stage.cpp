@@ -32,11 +32,11 @@ constexpr size_t kPage = 4096;
 // way: 2.27 -> 2.07 ms; 3 x 32 MB: 13.0 -> 6.5 ms).  Between the two the
 // driver's own staging is as good.
 constexpr size_t kSmall = size_t{4} << 20, kLarge = size_t{16} << 20;
-inline bool staged(size_t bytes) { return bytes <= kSmall || bytes >= kLarge; }
 
 struct Stage {
     std::mutex mu;
     char* pinned = nullptr;
+    size_t bytes = 0;
     cudaEvent_t ev[kChunks] = {};
 };
 
@@ -113,22 +113,36 @@ struct HostStage::Impl {
 HostStage::HostStage() : im(new Impl) {
     im->s = &stage_for_device(&im->dev);
     im->lk = std::unique_lock<std::mutex>(im->s->mu, std::try_to_lock);
-    if (im->lk && !im->s->pinned) {
-        if (cudaMallocHost(&im->s->pinned, kStageBytes) != cudaSuccess) {
-            cudaGetLastError();
-            im->s->pinned = nullptr;
-        } else {
-            for (auto& e : im->s->ev)
-                if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
-                    cudaGetLastError();
-                    e = nullptr;
-                    cudaFreeHost(im->s->pinned);
-                    im->s->pinned = nullptr;
-                    break;
-                }
+    usable = im->lk.owns_lock();
+}
+
+// Makes the buffer hold a transfer of `total` bytes (kSmall, or kStageBytes
+// for the large ones: 32 MB of pinned memory take 13 ms to get, 4 MB 2).
+bool HostStage::reserve(size_t total) {
+    if (!usable || (total > kSmall && total < kLarge)) return false;
+    Stage& s = *im->s;
+    const size_t want = total <= kSmall ? kSmall : kStageBytes;
+    if (s.bytes >= want) return true;
+    if (pending) check_cuda(cudaStreamSynchronize(pending), "host copy");
+    pending = nullptr;
+    used = 0;
+    if (s.pinned) cudaFreeHost(s.pinned);
+    s.pinned = nullptr;
+    s.bytes = 0;
+    bool ok = true;
+    for (auto& e : s.ev)
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            e = nullptr;
+            ok = false;
         }
+    if (!ok || cudaMallocHost(&s.pinned, want) != cudaSuccess) {
+        cudaGetLastError();
+        s.pinned = nullptr;
+        usable = false;
+        return false;
     }
-    usable = im->lk && im->s->pinned;
+    s.bytes = want;
+    return true;
 }
 
 HostStage::~HostStage() {
@@ -141,6 +155,7 @@ void HostStage::trim() {
     std::lock_guard<std::mutex> lk(s.mu);
     if (s.pinned) cudaFreeHost(s.pinned);
     s.pinned = nullptr;
+    s.bytes = 0;
 }
 
 namespace {
@@ -162,12 +177,12 @@ void parts_of(Ptr const* piece, const size_t* len, int pieces, size_t a, size_t 
 void HostStage::upload(void* d_dst, const void* const* src, const size_t* len, int pieces,
                        cudaStream_t st) {
     size_t total = 0;
-    bool direct = !usable;
+    bool direct = false;
     for (int i = 0; i < pieces; ++i) {
         total += len[i];
         direct = direct || (len[i] && is_pinned(src[i]));
     }
-    direct = direct || !staged(total);
+    direct = direct || !reserve(total);
     if (direct) {
         size_t o = 0;
         for (int i = 0; i < pieces; ++i) {
@@ -179,11 +194,11 @@ void HostStage::upload(void* d_dst, const void* const* src, const size_t* len, i
     }
     Stage& s = *im->s;
     for (size_t at = 0; at < total;) {
-        if (used == kStageBytes) {   // earlier copies still read the buffer
+        if (used == s.bytes) {   // earlier copies still read the buffer
             check_cuda(cudaStreamSynchronize(pending), "host upload");
             used = 0;
         }
-        const size_t round = std::min(kStageBytes - used, total - at);
+        const size_t round = std::min(s.bytes - used, total - at);
         const int n = static_cast<int>((round + kChunk - 1) / kChunk);
         char* base = s.pinned + used;
         pending = st;
@@ -202,19 +217,19 @@ void HostStage::upload(void* d_dst, const void* const* src, const size_t* len, i
         });
         if (bad) check_cuda(static_cast<cudaError_t>(bad.load()), "host upload");
         at += round;
-        used = std::min(kStageBytes, (used + round + 255) & ~size_t{255});
+        used = std::min(s.bytes, (used + round + 255) & ~size_t{255});
     }
 }
 
 void HostStage::download(void* const* dst, const size_t* len, int pieces, const void* d_src,
                          cudaStream_t st) {
     size_t total = 0;
-    bool direct = !usable;
+    bool direct = false;
     for (int i = 0; i < pieces; ++i) {
         total += len[i];
         direct = direct || (len[i] && is_pinned(dst[i]));
     }
-    direct = direct || !staged(total);
+    direct = direct || !reserve(total);
     if (direct) {
         size_t o = 0;
         for (int i = 0; i < pieces; ++i) {
@@ -227,8 +242,8 @@ void HostStage::download(void* const* dst, const size_t* len, int pieces, const 
     }
     Stage& s = *im->s;
     if (pending && pending != st) check_cuda(cudaStreamSynchronize(pending), "host download");
-    for (size_t at = 0; at < total; at += kStageBytes) {
-        const size_t round = std::min(kStageBytes, total - at);
+    for (size_t at = 0; at < total; at += s.bytes) {
+        const size_t round = std::min(s.bytes, total - at);
         const int n = static_cast<int>((round + kChunk - 1) / kChunk);
         for (int c = 0; c < n; ++c) {
             const size_t o = static_cast<size_t>(c) * kChunk, l = std::min(kChunk, round - o);

@@ -73,6 +73,7 @@ class HostStage {
     static void trim();   // frees the current device's buffer
 
   private:
+    bool reserve(size_t total);
     struct Impl;
     Impl* im;
     bool usable = false;
