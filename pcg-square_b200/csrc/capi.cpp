@@ -607,7 +607,7 @@ int pcgb_dpf_keyed_full_eval(int K, int n, int w, int prg, const pcgb_blk* d_roo
         const int levels = n / w, nk = (1 << w) - 1;
         uint32_t* d_rk = nullptr;
         if (prg == PCGB_PRG_AES) d_rk = pcgb::aes_upload_round_keys(round_keys, nk, st);
-        const size_t sn = pcgb::keyed_tops_scratch_nodes(K, w, levels);
+        const size_t sn = pcgb::keyed_tops_scratch_nodes(K, w, prg, levels);
         Blk* scratch = nullptr;
         if (sn) scratch = static_cast<Blk*>(pcgb::pool_alloc(sn * sizeof(Blk), st));
         pcgb::keyed_expand_tops(K, n, w, prg, reinterpret_cast<const Blk*>(d_roots),

@@ -11,24 +11,31 @@
 
 namespace pcgb {
 
-std::vector<int> tops_stages(int K, int w, int to_level) {
+std::vector<int> tops_stages(int K, int w, int prg, int to_level) {
+    // Whether level l has enough subtrees for the final stage.  The persistent
+    // AES walk is full with one stride of its grid (148 x 1024), so binary AES
+    // takes half the count when that leaves it at most 6 levels (777 keys x 2^14:
+    // 358 -> 341 us, 2000 x 2^12 272 -> 246); with 7 the last, nearly empty stride
+    // is a chain of 127 hashes (300 x 2^17: 974 -> 1024 us).
+    auto enough = [&](int l) {
+        const size_t n = static_cast<size_t>(K) << (w * l);
+        return n >= kTopsStage2Threads ||
+               (prg == PCGB_PRG_AES && w == 1 && n >= kTopsStage2Threads / 2 && to_level - l <= 6);
+    };
     std::vector<int> b{0};
     int l = 0;
     while (l < to_level && tops_bfs_ok(K, w, 0, l + 1) &&
-           ((static_cast<size_t>(K) << (w * l)) < kTopsStage2Threads ||
-            (w == 1 && to_level - l > kTopsFixedLevels)))
+           (!enough(l) || (w == 1 && to_level - l > kTopsFixedLevels)))
         ++l;
     const bool bfs = l > 0;
     if (bfs) b.push_back(l);
     while (l < to_level) {
-        if ((static_cast<size_t>(K) << (w * l)) >= kTopsStage2Threads) {
+        if (enough(l)) {
             b.push_back(to_level);
             break;
         }
         int s = 1;
-        while (l + s < to_level && (static_cast<size_t>(K) << (w * (l + s))) < kTopsStage2Threads &&
-               (1 << (w * (s + 1))) <= 32)
-            ++s;
+        while (l + s < to_level && !enough(l + s) && (1 << (w * (s + 1))) <= 32) ++s;
         l += s;
         b.push_back(l);
     }
@@ -51,8 +58,8 @@ std::vector<int> tops_stages(int K, int w, int to_level) {
 }
 
 // Two ping-pong halves, each holding the largest intermediate level.
-size_t keyed_tops_scratch_nodes(int K, int w, int to_level) {
-    const std::vector<int> b = tops_stages(K, w, to_level);
+size_t keyed_tops_scratch_nodes(int K, int w, int prg, int to_level) {
+    const std::vector<int> b = tops_stages(K, w, prg, to_level);
     if (b.size() <= 2) return 0;
     return 2 * (static_cast<size_t>(K) << (w * b[b.size() - 2]));
 }
@@ -100,7 +107,7 @@ void keyed_tops_multi(int groups, const int* K, const int* n, const int* to_leve
         if (!roots[g] || !cws[g] || !out[g]) fail(PCGB_EINVAL, "keyed eval multi: null group buffer");
         Plan& P = plan[g];
         P.levels = n[g] / w;
-        P.b = tops_stages(K[g], w, to_level[g]);
+        P.b = tops_stages(K[g], w, prg, to_level[g]);
         if (P.b.size() > 2) P.half = static_cast<size_t>(K[g]) << (w * P.b[P.b.size() - 2]);
         if (scratch && scratch[g]) P.base = scratch[g];
         else pool_nodes += 2 * P.half;

@@ -798,7 +798,7 @@ void tops_dispatch(int K, int levels, const Blk* roots, const Blk* cws, const ui
                    const uint32_t* rk, int to_level, Blk* out, Blk* scratch, cudaStream_t st) {
     // Stages (tops_stages): intermediate levels alternate between the two
     // halves of the scratch, the last stage writes `out`.
-    const std::vector<int> b = tops_stages(K, W, to_level);
+    const std::vector<int> b = tops_stages(K, W, PRG, to_level);
     const size_t half = b.size() > 2 ? (static_cast<size_t>(K) << (W * b[b.size() - 2])) : 0;
     const Blk* src = roots;
     for (size_t k = 0; k + 1 < b.size(); ++k) {

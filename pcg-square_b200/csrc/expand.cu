@@ -378,14 +378,14 @@ void expander_destroy(pcgb_expander* e) {
 // admitted request so expansions of the same shape can overlap.
 size_t workspace_bytes(const pcgb_expander* e) {
     const size_t fnodes = static_cast<size_t>(e->K) << (e->w * e->gp.hl);
-    const size_t tnodes = keyed_tops_scratch_nodes(e->K, e->w, e->gp.hl);
+    const size_t tnodes = keyed_tops_scratch_nodes(e->K, e->w, e->prg, e->gp.hl);
     return sizeof(Blk) * (fnodes + tnodes) +
            sizeof(uint64_t) * static_cast<size_t>(e->N) * std::max(e->gp.Qs, 1);
 }
 
 Workspace workspace_carve(const pcgb_expander* e, void* base) {
     const size_t fnodes = static_cast<size_t>(e->K) << (e->w * e->gp.hl);
-    const size_t tnodes = keyed_tops_scratch_nodes(e->K, e->w, e->gp.hl);
+    const size_t tnodes = keyed_tops_scratch_nodes(e->K, e->w, e->prg, e->gp.hl);
     Workspace ws;
     ws.F = static_cast<Blk*>(base);
     ws.tops = tnodes ? ws.F + fnodes : nullptr;

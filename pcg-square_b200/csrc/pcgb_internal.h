@@ -95,7 +95,7 @@ int sm_count();
 // m^to_level nodes per key to `out` ([k][node], natural order).  scratch
 // must hold K * m^min(to_level, first_stage_levels) nodes (may be nullptr
 // when to_level is small; see keyed_tops_scratch_nodes).
-size_t keyed_tops_scratch_nodes(int K, int w, int to_level);
+size_t keyed_tops_scratch_nodes(int K, int w, int prg, int to_level);
 
 // One key group's part of a multi-group top-walk stage (expand_tops_multi_kernel).
 struct TopsJob {
@@ -109,7 +109,7 @@ struct TopsJob {
 // Top-level walk of `groups` key groups of different domains (same w and
 // PRG), each to its own level to_level[g] into out[g]: one launch per stage
 // for all groups.  scratch[g] holds keyed_tops_scratch_nodes(K[g], w,
-// to_level[g]) nodes, or is null (scratch from the pool); scratch may be null.
+// prg, to_level[g]) nodes, or is null (scratch from the pool); scratch may be null.
 void keyed_tops_multi(int groups, const int* K, const int* n, const int* to_level, int w, int prg,
                       const Blk* const* roots, const Blk* const* cws, const uint32_t* d_rk,
                       Blk* const* out, Blk* const* scratch, cudaStream_t st);
@@ -147,7 +147,7 @@ inline bool tops_bfs_ok(int K, int w, int src_lvl, int nlev) {
     return src_lvl == 0 && nlev > 0 && w * nlev <= kTopsBfsLog && K <= kTopsBfsKeys;
 }
 // Stage boundaries 0 = l_0 < l_1 < ... < l_s = to_level.
-std::vector<int> tops_stages(int K, int w, int to_level);
+std::vector<int> tops_stages(int K, int w, int prg, int to_level);
 
 struct GatherPlan {
     int N = 0, c = 0, t = 0, n = 0, w = 0, Q = 0;
