@@ -650,7 +650,7 @@ def run_polymul(L, batch=16, logN=20, steps=10, warmup=3, seed=11):
     out["roofline"]["bound_by"] = ("64-bit integer multiplies (FMA-heavy pipe, math-pipe "
                                    "throttle the top stall; profiles/ntt_polymul_16x2e20.txt)")
 
-    # Mixed lengths in one call (five launches for the batch): 6 x 2^20,
+    # Mixed lengths in one call (four launches for the batch): 6 x 2^20,
     # 5 x 2^18, 5 x 2^16, interleaved, through pcgb_poly_mul_device_multi.
     import ctypes as C
     sizes = [1 << 20, 1 << 16, 1 << 18] * 5 + [1 << 20]

@@ -82,7 +82,7 @@ int pcgb_device_synchronize(void);
  * helpers, server requests) comes from a stream-ordered pool of its own on
  * each device, which keeps freed memory mapped so the next call of the same
  * size maps nothing.  Returns that memory on the current device to the
- * driver. */
+ * driver, and the pinned staging buffer of the host-array calls. */
 int pcgb_trim_pool(void);
 void* pcgb_default_stream(void);
 /* Kernel launches issued by the library since load (all devices). */
@@ -292,9 +292,9 @@ int pcgb_poly_mul_device(uint64_t* d_c, const uint64_t* d_a, const uint64_t* d_b
                          int N, void* stream);
 /* Uneven batch: polys of different lengths in one call; d_a[i], d_b[i],
  * d_c[i] each of length N[i]; d_c[i] may alias d_a[i] or d_b[i].  When every
- * N[i] is in 2^16 .. 2^20 the whole batch runs as five launches (one per
- * pass, each CTA reading its polynomial and tile from a job table); other
- * lengths run one product at a time. */
+ * N[i] is in 2^16 .. 2^20 the whole batch runs as four launches (one per
+ * pass, each CTA reading its polynomial and tile from a job table; five when
+ * some d_c[i] overlaps a d_a[j]); other lengths run one product at a time. */
 int pcgb_poly_mul_device_multi(int count, uint64_t* const* d_c, const uint64_t* const* d_a,
                                const uint64_t* const* d_b, const int* N, void* stream);
 
@@ -341,8 +341,8 @@ int pcgb_expand_device(pcgb_expander* e, int party, const pcgb_blk* d_roots,
  * counterpart; the batching form of GPU_baseline/e2e_full_bench.cu's
  * expansion loop): request i runs expander e[i] for party[i] on the
  * device-resident inputs of pcgb_expand_device.  One launch per top-walk
- * stage and walk depth, one fused leaf launch, one x launch and three NTT
- * launches cover the whole batch.  The expanders must share w, the ChaCha8 PRG and the leaf
+ * stage and walk depth, one fused leaf launch per 32 requests, one x launch and
+ * four NTT launches cover the whole batch.  The expanders must share w, the ChaCha8 PRG and the leaf
  * shape (leaves per thread; set with pcgb_expander_set_leaf_shape), be
  * unsharded, and have N in 2^14 .. 2^20; each request's x, z equal its
  * pcgb_expand_device outputs.  Each request's scratch comes from the

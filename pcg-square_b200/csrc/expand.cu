@@ -142,7 +142,6 @@ __global__ void digest_multi_kernel(const DigestJob* __restrict__ jobs, unsigned
     }
 }
 
-// d[i] = mont(s[i], k): multiply by a constant given in Montgomery form.
 // g'_q = g_ij (+ g_ji when i != j) mod p for the Q pairs i <= j, from the
 // c*c per-block output-layer vectors g[(i*c + j)*N ..] (each in [0, p)).
 __global__ void pair_merge_kernel(const uint64_t* __restrict__ g, int c, size_t N,
@@ -159,6 +158,7 @@ __global__ void pair_merge_kernel(const uint64_t* __restrict__ g, int c, size_t 
     gq[static_cast<size_t>(q) * N + idx] = v;
 }
 
+// d[i] = mont(s[i], k): multiply by a constant given in Montgomery form.
 __global__ void scale_kernel(uint64_t* d, const uint64_t* s, size_t n, uint64_t k) {
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) d[i] = mont_mul(reduce_p(s[i]), k);
@@ -437,9 +437,9 @@ void expand_device_ws(pcgb_expander* e, const Workspace& ws, int party, const Bl
 
 // Expansions of different shapes as one batch (ChaCha8, one w and one leaf
 // depth sl for all): one launch per top-walk stage, one fused leaf launch,
-// one x launch and three NTT launches for the whole batch, each CTA finding
-// its expansion in a job table.  Outputs equal expand_device_ws's, request by
-// request.  All job tables travel in one copy from pinned or pageable host
+// one x launch and four NTT launches for the whole batch, each CTA finding
+// its expansion in a job table (the leaf launch holds up to 32 expansions).
+// Outputs equal expand_device_ws's, request by request.  All job tables travel in one copy from pinned or pageable host
 // memory on `st`.
 void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, const int* party,
                      const Blk* const* roots, const Blk* const* cws,

@@ -1,8 +1,7 @@
 // Arithmetic mod p = 2^62 - 3*2^25 + 1 on 64-bit words (device + host).
 //
-// Values are kept canonical in [0, p).  Multiplication by a fixed constant
-// uses Shoup's precomputed quotient (w' = floor(w*2^64/p)); a product of two
-// variables uses Montgomery reduction with R = 2^64.
+// Values are kept canonical in [0, p); products use Montgomery reduction with
+// R = 2^64.  The transforms have their own lazy forms (ntt_arith.cuh).
 #ifndef PCGB_FIELD_CUH_
 #define PCGB_FIELD_CUH_
 
@@ -58,13 +57,6 @@ PCGB_HD uint64_t mont_mul(uint64_t a, uint64_t b) {
     return r >= kPm ? r - kPm : r;
 }
 
-// a*w mod p with wq = floor(w*2^64/p); a any 64-bit value below 2^63.
-PCGB_HD uint64_t shoup_mul(uint64_t a, uint64_t w, uint64_t wq) {
-    const uint64_t q = mulhi64(a, wq);
-    uint64_t r = a * w - q * kPm;
-    return r >= kPm ? r - kPm : r;
-}
-
 inline uint64_t mul_p_host(uint64_t a, uint64_t b) {
     return static_cast<uint64_t>((static_cast<unsigned __int128>(a) * b) % kPm);
 }
@@ -77,9 +69,6 @@ inline uint64_t pow_p_host(uint64_t b, uint64_t e) {
         e >>= 1;
     }
     return r;
-}
-inline uint64_t shoup_q_host(uint64_t w) {
-    return static_cast<uint64_t>((static_cast<unsigned __int128>(w) << 64) / kPm);
 }
 // 2^64 mod p and 2^128 mod p.
 inline uint64_t r_mod_p() { return static_cast<uint64_t>(((unsigned __int128)1 << 64) % kPm); }
