@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <string>
 #include <vector>
 
@@ -124,43 +125,52 @@ __device__ __forceinline__ unsigned __int128 leaf_y(uint64_t w, uint64_t cw) {
 template <class In>
 __host__ __device__ constexpr int gather_ahead() { return sizeof(In) == 16 ? 1 : 8; }
 
-// Gather scatter: thread per output word p, p0 <= p < p1.  The instances b = kk*t + (s -
+// Gather scatter of the output words p, p0 <= p < p1.  The instances b = kk*t + (s -
 // kk) of one (fold, s) are t - 1 apart, so their leaves are walked with one
-// stride, gather_ahead of them loaded before they are used: 14.3 us for
+// stride, gather_ahead of them loaded before they are used: 12.3 us for
 // converted words at N = 2^16, t = 16, where one load at a time took 20.8.  The
-// leaf form (2^20, t = 16: 501 us, 422 of them the hashes' at the ALU peak) is
+// leaf form (2^20, t = 16: 490 us, 422 of them the hashes' at the ALU peak) is
 // bound by the integer ALU either way.
-template <class In>
+//
+// SHARES (a power of two) threads, kTPB/SHARES apart, take a word's leaves
+// between them: the first bit of the share picks the runs s (fs = 0, 2: t leaves
+// in all) or s - 1 (fs = 1, 3: t as well), the rest every (SHARES/2)-th leaf of
+// these.
+template <class In, int SHARES>
 __global__ void __launch_bounds__(kTPB, 4) out_gather_kernel(const In* __restrict__ leaves,
                                                           int B, size_t D, int t, int party,
                                                           const uint64_t* __restrict__ cws,
                                                           uint64_t* __restrict__ g, size_t N,
                                                           size_t p0, size_t p1) {
     constexpr int U = gather_ahead<In>();
-    const size_t p = p0 + static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= p1) return;
+    constexpr int kWords = kTPB / SHARES;
+    constexpr int kRuns = SHARES > 1 ? 2 : 1, kEvery = SHARES / kRuns;
+    const int share = threadIdx.x / kWords;
+    const size_t p = p0 + static_cast<size_t>(blockIdx.x) * kWords + threadIdx.x % kWords;
+    if (SHARES == 1 && p >= p1) return;
     const size_t bin = D >> 1;
     const int kk_max = (B - 1) / t;
     const long s_max = static_cast<long>(kk_max) + t - 1;
     unsigned __int128 acc = 0;   // two's complement; reduced mod p once, below
 #pragma unroll 1
-    for (int fs = 0; fs < 4; ++fs) {
+    for (int fs = share % kRuns; fs < 4; fs += kRuns) {
         const bool f = fs >= 2;
         const size_t P = p + (f ? N : 0);   // pre-fold position
         const long s = static_cast<long>(P / bin) - (fs & 1);
         if (s < 0 || s > s_max) continue;
         const size_t d = P - static_cast<size_t>(s) * bin;
-        if (d >= D) continue;
-        const int kk0 = static_cast<int>(s - (t - 1) > 0 ? s - (t - 1) : 0);
+        if (d >= D || p >= p1) continue;
+        int kk0 = static_cast<int>(s - (t - 1) > 0 ? s - (t - 1) : 0);
         // b = kk*t + s - kk grows with kk, so instances beyond B are at the end.
         int kk1 = static_cast<int>(s < kk_max ? s : kk_max);
         while (kk1 >= kk0 && kk1 * t + static_cast<int>(s - kk1) >= B) --kk1;
+        kk0 += share / kRuns;
         const bool neg = (party != 0) != f;
         const size_t b0 = static_cast<size_t>(kk0) * t + static_cast<size_t>(s - kk0);
-        const int n = kk1 - kk0 + 1;
+        const int n = (kk1 - kk0 + kEvery) / kEvery;
         const In* leaf = leaves + b0 * D + d;
         const uint64_t* cw = cws + b0;
-        const size_t step = static_cast<size_t>(t - 1);
+        const size_t step = static_cast<size_t>(t - 1) * kEvery;
         In ahead[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -180,6 +190,17 @@ __global__ void __launch_bounds__(kTPB, 4) out_gather_kernel(const In* __restric
                 else acc += y;
             }
         }
+    }
+    if constexpr (SHARES > 1) {
+        __shared__ ulonglong2 part[SHARES - 1][kWords];
+        const int c = threadIdx.x % kWords;
+        if (share > 0)
+            part[share - 1][c] = {static_cast<uint64_t>(acc), static_cast<uint64_t>(acc >> 64)};
+        __syncthreads();
+        if (share > 0 || p >= p1) return;
+#pragma unroll
+        for (int i = 0; i < SHARES - 1; ++i)
+            acc += static_cast<unsigned __int128>(part[i][c].y) << 64 | part[i][c].x;
     }
     g[p] = mod_p_128(acc);
 }
@@ -280,13 +301,34 @@ void out_sums_launch(const Blk* d_leaves, int B, size_t D, uint64_t* partials, u
     PCGB_POST_LAUNCH();
 }
 
+template <class In>
+void out_gather_launch(const In* d_leaves, int B, size_t D, int t, int party,
+                       const uint64_t* d_cws, uint64_t* d_g, size_t N, size_t p0, size_t p1,
+                       cudaStream_t st) {
+    const size_t n = p1 - p0;
+    auto run = [&](auto shares) {
+        constexpr int S = decltype(shares)::value;
+        constexpr size_t words = kTPB / S;
+        out_gather_kernel<In, S><<<static_cast<unsigned>((n + words - 1) / words), kTPB, 0, st>>>(
+            d_leaves, B, D, t, party, d_cws, d_g, N, p0, p1);
+    };
+    // A word's leaves in one chain leave a short launch waiting for latency: two
+    // shares while one thread per word does not fill the chip, four up to an
+    // eighth of that.  (N, t), leaf form / converted words: 2^14, 16: 22.6 ->
+    // 13.4 / 10.3 -> 6.7 us; 2^16, 16: 41.0 -> 39.0 / 12.3 -> 10.3; 2^17, 16: 74.4
+    // -> 65.5 / 16.5 -> 15.4; nothing at 2^18, and four shares are slower from
+    // 2^16 on (20.6 at 2^17, converted words), eight from 2^14 on (8.2).
+    const size_t wave = static_cast<size_t>(sm_count()) * kGatherCtas * kTPB;
+    if (n > wave) run(std::integral_constant<int, 1>{});
+    else if (n > wave / 8) run(std::integral_constant<int, 2>{});
+    else run(std::integral_constant<int, 4>{});
+    PCGB_POST_LAUNCH();
+}
 void out_gather_launch(const Blk* d_leaves, int B, size_t D, int t, int party,
                        const uint64_t* d_cws, uint64_t* d_g, size_t N, size_t p0, size_t p1,
                        cudaStream_t st) {
-    out_gather_kernel<ulonglong2>
-        <<<static_cast<unsigned>((p1 - p0 + kTPB - 1) / kTPB), kTPB, 0, st>>>(
-            reinterpret_cast<const ulonglong2*>(d_leaves), B, D, t, party, d_cws, d_g, N, p0, p1);
-    PCGB_POST_LAUNCH();
+    out_gather_launch(reinterpret_cast<const ulonglong2*>(d_leaves), B, D, t, party, d_cws, d_g, N,
+                      p0, p1, st);
 }
 
 void dpf_out_sums_host(const Blk* d_leaves, int B, size_t D, uint64_t prime, uint64_t* sumC,
@@ -469,10 +511,8 @@ void dpf_out_scatter_conv_device(const uint64_t* d_conv, int B, size_t D, int t,
     const size_t s_max = static_cast<size_t>((B - 1) / t) + t - 1;
     if ((s_max + 2) * bin > 2 * static_cast<size_t>(N))
         fail(PCGB_EINVAL, "dpf_out_scatter_g_conv_device: N smaller than the instances' span");
-    out_gather_kernel<uint64_t><<<static_cast<unsigned>((N + kTPB - 1) / kTPB), kTPB, 0, st>>>(
-        d_conv, B, D, t, party, d_cw, d_g, static_cast<size_t>(N), size_t{0},
-        static_cast<size_t>(N));
-    PCGB_POST_LAUNCH();
+    out_gather_launch(d_conv, B, D, t, party, d_cw, d_g, static_cast<size_t>(N), 0,
+                      static_cast<size_t>(N), st);
 }
 
 void out_beaver_open_device(int B, int party, const uint64_t* d_sumC, const uint64_t* d_sumT,

@@ -66,3 +66,28 @@ def test_leaves_at_a_16_byte_address(pcg, prg, K, n, w):
     assert (words[0] == words[1]).all()
     few = O.dpf_keyed_full_eval(2, n, w, roots[:2], cws[:2 * (n // w) * nk], prg, rks).reshape(-1)
     assert (words[1][:few.size] == few).all()
+
+
+# N (the fold's length) on both sides of each step of the shares per output word
+# (148 SMs: 18944 and 151552 words), single instances, t = 1, a last row of
+# instances cut short, an N beyond the instances' span.
+@pytest.mark.parametrize("B,t,D,N", [(1, 1, 2, 1), (1, 1, 64, 100), (1, 4, 32, 64), (3, 4, 32, 70),
+                                     (16, 4, 512, 1024), (15, 4, 512, 1031), (49, 7, 1024, 18944),
+                                     (64, 8, 4096, 18945), (63, 8, 8192, 32768),
+                                     (16, 4, 65536, 151552), (16, 4, 65536, 151553)])
+@pytest.mark.parametrize("party", [0, 1])
+def test_scatter_with_shared_words(pcg, B, t, D, N, party):
+    rng = np.random.default_rng(B * 31 + N)
+    leaves = rng.integers(0, 2**64 - 1, (B * D, 2), dtype=np.uint64, endpoint=True)
+    leaves[:: 5] = np.uint64(2**64 - 1)
+    CW = rng.integers(0, O.P, B, dtype=np.uint64)
+    CW[0] = O.P - 1
+    want = O.out_scatter_g(leaves, B, D, t, party, CW, N)
+    d = dev(pcg, leaves)
+    conv, sums = pcg.DeviceBuffer(8 * B * D), pcg.DeviceBuffer(16 * B)
+    pcg.dpf_out_convert_device(d.ptr, B, D, conv.ptr, sums.ptr, sums.ptr + 8 * B)
+    d_cw, d_g = pcg.to_device(CW), pcg.DeviceBuffer(8 * N)
+    for f, src in ((pcg.dpf_out_scatter_g_device, d), (pcg.dpf_out_scatter_g_conv_device, conv)):
+        f(src.ptr, B, D, t, party, d_cw.ptr, d_g.ptr, N)
+        pcg.synchronize()
+        assert (d_g.download(np.uint64, N) == want).all()
