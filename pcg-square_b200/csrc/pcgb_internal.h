@@ -333,6 +333,12 @@ void ntt_forward(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st);
 // add[z]), add[z] null for none; inputs any uint64, outputs in [0, p).
 void ntt_forward3(const NttPlan& pl, const uint64_t* const (&src)[3],
                   const uint64_t* const (&add)[3], uint64_t* const (&dst)[3], cudaStream_t st);
+// Adds to *bad the number of slots where NTT(x0)*NTT(x1) != NTT(z0 + z1); inputs
+// any uint64.  scratch: 3N words when ntt_check_needs_scratch.
+bool ntt_check_needs_scratch(const NttPlan& pl);
+void ntt_check_ole(const NttPlan& pl, const uint64_t* x0, const uint64_t* x1, const uint64_t* z0,
+                   const uint64_t* z1, uint64_t* scratch, unsigned long long* bad,
+                   cudaStream_t st);
 void ntt_log_sizes(const NttPlan& pl, int* l1, int* l2);   // see ntt_layout.cuh
 // c = a * b mod (X^N+1) for `batch` polys; c may alias a or b; inputs any
 // uint64 (reduced mod p first).  scratch: batch*N words when

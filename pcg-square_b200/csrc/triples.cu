@@ -51,18 +51,6 @@ __global__ void triple_slots_kernel(const uint64_t* A, const uint64_t* B, const 
     c[k] = add_p(mont_mul(mont_mul(x, y), r2), v);
 }
 
-// Counts slots where X0*X1 != Z (all transformed, in [0, p)).
-__global__ void ole_check_kernel(const uint64_t* X0, const uint64_t* X1, const uint64_t* Z,
-                                 size_t n, uint64_t r2, unsigned long long* bad) {
-    chain_begin();
-    unsigned long long mine = 0;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x)
-        mine += mont_mul(mont_mul(ld_chained(X0 + i), ld_chained(X1 + i)), r2) != ld_chained(Z + i);
-    for (int o = 16; o; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(bad, mine);
-}
-
 // Counts slots where (a0+a1)(b0+b1) != c0+c1 (slot values any 64-bit).
 __global__ void triple_check_kernel(const uint64_t* __restrict__ a0, const uint64_t* __restrict__ b0,
                                     const uint64_t* __restrict__ c0, const uint64_t* __restrict__ a1,
@@ -120,13 +108,12 @@ void verify_ole_device(int N, const uint64_t* x0, const uint64_t* z0, const uint
                        const uint64_t* z1, unsigned long long* bad, cudaStream_t st) {
     if (!x0 || !z0 || !x1 || !z1 || !bad) fail(PCGB_EINVAL, "verify_ole: null pointer");
     const NttPlan& pl = ntt_plan(log2_checked(N, "verify_ole"));
-    const size_t n = static_cast<size_t>(N);
-    uint64_t* T = static_cast<uint64_t*>(pool_alloc(3 * n * sizeof(uint64_t), st));  // X0 | X1 | Z
+    uint64_t* T = nullptr;   // X0 | X1 | Z after the column pass
+    if (ntt_check_needs_scratch(pl))
+        T = static_cast<uint64_t*>(pool_alloc(3 * sizeof(uint64_t) * static_cast<size_t>(N), st));
     PCGB_CK(cudaMemsetAsync(bad, 0, sizeof(unsigned long long), st));
-    ntt_forward3(pl, {x0, x1, z0}, {nullptr, nullptr, z1}, {T, T + n, T + 2 * n}, st);
-    launch({check_grid(n), kTpb, 0, true}, st, ole_check_kernel, T, T + n, T + 2 * n, n, r2_mod_p(),
-           bad);
-    PCGB_CK(cudaFreeAsync(T, st));
+    ntt_check_ole(pl, x0, x1, z0, z1, T, bad, st);
+    if (T) PCGB_CK(cudaFreeAsync(T, st));
 }
 
 void verify_triples_device(int N, const uint64_t* a0, const uint64_t* b0, const uint64_t* c0,

@@ -50,3 +50,32 @@ def test_square_in_place(pcg):
         d = dev(pcg, a)
         pcg.poly_mul_device(d.ptr, d.ptr, d.ptr, 1, 1 << lg)
         assert (d.download(np.uint64, 1 << lg) == O.poly_mul(a, a, 1 << lg)).all()
+
+
+# One row (2^1 .. 2^9, ragged rows per CTA), the shortest and longest four-step
+# rows, odd and even logN; words at the extremes of 64 bits.
+@pytest.mark.parametrize("logN", [1, 3, 4, 5, 9, 10, 11, 13, 16, 19, 22, 24])
+def test_ole_check_counts_slots(pcg, logN):
+    """0 for a product; N / 2 with X^(N/2) - I added (I^2 = -1: it vanishes in
+    every other slot); N with a constant added."""
+    N = 1 << logN
+    rng = np.random.default_rng(logN)
+    x0 = rng.integers(0, 2**64 - 1, N, dtype=np.uint64, endpoint=True)
+    x1 = rng.integers(0, 2**64 - 1, N, dtype=np.uint64, endpoint=True)
+    z1 = rng.integers(0, P, N, dtype=np.uint64)
+    x0[0] = x1[-1] = np.uint64(2**64 - 1)
+    d0, d1, dz1 = (pcg.to_device(a) for a in (x0, x1, z1))
+    prod, bad = pcg.DeviceBuffer(8 * N), pcg.DeviceBuffer(8)
+    pcg.poly_mul_device(prod.ptr, d0.ptr, d1.ptr, 1, N)
+    pcg.synchronize()
+    z0 = (prod.download(np.uint64, N) + np.uint64(P) - z1) % np.uint64(P)
+    I = pow(3, (P - 1) // 4, P)
+    half, full = z0.copy(), z0.copy()
+    half[N // 2] = (int(half[N // 2]) + 1) % P
+    half[0] = (int(half[0]) - I) % P
+    full[0] = (int(full[0]) + 7) % P
+    for z, want in ((z0, 0), (half, N // 2), (full, N)):
+        dz = pcg.to_device(z)
+        pcg.verify_ole_device(N, d0.ptr, dz.ptr, d1.ptr, dz1.ptr, bad.ptr)
+        pcg.synchronize()
+        assert int(bad.download(np.uint64, 1)[0]) == want
