@@ -14,13 +14,16 @@ namespace pcgb {
 std::vector<int> tops_stages(int K, int w, int prg, int to_level) {
     // Whether level l has enough subtrees for the final stage.  The persistent
     // AES walk is full with one stride of its grid (148 x 1024), so binary AES
-    // takes half the count when that leaves it at most 6 levels (777 keys x 2^14:
-    // 358 -> 341 us, 2000 x 2^12 272 -> 246); with 7 the last, nearly empty stride
-    // is a chain of 127 hashes (300 x 2^17: 974 -> 1024 us).
+    // takes half the count when that leaves it at most 5 levels (777 keys x 2^14:
+    // 357 -> 337 us, 2000 x 2^12 272 -> 243, 20 x 2^17 166 -> 142, 30000 x 2^6 122 ->
+    // 98); with more, a last, nearly empty stride is a longer chain than the stage
+    // saved (300 x 2^16: 519 -> 529, 300 x 2^17 974 -> 1024).  Walks of two levels
+    // are one stage (168649 x 2^2: 39 us, 44 in two).
     auto enough = [&](int l) {
         const size_t n = static_cast<size_t>(K) << (w * l);
         return n >= kTopsStage2Threads ||
-               (prg == PCGB_PRG_AES && w == 1 && n >= kTopsStage2Threads / 2 && to_level - l <= 6);
+               (prg == PCGB_PRG_AES && w == 1 && to_level > 2 && to_level - l <= 5 &&
+                n >= kTopsStage2Threads / 2);
     };
     std::vector<int> b{0};
     int l = 0;
