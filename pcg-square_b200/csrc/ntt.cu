@@ -1006,14 +1006,21 @@ struct OptinOnce {
 };
 OptinOnce g_optin;
 
-// Column tile width for a launch over `work` = columns x batch: the widest
-// one that still gives every SM its 1024 threads, else the narrowest.
+// Column tile width for a launch over `work` = columns x batch: the widest one
+// if that still gives every SM its 1024 threads, else 8 columns (64-byte row
+// segments) if that gives ctas8 CTAs, else 4.  ctas8 is one per SM for the
+// forward pass and three quarters of that for the inverse.  Products in us, with 4
+// columns below the first line / with this: 64 x 2^13 37.5 / 29.6 (4 columns are
+// half a warp there), 1 x 2^19 49.6 / 47.7, 2 x 2^19 63.4 / 60, 1 x 2^20 79.9 / 76,
+// three transforms of 2^19 and the checks 122.7 / 119.5.  With 8 columns below
+// that 1 x 2^14 goes from 18.5 to 20.5 and 1 x 2^18 (128 forward CTAs) from 32.8 to
+// 34.3; with 4 in the inverse pass of 2^19 (128 CTAs) it stays at 50.5.
 template <int L, int C = col_C(L), class F>
-void col_width(size_t work, F&& f) {
+void col_width(size_t work, size_t ctas8, F&& f) {
     if constexpr (C > col_C_min(L)) {
-        const size_t want = static_cast<size_t>(sm_count()) * (1024 / col_threads<L, C>());
-        if (work / C < want) {
-            col_width<L, C / 2>(work, f);
+        const size_t full = static_cast<size_t>(sm_count()) * (1024 / col_threads<L, C>());
+        if (work / C < (C > 8 ? full : ctas8)) {
+            col_width<L, C / 2>(work, ctas8, f);
             return;
         }
     }
@@ -1023,7 +1030,7 @@ void col_width(size_t work, F&& f) {
 template <int L>
 void col_fwd_l(const NttPlan& pl, const FwdIn& in, int count, int batch, bool chained,
                cudaStream_t st) {
-    col_width<L>(static_cast<size_t>(pl.n2) * batch * count, [&](auto CC) {
+    col_width<L>(static_cast<size_t>(pl.n2) * batch * count, sm_count(), [&](auto CC) {
         constexpr int C = decltype(CC)::value;
         constexpr size_t sm = col_smem<L, C>();
         auto go = [&](auto kernel) {
@@ -1037,7 +1044,7 @@ void col_fwd_l(const NttPlan& pl, const FwdIn& in, int count, int batch, bool ch
 
 template <int L>
 void col_inv_l(const NttPlan& pl, uint64_t* d, int batch, cudaStream_t st) {
-    col_width<L>(static_cast<size_t>(pl.n2) * batch, [&](auto CC) {
+    col_width<L>(static_cast<size_t>(pl.n2) * batch, sm_count() * 3 / 4, [&](auto CC) {
         constexpr int C = decltype(CC)::value;
         constexpr size_t sm = col_smem<L, C>();
         auto go = [&](auto kernel) {

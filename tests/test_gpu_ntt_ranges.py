@@ -79,3 +79,22 @@ def test_ole_check_counts_slots(pcg, logN):
         pcg.verify_ole_device(N, d0.ptr, dz.ptr, d1.ptr, dz1.ptr, bad.ptr)
         pcg.synchronize()
         assert int(bad.download(np.uint64, 1)[0]) == want
+
+
+# Batches on both sides of the column tile widths' steps (16, 8, 4 columns).
+@pytest.mark.parametrize("batch,logN", [(9, 13), (10, 13), (64, 13), (296, 13), (3, 14), (37, 14),
+                                        (5, 16), (2, 18), (1, 19), (2, 19)])
+def test_column_tile_widths(pcg, batch, logN):
+    N = 1 << logN
+    rng = np.random.default_rng(batch * 100 + logN)
+    a, b = (rng.integers(0, P, batch * N, dtype=np.uint64) for _ in range(2))
+    da, db = pcg.to_device(a), pcg.to_device(b)
+    c, one = pcg.DeviceBuffer(8 * batch * N), pcg.DeviceBuffer(8 * batch * N)
+    pcg.poly_mul_device(c.ptr, da.ptr, db.ptr, batch, N)
+    for k in range(batch):
+        o = 8 * k * N
+        pcg.poly_mul_device(one.ptr + o, da.ptr + o, db.ptr + o, 1, N)
+    pcg.synchronize()
+    got = c.download(np.uint64, batch * N)
+    assert (got == one.download(np.uint64, batch * N)).all()
+    assert (got[-N:] == O.poly_mul(a[-N:], b[-N:], N)).all()
