@@ -67,13 +67,14 @@ inline void pause() {
 }
 
 // Up to kHelpers threads running f(i, count), joined on destruction; fewer
-// (count) where the system gives fewer.
+// (count) where the system gives fewer.  The threads call the caller's own f,
+// which is declared before them and so outlives them: a temporary does not bind.
 struct Helpers {
     std::thread th[kHelpers];
     std::atomic<int> go{0};   // 0: not all started, then count
     int count = 0;
     template <class F>
-    Helpers(int want, const F& f) {
+    Helpers(int want, F& f) {
         try {
             for (; count < want; ++count) {
                 const int i = count;
@@ -95,9 +96,10 @@ struct Helpers {
 // f(c) for every chunk c < n, on helpers when the whole range is large.
 template <class F>
 void each_chunk(int n, size_t bytes, const F& f) {
-    Helpers h(bytes >= kLarge ? std::min(kHelpers, n) : 0, [&](int i, int of) {
+    auto share = [&](int i, int of) {
         for (int c = i; c < n; c += of) f(c);
-    });
+    };
+    Helpers h(bytes >= kLarge ? std::min(kHelpers, n) : 0, share);
     if (h.count == 0)
         for (int c = 0; c < n; ++c) f(c);
 }
@@ -269,17 +271,18 @@ void HostStage::download(void* const* dst, const size_t* len, int pieces, const 
                          std::memcpy(static_cast<char*>(dst[i]) + in, s.pinned + o + from, m);
                      });
         };
+        auto share = [&](int h, int of) {
+            for (int c = h; c < n; c += of) touch(c);
+            for (int c = h; c < n; c += of) {
+                int r;
+                while ((r = ready.load(std::memory_order_acquire)) <= c && r >= 0) pause();
+                if (r < 0) return;
+                move(c);
+            }
+        };
         cudaError_t err = cudaSuccess;
         {
-            Helpers helpers(total >= kLarge ? std::min(kHelpers, n) : 0, [&](int h, int of) {
-                for (int c = h; c < n; c += of) touch(c);
-                for (int c = h; c < n; c += of) {
-                    int r;
-                    while ((r = ready.load(std::memory_order_acquire)) <= c && r >= 0) pause();
-                    if (r < 0) return;
-                    move(c);
-                }
-            });
+            Helpers helpers(total >= kLarge ? std::min(kHelpers, n) : 0, share);
             if (helpers.count == 0)
                 for (int c = 0; c < n; ++c) touch(c);
             for (int c = 0; c < n && err == cudaSuccess; ++c) {

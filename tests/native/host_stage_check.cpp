@@ -1,0 +1,94 @@
+// Runs host_stage.cpp against a CUDA runtime of plain host memory: streams
+// complete at once, device pointers are host pointers.  Modes (argv[1]):
+//   move MB    an upload and a download of MB megabytes in three pieces
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+
+#include "pcgb_internal.h"
+
+namespace pcgb {
+void fail(int code, const std::string& msg) { throw Error(code, msg); }
+void check_cuda(cudaError_t e, const char* what) {
+    if (e != cudaSuccess) throw Error(PCGB_ECUDA, what);
+}
+}  // namespace pcgb
+
+extern "C" {
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
+    a->type = cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+    *e = reinterpret_cast<cudaEvent_t>(1);
+    return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+}
+
+namespace {
+
+const cudaStream_t kStream = reinterpret_cast<cudaStream_t>(8);
+
+// Three ragged pieces of `total` bytes and a "device" buffer of as many.
+struct Arrays {
+    std::vector<char> part[3], out[3], dev;
+    size_t len[3];
+    explicit Arrays(size_t total) : dev(total) {
+        len[0] = total / 3 + 5;
+        len[1] = total / 7;
+        len[2] = total - len[0] - len[1];
+        unsigned s = 12345;
+        for (int i = 0; i < 3; ++i) {
+            part[i].resize(len[i]);
+            for (auto& c : part[i]) c = static_cast<char>((s = s * 1664525u + 1013904223u) >> 24);
+            out[i].assign(len[i], 0x5a);
+        }
+    }
+};
+
+void expect(bool ok, const char* what) {
+    if (ok) return;
+    std::fprintf(stderr, "FAILED: %s\n", what);
+    std::exit(1);
+}
+
+void move(Arrays& a) {
+    const void* src[3];
+    void* dst[3];
+    for (int i = 0; i < 3; ++i) {
+        src[i] = a.part[i].data();
+        dst[i] = a.out[i].data();
+    }
+    pcgb::HostStage io;
+    io.upload(a.dev.data(), src, a.len, 3, kStream);
+    io.download(dst, a.len, 3, a.dev.data(), kStream);
+}
+
+int run_move(size_t mb) {
+    Arrays a(mb << 20);
+    move(a);
+    for (int i = 0; i < 3; ++i) expect(a.out[i] == a.part[i], "bytes after the round trip");
+    pcgb::HostStage::trim();
+    return 0;
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+    const std::string mode = argc > 1 ? argv[1] : "";
+    if (mode == "move" && argc > 2) return run_move(std::strtoul(argv[2], nullptr, 10));
+    return 2;
+}
