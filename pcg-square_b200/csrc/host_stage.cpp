@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <condition_variable>
 #include <cstring>
 #include <mutex>
 #include <system_error>
@@ -66,27 +67,18 @@ inline void pause() {
 #endif
 }
 
-// Up to kHelpers threads running f(i, count), joined on destruction; fewer
-// (count) where the system gives fewer.  The threads call the caller's own f,
-// which is declared before them and so outlives them: a temporary does not bind.
+// Up to kHelpers threads running f(), joined on destruction; fewer (count)
+// where the system gives fewer.  The threads call the caller's own f, which is
+// declared before them and so outlives them: a temporary does not bind.
 struct Helpers {
     std::thread th[kHelpers];
-    std::atomic<int> go{0};   // 0: not all started, then count
     int count = 0;
     template <class F>
     Helpers(int want, F& f) {
         try {
-            for (; count < want; ++count) {
-                const int i = count;
-                th[i] = std::thread([this, i, &f] {
-                    int of;
-                    while ((of = go.load(std::memory_order_acquire)) == 0) pause();
-                    f(i, of);
-                });
-            }
+            for (; count < want; ++count) th[count] = std::thread([&f] { f(); });
         } catch (const std::system_error&) {
         }
-        go.store(count ? count : -1, std::memory_order_release);
     }
     ~Helpers() {
         for (int i = 0; i < count; ++i) th[i].join();
@@ -96,13 +88,46 @@ struct Helpers {
 // f(c) for every chunk c < n, on helpers when the whole range is large.
 template <class F>
 void each_chunk(int n, size_t bytes, const F& f) {
-    auto share = [&](int i, int of) {
-        for (int c = i; c < n; c += of) f(c);
+    std::atomic<int> next{0};
+    auto share = [&] {
+        for (int c; (c = next.fetch_add(1, std::memory_order_relaxed)) < n;) f(c);
     };
     Helpers h(bytes >= kLarge ? std::min(kHelpers, n) : 0, share);
-    if (h.count == 0)
-        for (int c = 0; c < n; ++c) f(c);
+    if (h.count == 0) share();
 }
+
+// Chunks announced by the one thread that waits on the driver.  The others
+// look a few microseconds (chunks of a running copy are 20 us apart), then
+// sleep: the first chunk comes only after the call's kernels, 15 ms for an
+// expansion of 2^20.
+class Progress {
+  public:
+    // Chunks [0, r) are there; r < 0: no more will come.
+    void announce(int r) {
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            ready.store(r, std::memory_order_release);
+        }
+        cv.notify_all();
+    }
+    // Whether chunk c is there, waiting for it or for the end.
+    bool wait(int c) {
+        for (int k = 0; k < kLooks; ++k) {
+            const int r = ready.load(std::memory_order_acquire);
+            if (r > c || r < 0) return r > c;
+            pause();
+        }
+        std::unique_lock<std::mutex> lk(mu);
+        cv.wait(lk, [&] { return ready.load() > c || ready.load() < 0; });
+        return ready.load() > c;
+    }
+
+  private:
+    static constexpr int kLooks = 1000;
+    std::mutex mu;
+    std::condition_variable cv;
+    std::atomic<int> ready{0};
+};
 
 }  // namespace
 
@@ -256,7 +281,7 @@ void HostStage::download(void* const* dst, const size_t* len, int pieces, const 
         // Helpers take the page faults of their chunks while the device is at
         // work, then move each chunk as this thread, which alone waits on the
         // driver, announces it.
-        std::atomic<int> ready{0};
+        Progress progress;
         auto touch = [&](int c) {
             const size_t o = static_cast<size_t>(c) * kChunk, l = std::min(kChunk, round - o);
             parts_of(dst, len, pieces, at + o, at + o + l, [&](int i, size_t in, size_t, size_t m) {
@@ -271,12 +296,17 @@ void HostStage::download(void* const* dst, const size_t* len, int pieces, const 
                          std::memcpy(static_cast<char*>(dst[i]) + in, s.pinned + o + from, m);
                      });
         };
-        auto share = [&](int h, int of) {
-            for (int c = h; c < n; c += of) touch(c);
-            for (int c = h; c < n; c += of) {
-                int r;
-                while ((r = ready.load(std::memory_order_acquire)) <= c && r >= 0) pause();
-                if (r < 0) return;
+        std::atomic<int> next{0};
+        auto share = [&] {
+            static_assert(kChunks <= 32, "a bit per chunk");
+            uint32_t mine = 0;   // a chunk is moved by the thread that touched it
+            for (int c; (c = next.fetch_add(1, std::memory_order_relaxed)) < n;) {
+                touch(c);
+                mine |= uint32_t{1} << c;
+            }
+            for (int c = 0; c < n; ++c) {
+                if (!(mine >> c & 1)) continue;
+                if (!progress.wait(c)) return;
                 move(c);
             }
         };
@@ -287,7 +317,7 @@ void HostStage::download(void* const* dst, const size_t* len, int pieces, const 
                 for (int c = 0; c < n; ++c) touch(c);
             for (int c = 0; c < n && err == cudaSuccess; ++c) {
                 err = cudaEventSynchronize(s.ev[c]);
-                ready.store(err == cudaSuccess ? c + 1 : -1, std::memory_order_release);
+                progress.announce(err == cudaSuccess ? c + 1 : -1);
                 if (helpers.count == 0 && err == cudaSuccess) move(c);
             }
         }

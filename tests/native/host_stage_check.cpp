@@ -1,9 +1,14 @@
 // Runs host_stage.cpp against a CUDA runtime of plain host memory: streams
 // complete at once, device pointers are host pointers.  Modes (argv[1]):
 //   move MB    an upload and a download of MB megabytes in three pieces
+//   idle MB    processor time of a download whose first chunk comes after 300 ms
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <atomic>
+#include <chrono>
+#include <ctime>
+#include <thread>
 #include <vector>
 
 #include "pcgb_internal.h"
@@ -14,6 +19,8 @@ void check_cuda(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw Error(PCGB_ECUDA, what);
 }
 }  // namespace pcgb
+
+static std::atomic<int> event_delay_ms{0};   // of the next event wait
 
 extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
@@ -35,7 +42,10 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
     return cudaSuccess;
 }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) {
+    std::this_thread::sleep_for(std::chrono::milliseconds(event_delay_ms.exchange(0)));
+    return cudaSuccess;
+}
 }
 
 namespace {
@@ -85,10 +95,25 @@ int run_move(size_t mb) {
     return 0;
 }
 
+// Four threads that wait by spinning would burn 1200 ms; touching and copying
+// 16 MB takes 10 to 30.
+int run_idle(size_t mb) {
+    Arrays a(mb << 20);
+    move(a);   // threads, pages and the buffer are warm
+    event_delay_ms = 300;
+    const std::clock_t t0 = std::clock();   // all threads of the process
+    move(a);
+    const double ms = 1e3 * static_cast<double>(std::clock() - t0) / CLOCKS_PER_SEC;
+    std::fprintf(stderr, "%.1f ms of processor time\n", ms);
+    expect(ms < 150, "helpers sleep while the device works");
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "move" && argc > 2) return run_move(std::strtoul(argv[2], nullptr, 10));
+    if (mode == "idle" && argc > 2) return run_idle(std::strtoul(argv[2], nullptr, 10));
     return 2;
 }

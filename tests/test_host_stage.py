@@ -34,3 +34,12 @@ def sanitized(tmp_path_factory):
 @pytest.mark.parametrize("mb", [1, 9, 17, 40])
 def test_transfers_within_lifetimes(sanitized, mb):
     run(sanitized, "move", str(mb))
+
+
+@pytest.fixture(scope="module")
+def plain(tmp_path_factory):
+    return build(tmp_path_factory.mktemp("plain"), "-O2")
+
+
+def test_helpers_sleep_while_the_device_works(plain):
+    run(plain, "idle", "16")
