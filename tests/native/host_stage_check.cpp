@@ -1,6 +1,7 @@
 // Runs host_stage.cpp against a CUDA runtime of plain host memory: streams
 // complete at once, device pointers are host pointers.  Modes (argv[1]):
 //   move MB    an upload and a download of MB megabytes in three pieces
+//   threads MB  as move, where only N threads can be had, N = 0 .. 4
 //   idle MB    processor time of a download whose first chunk comes after 300 ms
 #include <cstdio>
 #include <cstdlib>
@@ -8,6 +9,7 @@
 #include <atomic>
 #include <chrono>
 #include <ctime>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -21,6 +23,17 @@ void check_cuda(cudaError_t e, const char* what) {
 }  // namespace pcgb
 
 static std::atomic<int> event_delay_ms{0};   // of the next event wait
+// Allocations until one throws (those of a transfer are its threads' states); < 0: none does.
+static thread_local int allocations_left = -1;
+
+void* operator new(std::size_t n) {
+    if (allocations_left == 0) throw std::bad_alloc();
+    if (allocations_left > 0) --allocations_left;
+    if (void* p = std::malloc(n)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
 
 extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
@@ -95,6 +108,26 @@ int run_move(size_t mb) {
     return 0;
 }
 
+int run_threads(size_t mb) {
+    for (int threads = 0; threads <= 4; ++threads) {
+        Arrays a(mb << 20);
+        const void* src[3];
+        void* dst[3];
+        for (int i = 0; i < 3; ++i) {
+            src[i] = a.part[i].data();
+            dst[i] = a.out[i].data();
+        }
+        pcgb::HostStage io;
+        allocations_left = threads;
+        io.upload(a.dev.data(), src, a.len, 3, kStream);
+        allocations_left = threads;
+        io.download(dst, a.len, 3, a.dev.data(), kStream);
+        allocations_left = -1;
+        for (int i = 0; i < 3; ++i) expect(a.out[i] == a.part[i], "bytes with fewer threads");
+    }
+    return 0;
+}
+
 // Four threads that wait by spinning would burn 1200 ms; touching and copying
 // 16 MB takes 10 to 30.
 int run_idle(size_t mb) {
@@ -114,6 +147,7 @@ int run_idle(size_t mb) {
 int main(int argc, char** argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "move" && argc > 2) return run_move(std::strtoul(argv[2], nullptr, 10));
+    if (mode == "threads" && argc > 2) return run_threads(std::strtoul(argv[2], nullptr, 10));
     if (mode == "idle" && argc > 2) return run_idle(std::strtoul(argv[2], nullptr, 10));
     return 2;
 }

@@ -43,3 +43,7 @@ def plain(tmp_path_factory):
 
 def test_helpers_sleep_while_the_device_works(plain):
     run(plain, "idle", "16")
+
+
+def test_a_thread_that_cannot_be_had(plain):
+    run(plain, "threads", "17")
