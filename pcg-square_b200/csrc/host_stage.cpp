@@ -17,6 +17,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <thread>
 
@@ -136,10 +137,12 @@ struct HostStage::Impl {
     std::unique_lock<std::mutex> lk;
 };
 
-HostStage::HostStage() : im(new Impl) {
-    im->s = &stage_for_device(&im->dev);
-    im->lk = std::unique_lock<std::mutex>(im->s->mu, std::try_to_lock);
-    usable = im->lk.owns_lock();
+HostStage::HostStage() {
+    auto p = std::make_unique<Impl>();
+    p->s = &stage_for_device(&p->dev);
+    p->lk = std::unique_lock<std::mutex>(p->s->mu, std::try_to_lock);
+    usable = p->lk.owns_lock();
+    im = p.release();
 }
 
 // Makes the buffer hold a transfer of `total` bytes (kSmall, or kStageBytes
@@ -210,6 +213,8 @@ void HostStage::upload(void* d_dst, const void* const* src, const size_t* len, i
     }
     direct = direct || !reserve(total);
     if (direct) {
+        if (pending && pending != st) check_cuda(cudaStreamSynchronize(pending), "host upload");
+        pending = st;   // pinned sources are read until the stream gets there
         size_t o = 0;
         for (int i = 0; i < pieces; ++i) {
             check_cuda(cudaMemcpyAsync(static_cast<char*>(d_dst) + o, src[i], len[i],
@@ -256,6 +261,8 @@ void HostStage::download(void* const* dst, const size_t* len, int pieces, const 
         direct = direct || (len[i] && is_pinned(dst[i]));
     }
     direct = direct || !reserve(total);
+    if (pending && pending != st) check_cuda(cudaStreamSynchronize(pending), "host download");
+    pending = st;   // until the end: a failure leaves copies queued
     if (direct) {
         size_t o = 0;
         for (int i = 0; i < pieces; ++i) {
@@ -264,10 +271,11 @@ void HostStage::download(void* const* dst, const size_t* len, int pieces, const 
             o += len[i];
         }
         check_cuda(cudaStreamSynchronize(st), "host download");
+        pending = nullptr;
+        used = 0;
         return;
     }
     Stage& s = *im->s;
-    if (pending && pending != st) check_cuda(cudaStreamSynchronize(pending), "host download");
     for (size_t at = 0; at < total; at += s.bytes) {
         const size_t round = std::min(s.bytes, total - at);
         const int n = static_cast<int>((round + kChunk - 1) / kChunk);

@@ -57,9 +57,11 @@ inline cudaStream_t as_stream(void* s) {
 // Host buffers to and from the device through a pinned buffer (host_stage.cpp).
 // One object per call: it holds the device's buffer until it goes out of scope
 // (another thread's call then copies directly).  `pieces` host ranges of len
-// bytes each make up one contiguous device range.  upload: the sources may be
-// reused on return.  download: waits for everything queued on the stream,
-// the pieces are complete on return; call it last.
+// bytes each make up one contiguous device range.  upload: the sources stay
+// valid until download returns or the object is gone (pinned ones are read by
+// the device until then).  download: waits for everything queued on the stream,
+// the pieces are complete on return; call it last.  An object that goes out of
+// scope before, on an error, waits for the copies it queued.
 class HostStage {
   public:
     HostStage();
@@ -75,10 +77,10 @@ class HostStage {
   private:
     bool reserve(size_t total);
     struct Impl;
-    Impl* im;
+    Impl* im = nullptr;
     bool usable = false;
     size_t used = 0;                  // bytes of the buffer that copies may still read
-    cudaStream_t pending = nullptr;   // their stream
+    cudaStream_t pending = nullptr;   // the stream with copies that may not have ended
 };
 void upload_blocking(void* d_dst, const void* src, size_t bytes);
 // Stream-ordered allocation from the library's own per-device pool, which

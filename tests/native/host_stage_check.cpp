@@ -2,6 +2,7 @@
 // complete at once, device pointers are host pointers.  Modes (argv[1]):
 //   move MB    an upload and a download of MB megabytes in three pieces
 //   threads MB  as move, where only N threads can be had, N = 0 .. 4
+//   failed MB  transfers that fail half way leave nothing in flight
 //   idle MB    processor time of a download whose first chunk comes after 300 ms
 #include <cstdio>
 #include <cstdlib>
@@ -23,6 +24,9 @@ void check_cuda(cudaError_t e, const char* what) {
 }  // namespace pcgb
 
 static std::atomic<int> event_delay_ms{0};   // of the next event wait
+static std::atomic<int> events_left{-1};     // event waits until one fails; < 0: none does
+static std::atomic<int> in_flight{0};        // copies the stream was not waited for since
+static const void* pinned_at = nullptr;      // an address that counts as pinned memory
 // Allocations until one throws (those of a transfer are its threads' states); < 0: none does.
 static thread_local int allocations_left = -1;
 
@@ -39,17 +43,21 @@ extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
-    a->type = cudaMemoryTypeUnregistered;
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+    a->type = p == pinned_at ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
     return cudaSuccess;
 }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
     std::memcpy(d, s, n);
+    ++in_flight;
     return cudaSuccess;
 }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) {
+    in_flight = 0;
+    return cudaSuccess;
+}
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
     *e = reinterpret_cast<cudaEvent_t>(1);
     return cudaSuccess;
@@ -57,6 +65,8 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) {
     std::this_thread::sleep_for(std::chrono::milliseconds(event_delay_ms.exchange(0)));
+    if (events_left == 0) return cudaErrorUnknown;
+    if (events_left > 0) --events_left;
     return cudaSuccess;
 }
 }
@@ -128,6 +138,38 @@ int run_threads(size_t mb) {
     return 0;
 }
 
+int run_failed(size_t mb) {
+    Arrays a(mb << 20);
+    const void* src[3];
+    void* dst[3];
+    for (int i = 0; i < 3; ++i) {
+        src[i] = a.part[i].data();
+        dst[i] = a.out[i].data();
+    }
+    pinned_at = src[1];
+    {
+        pcgb::HostStage io;   // a call that fails between its upload and its download
+        io.upload(a.dev.data(), src, a.len, 3, kStream);
+        expect(in_flight > 0, "the upload is queued");
+    }
+    expect(in_flight == 0, "copies from pinned sources have ended");
+    pinned_at = nullptr;
+    for (int good = 0; good < 2; ++good) {
+        bool thrown = false;
+        try {
+            pcgb::HostStage io;
+            events_left = good;
+            io.download(dst, a.len, 3, a.dev.data(), kStream);
+        } catch (const pcgb::Error&) {
+            thrown = true;
+        }
+        events_left = -1;
+        expect(thrown, "the error is reported");
+        expect(in_flight == 0, "copies into the buffer have ended");
+    }
+    return 0;
+}
+
 // Four threads that wait by spinning would burn 1200 ms; touching and copying
 // 16 MB takes 10 to 30.
 int run_idle(size_t mb) {
@@ -148,6 +190,7 @@ int main(int argc, char** argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "move" && argc > 2) return run_move(std::strtoul(argv[2], nullptr, 10));
     if (mode == "threads" && argc > 2) return run_threads(std::strtoul(argv[2], nullptr, 10));
+    if (mode == "failed" && argc > 2) return run_failed(std::strtoul(argv[2], nullptr, 10));
     if (mode == "idle" && argc > 2) return run_idle(std::strtoul(argv[2], nullptr, 10));
     return 2;
 }

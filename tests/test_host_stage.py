@@ -47,3 +47,8 @@ def test_helpers_sleep_while_the_device_works(plain):
 
 def test_a_thread_that_cannot_be_had(plain):
     run(plain, "threads", "17")
+
+
+@pytest.mark.parametrize("mb", [3, 17])
+def test_failed_transfers_leave_nothing_in_flight(sanitized, mb):
+    run(sanitized, "failed", str(mb))
