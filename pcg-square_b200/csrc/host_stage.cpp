@@ -286,14 +286,14 @@ void HostStage::download(void* const* dst, const size_t* len, int pieces, const 
             check_cuda(cudaEventRecord(s.ev[c], st), "host download");
         }
         // Helpers take the page faults of their chunks while the device is at
-        // work, then move each chunk as this thread, which alone waits on the
-        // driver, announces it.
+        // work (a write that keeps the byte), then move each chunk as this thread,
+        // which alone waits on the driver, announces it.
         Progress progress;
         auto touch = [&](int c) {
             const size_t o = static_cast<size_t>(c) * kChunk, l = std::min(kChunk, round - o);
             parts_of(dst, len, pieces, at + o, at + o + l, [&](int i, size_t in, size_t, size_t m) {
-                volatile char* p = static_cast<char*>(dst[i]) + in;
-                for (size_t k = 0; k < m; k += kPage) p[k] = 0;
+                char* p = static_cast<char*>(dst[i]) + in;
+                for (size_t k = 0; k < m; k += kPage) __atomic_fetch_or(p + k, 0, __ATOMIC_RELAXED);
             });
         };
         auto move = [&](int c) {

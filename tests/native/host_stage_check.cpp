@@ -166,6 +166,12 @@ int run_failed(size_t mb) {
         events_left = -1;
         expect(thrown, "the error is reported");
         expect(in_flight == 0, "copies into the buffer have ended");
+        // Chunks that did not come leave their part of the outputs alone.
+        size_t at = 0;
+        for (int i = 0; i < 3; ++i)
+            for (size_t k = 0; k < a.len[i]; ++k, ++at)
+                expect(at < static_cast<size_t>(good) << 20 || a.out[i][k] == 0x5a,
+                       "outputs a failed call does not reach");
     }
     return 0;
 }
