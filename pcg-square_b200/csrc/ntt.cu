@@ -19,7 +19,7 @@
 //
 // Each sub-transform is the merged-twist Cooley-Tukey (forward) /
 // Gentleman-Sande (inverse) negacyclic NTT of Longa and Naehrig (CANS 2016,
-// Algorithms 1-2).  Values are signed and lazily reduced: |v| < 2p < 2^63,
+// Algorithms 1-2).  Values are signed and lazily reduced: |v| <= 1.7p < 2^63,
 // with products by table entries in (-0.05p, 1.05p) (ntt_arith.cuh).  What
 // bounds the passes is the multiplier pipe together with the register ports
 // it shares with the integer ALU: a butterfly is about 19 instructions (5
@@ -91,51 +91,6 @@ struct NttPlan {
 };
 
 namespace {
-
-// ---- butterflies -------------------------------------------------------------
-// Values are signed and lazily reduced (ntt_arith.cuh): a product t lies in
-// [-e p, (1 + e)p], e < 0.05, for a factor below 1.7p in magnitude.
-
-// Forward butterfly X + wY, X - wY.  A stage with FOLD brings X back first;
-// the next one adds another product to that, shifted by p so that the range
-// stays centred, which needs the role the element had in the last stage:
-//   FIRST  X in [-e, 1 + e]p           -> both within (1 + 2e)p
-//   FOLD   |X| < 1.75p, folded to +-p/2 -> X' in [-1/2 - e, 3/2 + e]p, Y' in
-//                                         its negative
-//   XROLE  X an X' of a FOLD stage     -> both within (1.5 + 2e)p
-//   YROLE  X a Y' of a FOLD stage      -> both within (1.5 + 2e)p
-enum CtKind { kCtFirst, kCtFold, kCtXRole, kCtYRole };
-__device__ __forceinline__ void ct_bfly(int64_t& X, int64_t& Y, const NttTw& w, CtKind kind) {
-    const int64_t x = kind == kCtFold ? fold_centred(X) : X;
-    const int64_t t = mul_tw(Y, w);
-    X = (kind == kCtFirst || kind == kCtXRole) ? x + t - kPs : x + t;
-    Y = kind == kCtYRole ? x - t + kPs : x - t;
-}
-// Stage q of a phase starting at stage s0: phase 0 begins on reduced values
-// and folds at q = 1, 3; later phases fold at q = 0, 2.  xrole: the X operand
-// was an X' of the previous stage.
-__host__ __device__ constexpr CtKind ct_kind(int s0, int q, bool xrole) {
-    if (s0 + q == 0) return kCtFirst;
-    if ((q & 1) == (s0 == 0 ? 1 : 0)) return kCtFold;
-    return xrole ? kCtXRole : kCtYRole;
-}
-
-// Inverse butterfly: X, Y in [-0.25p, 1.25p] -> X + Y in [0, p] up to 2d,
-// (X - Y) w in [-e p, (1 + e)p].
-__device__ __forceinline__ void gs_bfly(int64_t& X, int64_t& Y, const NttTw& w) {
-    const int64_t s = fold(X + Y - kPs);
-    Y = mul_tw(X - Y, w);
-    X = s;
-}
-
-// Butterfly of a stage whose root has been folded into the per-element
-// twiddles (the row pass's first forward stage and last inverse stage):
-// X, Y in [-e p, (1 + e)p] -> X + Y, X - Y within (1 + 2e)p.
-__device__ __forceinline__ void add_sub_bfly(int64_t& X, int64_t& Y) {
-    const int64_t s = X + Y - kPs;
-    Y = X - Y;
-    X = s;
-}
 
 __device__ __forceinline__ NttTw ldtw(const NttTw* __restrict__ w) {
     const int4 v = __ldg(reinterpret_cast<const int4*>(w));
@@ -332,7 +287,7 @@ __device__ __forceinline__ T pick(T const (&v)[3], int z) {
 // Any 64-bit word (plus another) as a residue in [0, p] up to 3d.
 __device__ __forceinline__ int64_t load_raw(const uint64_t* src, const uint64_t* add, size_t i) {
     int64_t v = fold_raw(src[i]);
-    if (add) v = fold(v + fold_raw(add[i]) - kPs);
+    if (add) v = fold(add_shift(v, fold_raw(add[i])));
     return v;
 }
 
@@ -438,7 +393,7 @@ __device__ __forceinline__ void row_inv_body(const uint64_t* g, const uint64_t* 
 #pragma unroll
             for (int e = 0; e < E; ++e) {
                 const int64_t y = valid ? static_cast<int64_t>(g[perm_pos<L>(eidx<L, LP>(t, e))]) : 0;
-                x[e] = fold(x[e] + y - kPs);
+                x[e] = fold(add_shift(x[e], y));
             }
         }
     }

@@ -19,8 +19,9 @@
 // 2^31 < 2^61, so M >> 30 fits 32 bits; times d < 2^26.6 it adds at most
 // 2^57.6 to the 62-bit remainder.
 //
-// Values between butterflies are signed 64-bit with |v| < 2p (2p < 2^63).
-// fold() brings one back to [0, p] up to 2d with one IMAD.WIDE.
+// Values between butterflies are signed 64-bit with |v| <= 1.7p, inside the
+// range of mul_tw and mul_var.  fold() brings one back to [0, p] up to 2d with one
+// IMAD.WIDE.
 #ifndef PCGB_NTT_ARITH_CUH_
 #define PCGB_NTT_ARITH_CUH_
 
@@ -129,6 +130,59 @@ PCGB_HD int64_t mul_var(int64_t a, int64_t b) {
 PCGB_HD uint64_t canon(int64_t v) {
     uint64_t u = static_cast<uint64_t>(v + ((v >> 63) & kPs));
     return u >= kPm ? u - kPm : u;
+}
+
+// ---- butterflies -------------------------------------------------------------
+// Values are signed and lazily reduced: a product t lies in [-e p, (1 + e)p],
+// e < 0.05, for a factor of at most 1.7p in magnitude.
+
+// a + b - p for values whose plain sum may pass 2^63: 2p is only 2d below it.
+// (Here and in the butterflies p goes in before the second operand, so that no
+// intermediate leaves the signed range.)
+PCGB_HD int64_t add_shift(int64_t a, int64_t b) { return a - kPs + b; }
+
+// Forward butterfly X + wY, X - wY.  A stage with FOLD brings X back first;
+// the next one adds another product to that, shifted by p so that the range
+// stays centred, which needs the role the element had in the last stage:
+//   FIRST  X in [-e, 1 + e]p           -> both within (1 + 2e)p
+//   FOLD   |X| < 1.75p, folded to +-p/2 -> X' in [-1/2 - e, 3/2 + e]p, Y' in
+//                                         its negative
+//   XROLE  X an X' of a FOLD stage     -> both within (1.5 + 2e)p
+//   YROLE  X a Y' of a FOLD stage      -> both within (1.5 + 2e)p
+enum CtKind { kCtFirst, kCtFold, kCtXRole, kCtYRole };
+PCGB_HD void ct_bfly(int64_t& X, int64_t& Y, const NttTw& w, CtKind kind) {
+    const int64_t x = kind == kCtFold ? fold_centred(X) : X;
+    const int64_t t = mul_tw(Y, w);
+    X = (kind == kCtFirst || kind == kCtXRole) ? add_shift(x, t) : x + t;
+    Y = kind == kCtYRole ? x + kPs - t : x - t;
+}
+// Stage q of a phase starting at stage s0: phase 0 begins on reduced values
+// and folds at q = 1, 3; later phases fold at q = 0, 2.  xrole: the X operand
+// was an X' of the previous stage.
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+constexpr CtKind ct_kind(int s0, int q, bool xrole) {
+    if (s0 + q == 0) return kCtFirst;
+    if ((q & 1) == (s0 == 0 ? 1 : 0)) return kCtFold;
+    return xrole ? kCtXRole : kCtYRole;
+}
+
+// Inverse butterfly: X, Y in [-0.25p, 1.25p] -> X + Y in [0, p] up to 2d,
+// (X - Y) w in [-e p, (1 + e)p].
+PCGB_HD void gs_bfly(int64_t& X, int64_t& Y, const NttTw& w) {
+    const int64_t s = fold(add_shift(X, Y));
+    Y = mul_tw(X - Y, w);
+    X = s;
+}
+
+// Butterfly of a stage whose root has been folded into the per-element
+// twiddles (the row pass's first forward stage and last inverse stage):
+// X, Y in [-e p, (1 + e)p] -> X + Y, X - Y within (1 + 2e)p.
+PCGB_HD void add_sub_bfly(int64_t& X, int64_t& Y) {
+    const int64_t s = add_shift(X, Y);
+    Y = X - Y;
+    X = s;
 }
 
 }  // namespace pcgb
