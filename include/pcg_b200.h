@@ -333,7 +333,8 @@ int pcgb_expander_shard(const pcgb_expander* e, int* rank, int* world, int* pair
 int pcgb_reduce_mod_p(uint64_t* d, const uint64_t* s, size_t count, void* stream);
 /* One party's expansion from device-resident inputs:
  *   d_roots[K], d_cws[K*levels*nk], d_cw_out[K], d_pos[c*t], d_val[c*t]
- *   -> d_x[N], d_z[N] (x = sum a_i e_i, z = sum_{i,j} a_i a_j g_ij). */
+ *   -> d_x[N], d_z[N] (x = sum a_i e_i, z = sum_{i,j} a_i a_j g_ij).
+ * d_x may lie over the keys (roots, cws, cw_out), d_z over any input. */
 int pcgb_expand_device(pcgb_expander* e, int party, const pcgb_blk* d_roots,
                        const pcgb_blk* d_cws, const uint64_t* d_cw_out, const uint64_t* d_pos,
                        const uint64_t* d_val, uint64_t* d_x, uint64_t* d_z, void* stream);

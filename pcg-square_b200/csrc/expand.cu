@@ -24,6 +24,7 @@
 
 #include "chain.cuh"
 #include "field.cuh"
+#include "ranges.h"
 #include "synth.h"
 
 namespace pcgb {
@@ -90,7 +91,8 @@ __global__ void x_kernel(const uint64_t* __restrict__ pos, const uint64_t* __res
                          uint64_t* __restrict__ x) {
     extern __shared__ uint64_t nz[];
     // x depends only on the call's inputs: it fills what the leaf kernel's last
-    // wave leaves free, and waits for it at the end.
+    // wave leaves free, and waits for it at the end (chained only where x meets
+    // nothing the kernels before it read).
     chain_release();
     x_body(pos, val, aR, c, t, i0, N, x, blockIdx.x, nz);
     chain_wait();
@@ -393,6 +395,16 @@ Workspace workspace_carve(const pcgb_expander* e, void* base) {
     return ws;
 }
 
+// The keys the walk and the leaf kernel read.  x over one of them (a caller that
+// is done with its keys may reuse their memory) must wait for both kernels.
+static std::array<Range, 3> key_ranges(const pcgb_expander* e, const Blk* roots, const Blk* cws,
+                                       const uint64_t* cw_out) {
+    const size_t K = static_cast<size_t>(e->K);
+    return {range_of(roots, K * sizeof(Blk)),
+            range_of(cws, K * e->levels * e->nk * sizeof(Blk)),
+            range_of(cw_out, K * sizeof(uint64_t))};
+}
+
 // fork (while a graph is captured): x becomes a branch of its own beside the
 // walk and the leaf kernel, which leave the multiplier pipe and the L2 idle (its
 // 0.14 ms of the headline's 15.06, 4 of the 39 us at N = 2^12).  Launched directly
@@ -407,6 +419,13 @@ static void expand_stages(pcgb_expander* e, const Workspace& ws, int party, cons
     cudaEvent_t* ev = nullptr;
     if (e->prof_slots > 0 && e->prof_used < e->prof_slots) ev = &e->prof_ev[5 * e->prof_used++];
     const size_t sm = sizeof(uint64_t) * 2 * static_cast<size_t>(e->c) * e->t;
+    const size_t noise = sizeof(uint64_t) * static_cast<size_t>(e->c) * e->t;
+    const Range rx = range_of(x, NN * sizeof(uint64_t)), rz = range_of(z, NN * sizeof(uint64_t));
+    bool early = true;   // x may be written while the keys are still read
+    for (const Range& r : key_ranges(e, roots, cws, cw_out)) early = early && !overlap(rx, r);
+    // A branch also runs beside the kernel that writes z.
+    if (!early || overlap(rz, range_of(pos, noise)) || overlap(rz, range_of(val, noise)))
+        fork = nullptr;
     if (fork) {
         PCGB_CK(cudaEventRecord(fork->begin, st));
         PCGB_CK(cudaStreamWaitEvent(fork->side, fork->begin, 0));
@@ -420,7 +439,7 @@ static void expand_stages(pcgb_expander* e, const Workspace& ws, int party, cons
     keyed_leaf_gather(e->gp, party, e->prg, ws.F, cws, cw_out, e->d_rk, ws.g, st);
     if (ev) PCGB_CK(cudaEventRecord(ev[2], st));
     if (!fork)
-        launch({blocks_for(NN, 256), 256, sm, true}, st, x_kernel, pos, val, e->d_aR, e->c, e->t,
+        launch({blocks_for(NN, 256), 256, sm, early}, st, x_kernel, pos, val, e->d_aR, e->c, e->t,
                e->i0, NN, x);
     if (ev) PCGB_CK(cudaEventRecord(ev[3], st));
     if (e->gp.Qs > 0) ntt_mac_inverse(*e->ntt, ws.g, e->d_img, e->gp.Qs, z, st);
@@ -486,6 +505,7 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
     std::vector<XJob> xj(count);
     unsigned x_ctas = 0;
     size_t x_smem = 0;
+    std::vector<Range> outs, keys;
     for (int i = 0; i < count; ++i) {
         const pcgb_expander* E = e[i];
         LeafJob& L = leaf[i];
@@ -504,6 +524,8 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
         X.first = x_ctas;
         x_ctas += blocks_for(X.N, 256);
         x_smem = std::max(x_smem, sizeof(uint64_t) * 2 * static_cast<size_t>(E->c) * E->t);
+        outs.push_back(range_of(x[i], X.N * sizeof(uint64_t)));
+        for (const Range& k : key_ranges(E, roots[i], cws[i], cw_out[i])) keys.push_back(k);
     }
     char* tab = static_cast<char*>(pool_alloc(sizeof(XJob) * count, st));
     PCGB_CK(cudaMemcpyAsync(tab, xj.data(), sizeof(XJob) * count, cudaMemcpyHostToDevice, st));
@@ -519,7 +541,7 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
     lsplit = std::min(lsplit, leaf_lsplit(leaves, S, t_max));
     keyed_leaf_multi_chacha(w, sl, leaf.data(), count, lsplit, tpb, leaf_smem, nullptr, nullptr, st);
     // Stage 3: the sparse x products.
-    launch({x_ctas, 256, x_smem, true}, st, x_multi_kernel, reinterpret_cast<const XJob*>(tab), count);
+    launch({x_ctas, 256, x_smem, !any_overlap(outs, keys)}, st, x_multi_kernel, reinterpret_cast<const XJob*>(tab), count);
     // Stage 4: NTT multiply-accumulate and inverse, all lengths at once.
     std::vector<uint64_t*> g(count), zz(count);
     std::vector<const uint64_t*> img(count);
@@ -921,7 +943,9 @@ void expand_from_g_device(pcgb_expander* e, const uint64_t* g, const uint64_t* p
     pair_merge_kernel<<<dim3(blocks_for(NN, 256), e->Q), 256, 0, st>>>(g, e->c, NN, e->d_g);
     PCGB_POST_LAUNCH();
     const size_t sm = sizeof(uint64_t) * 2 * static_cast<size_t>(e->c) * e->t;
-    launch({blocks_for(NN, 256), 256, sm, true}, st, x_kernel, pos, val, e->d_aR, e->c, e->t, e->i0,
+    const size_t words = NN * sizeof(uint64_t);
+    const bool early = !overlap(range_of(x, words), range_of(g, words * e->c * e->c));
+    launch({blocks_for(NN, 256), 256, sm, early}, st, x_kernel, pos, val, e->d_aR, e->c, e->t, e->i0,
            NN, x);
     ntt_mac_inverse(*e->ntt, e->d_g, e->d_img, e->Q, z, st);
 }

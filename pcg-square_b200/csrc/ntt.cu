@@ -67,6 +67,7 @@
 #include "chain.cuh"
 #include "field.cuh"
 #include "ntt_arith.cuh"
+#include "ranges.h"
 
 namespace pcgb {
 
@@ -1168,11 +1169,6 @@ FwdIn fwd_two(const uint64_t* s0, uint64_t* d0, const uint64_t* s1, uint64_t* d1
     return in;
 }
 
-bool overlap(const uint64_t* a, size_t na, const uint64_t* b, size_t nb) {
-    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-    return x < y + nb * sizeof(uint64_t) && y < x + na * sizeof(uint64_t);
-}
-
 }  // namespace
 
 const NttPlan& ntt_plan(int logN) {
@@ -1253,8 +1249,8 @@ void poly_mul_device(const NttPlan& pl, uint64_t* c, const uint64_t* a, const ui
     auto product = [&](size_t first, int count, cudaStream_t s) {
         uint64_t *A = scratch + first, *C = c + first;
         const uint64_t *x = a + first, *y = b + first;
-        const size_t n = static_cast<size_t>(count) * pl.N;
-        if (overlap(C, n, x, n)) {
+        const size_t n = static_cast<size_t>(count) * pl.N * sizeof(uint64_t);
+        if (overlap(range_of(C, n), range_of(x, n))) {
             col_fwd(pl, fwd_one(x, A), 1, count, false, s);
             col_fwd(pl, fwd_one(y, C), 1, count, true, s);
         } else {
@@ -1304,23 +1300,12 @@ void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const*
     }
     // Both operands' column passes share a launch unless some output
     // overlaps a first operand (which must then be read before).
-    bool alias = false;
-    {
-        std::vector<std::pair<uintptr_t, uintptr_t>> ra(count), rc(count);
-        for (int i = 0; i < count; ++i) {
-            const uintptr_t len = sizeof(uint64_t) << logN[i];
-            ra[i] = {reinterpret_cast<uintptr_t>(a[i]), reinterpret_cast<uintptr_t>(a[i]) + len};
-            rc[i] = {reinterpret_cast<uintptr_t>(c[i]), reinterpret_cast<uintptr_t>(c[i]) + len};
-        }
-        std::sort(ra.begin(), ra.end());
-        // Furthest end of the operands that start at or before each one.
-        std::vector<uintptr_t> end(count);
-        for (int i = 0; i < count; ++i) end[i] = i ? std::max(end[i - 1], ra[i].second) : ra[i].second;
-        for (const auto& r : rc) {
-            const auto it = std::lower_bound(ra.begin(), ra.end(), std::make_pair(r.second, uintptr_t{0}));
-            if (it != ra.begin() && end[it - ra.begin() - 1] > r.first) alias = true;
-        }
+    std::vector<Range> outs(count), firsts(count);
+    for (int i = 0; i < count; ++i) {
+        outs[i] = range_of(c[i], sizeof(uint64_t) << logN[i]);
+        firsts[i] = range_of(a[i], sizeof(uint64_t) << logN[i]);
     }
+    const bool alias = any_overlap(outs, firsts);
     // Longest products first, so the last CTAs of each pass are short ones.
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return logN[x] > logN[y]; });
     std::vector<MixedPoly> polys(count);
