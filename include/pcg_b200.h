@@ -266,7 +266,7 @@ int pcgb_aes_tree_round_keys(const uint8_t master[16], int nk, uint8_t* round_ke
  * A keyed instance: root, CW[level][0..2^w-1) (the last child's CW is their
  * XOR), and for the output layer one field element cw_out.  Both parties
  * hold the same CWs; roots differ by Delta. */
-/* Full-domain leaves of K keys: d_leaves[K][2^n]. */
+/* Full-domain leaves of K keys: d_leaves[K][2^n]; d_roots may lie in d_leaves. */
 int pcgb_dpf_keyed_full_eval(int K, int n, int w, int prg, const pcgb_blk* d_roots,
                              const pcgb_blk* d_cws, const uint8_t* round_keys,
                              pcgb_blk* d_leaves, void* stream);

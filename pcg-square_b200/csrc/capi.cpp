@@ -12,6 +12,7 @@
 
 #include "pcg_b200.h"
 #include "pcgb_internal.h"
+#include "ranges.h"
 
 namespace pcgb {
 
@@ -608,11 +609,21 @@ int pcgb_dpf_keyed_full_eval(int K, int n, int w, int prg, const pcgb_blk* d_roo
         uint32_t* d_rk = nullptr;
         if (prg == PCGB_PRG_AES) d_rk = pcgb::aes_upload_round_keys(round_keys, nk, st);
         const size_t sn = pcgb::keyed_tops_scratch_nodes(K, w, prg, levels);
+        const Blk* roots = reinterpret_cast<const Blk*>(d_roots);
+        // Roots inside the leaves' memory are walked from a copy: a walk of one
+        // stage writes one key's leaves while another's root is still to be read.
+        const size_t rb = static_cast<size_t>(K) * sizeof(Blk);
+        const bool inside = pcgb::overlap(pcgb::range_of(d_roots, rb),
+                                          pcgb::range_of(d_leaves, rb << n));
+        const size_t nodes = sn + (inside ? K : 0);
         Blk* scratch = nullptr;
-        if (sn) scratch = static_cast<Blk*>(pcgb::pool_alloc(sn * sizeof(Blk), st));
-        pcgb::keyed_expand_tops(K, n, w, prg, reinterpret_cast<const Blk*>(d_roots),
-                                reinterpret_cast<const Blk*>(d_cws), d_rk, levels,
-                                reinterpret_cast<Blk*>(d_leaves), scratch, st);
+        if (nodes) scratch = static_cast<Blk*>(pcgb::pool_alloc(nodes * sizeof(Blk), st));
+        if (inside) {
+            PCGB_CK(cudaMemcpyAsync(scratch + sn, roots, rb, cudaMemcpyDeviceToDevice, st));
+            roots = scratch + sn;
+        }
+        pcgb::keyed_expand_tops(K, n, w, prg, roots, reinterpret_cast<const Blk*>(d_cws), d_rk,
+                                levels, reinterpret_cast<Blk*>(d_leaves), scratch, st);
         if (scratch) PCGB_CK(cudaFreeAsync(scratch, st));
         if (d_rk) {
             PCGB_CK(cudaStreamSynchronize(st));

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "field.cuh"
+#include "ranges.h"
 
 namespace pcgb {
 
@@ -167,7 +168,42 @@ void keyed_full_eval_multi(int groups, const int* K, const int* n, int w, int pr
     if (!n) fail(PCGB_EINVAL, "keyed eval multi: null array");
     std::vector<int> to(groups);
     for (int g = 0; g < groups; ++g) to[g] = (w >= 1 && w <= 4) ? n[g] / w : 0;
-    keyed_tops_multi(groups, K, n, to.data(), w, prg, roots, cws, d_rk, leaves, nullptr, st);
+    // Roots inside some group's leaves are walked from copies (as for one group,
+    // pcgb_dpf_keyed_full_eval).
+    size_t keys = 0;
+    if (K && roots && leaves) {
+        std::vector<Range> in, out;
+        for (int g = 0; g < groups; ++g) {
+            if (K[g] <= 0 || n[g] < 1 || n[g] > 30 || !roots[g] || !leaves[g]) continue;
+            const size_t rb = static_cast<size_t>(K[g]) * sizeof(Blk);
+            in.push_back(range_of(roots[g], rb));
+            out.push_back(range_of(leaves[g], rb << n[g]));
+            keys += static_cast<size_t>(K[g]);
+        }
+        if (!any_overlap(in, out)) keys = 0;
+    }
+    if (keys == 0) {
+        keyed_tops_multi(groups, K, n, to.data(), w, prg, roots, cws, d_rk, leaves, nullptr, st);
+        return;
+    }
+    Blk* copy = static_cast<Blk*>(pool_alloc(keys * sizeof(Blk), st));
+    try {
+        std::vector<const Blk*> from(roots, roots + groups);
+        size_t o = 0;
+        for (int g = 0; g < groups; ++g) {
+            if (K[g] <= 0 || n[g] < 1 || n[g] > 30 || !roots[g] || !leaves[g]) continue;
+            PCGB_CK(cudaMemcpyAsync(copy + o, roots[g], K[g] * sizeof(Blk),
+                                    cudaMemcpyDeviceToDevice, st));
+            from[g] = copy + o;
+            o += static_cast<size_t>(K[g]);
+        }
+        keyed_tops_multi(groups, K, n, to.data(), w, prg, from.data(), cws, d_rk, leaves, nullptr,
+                         st);
+    } catch (...) {
+        cudaFreeAsync(copy, st);
+        throw;
+    }
+    PCGB_CK(cudaFreeAsync(copy, st));
 }
 
 // Gather plan: for pair q = (i <= j) and output bin r, the key halves of

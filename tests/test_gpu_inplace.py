@@ -97,3 +97,36 @@ def test_expand_from_g_over_g(pcg):
         assert (d_g.download(np.uint64, c * c * N)[N * block:N * (block + 1)] == want[0]).all()
         assert (d_z.download(np.uint64, N) == want[1]).all()
     e.close()
+
+
+# Walks of one breadth-first stage (n <= 10), of two, and one deeper; the first
+# and the last keys' leaves hold the roots.
+@pytest.mark.parametrize("prg", ["chacha8", "aes"])
+@pytest.mark.parametrize("K,n,w", [(64, 9, 1), (300, 10, 2), (1000, 12, 1), (7, 4, 4)])
+def test_keyed_eval_over_its_roots(pcg, K, n, w, prg):
+    aes = prg == "aes"
+    rng = np.random.default_rng(K + n)
+    nk = (1 << w) - 1
+    words = lambda k: rng.integers(0, 2**64 - 1, 2 * k, dtype=np.uint64)
+    rk = pcg.aes_tree_round_keys(bytes(range(16)), nk) if aes else None
+    kind = pcg.PRG_AES if aes else pcg.PRG_CHACHA8
+    roots, d_cws = words(K), pcg.to_device(words(K * (n // w) * nk))
+    d_roots, d_l = pcg.to_device(roots), pcg.DeviceBuffer(16 * K << n)
+    pcg.dpf_keyed_full_eval_device(K, n, w, kind, d_roots.ptr, d_cws.ptr, d_l.ptr, rk)
+    pcg.synchronize()
+    want = d_l.download(np.uint64, 2 * K << n)
+    for at in (0, 16 * ((K << n) - K)):
+        d_l.upload_at(roots, at)
+        pcg.dpf_keyed_full_eval_device(K, n, w, kind, d_l.ptr + at, d_cws.ptr, d_l.ptr, rk)
+        pcg.synchronize()
+        assert (d_l.download(np.uint64, 2 * K << n) == want).all()
+        # Two groups, each with its roots in the other's leaves.
+        d_m = pcg.DeviceBuffer(16 * K << n)
+        d_l.upload_at(roots, at)
+        d_m.upload_at(roots, at)
+        pcg.dpf_keyed_full_eval_multi_device(
+            [(K, n, d_m.ptr + at, d_cws.ptr, d_l.ptr), (K, n, d_l.ptr + at, d_cws.ptr, d_m.ptr)],
+            w, kind, rk)
+        pcg.synchronize()
+        assert (d_l.download(np.uint64, 2 * K << n) == want).all()
+        assert (d_m.download(np.uint64, 2 * K << n) == want).all()
