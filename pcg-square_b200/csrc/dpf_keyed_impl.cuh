@@ -227,12 +227,28 @@ inline int tops_bfs_threads(int w, int nlev, int g) {
     const int parents = g << (w * (nlev - 1));
     return parents < 32 ? 32 : (parents < kTopsBfsThreads ? parents : kTopsBfsThreads);
 }
-// Two node buffers, the CWs, the AES tables: at most 32 KB + 8 KB + 35 KB.
+// Two node buffers, the CWs, the AES tables.
 template <int PRG>
 size_t tops_bfs_smem(int w, int nlev, int g) {
     const size_t nodes = (static_cast<size_t>(2 * g) << (w * (nlev - 1))) +
                          static_cast<size_t>(g) * nlev * ((1 << w) - 1);
     return nodes * sizeof(Blk) + (PRG == kPrgAes ? sizeof(AesSmem) : 0);
+}
+// The most a stage takes (tops_bfs_ok, tops_bfs_group): 2048 nodes in the two
+// buffers and 240 CWs (w = 4, 16 keys).
+constexpr size_t tops_bfs_smem_max(int prg) {
+    return (2048 + 240) * sizeof(Blk) + (prg == kPrgAes ? sizeof(AesSmem) : 0);
+}
+// A kernel's limit of dynamic shared memory is an attribute that all threads of
+// the process share.  It is set to one value, the most the kernel ever takes, and
+// not to what the launch at hand needs: another thread would lower it between
+// this one's setting and its launch.
+template <class... P>
+void allow_smem(void (*kern)(P...), size_t bytes, size_t most) {
+    if (bytes > most) fail(PCGB_EINVAL, "shared memory beyond the kernel's limit");
+    if (bytes > 48 * 1024)
+        PCGB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(most)));
 }
 
 // ---------------------------------------------------------------------------
@@ -729,10 +745,7 @@ void launch_tops(const Blk* src, int K, int src_lvl, int nlev, int levels, const
     if (tops_bfs_ok(K, W, src_lvl, nlev)) {
         const int G = tops_bfs_group(K, W, nlev);
         const size_t smem = tops_bfs_smem<PRG>(W, nlev, G);
-        if (smem > 48 * 1024)
-            PCGB_CK(cudaFuncSetAttribute(tops_bfs_kernel<W, PRG>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem)));
+        allow_smem(tops_bfs_kernel<W, PRG>, smem, tops_bfs_smem_max(PRG));
         tops_bfs_kernel<W, PRG><<<(K + G - 1) / G, tops_bfs_threads(W, nlev, G), smem, st>>>(
             src, K, G, nlev, levels, cws, te, rk, dst);
         PCGB_POST_LAUNCH();
@@ -934,10 +947,7 @@ void tops_multi_launch(const std::vector<TopsJob>& all, TopsJob* d_jobs, const u
     if (!first.empty()) {
         PCGB_CK(cudaMemcpyAsync(d_jobs, first.data(), first.size() * sizeof(TopsJob),
                                 cudaMemcpyHostToDevice, st));
-        if (bfs_smem > 48 * 1024)
-            PCGB_CK(cudaFuncSetAttribute(tops_bfs_multi_kernel<W, PRG>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(bfs_smem)));
+        allow_smem(tops_bfs_multi_kernel<W, PRG>, bfs_smem, tops_bfs_smem_max(PRG));
         tops_bfs_multi_kernel<W, PRG><<<static_cast<unsigned>(ctas), threads, bfs_smem, st>>>(
             d_jobs, static_cast<int>(first.size()), te, rk);
         PCGB_POST_LAUNCH();
@@ -1020,20 +1030,21 @@ void tops_multi_for_prg(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs
 }
 
 // After the top walk, in clusters of 1 << lsplit CTAs.
-template <class... P, class... A>
+template <int S, int PRG, class... P, class... A>
 void launch_split(void (*kern)(P...), dim3 grid, int tpb, size_t smem, int lsplit, cudaStream_t st,
                   const A&... args) {
-    if (smem > 48 * 1024)
-        PCGB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
+    // CTAs of up to 256 threads (the kernels' launch bound).
+    allow_smem(kern, smem,
+               256 * (S + 1) * sizeof(ulonglong2) + (PRG == kPrgAes ? sizeof(AesSmem) : 0));
     launch({grid, dim3(static_cast<unsigned>(tpb)), smem, true, 1u << lsplit}, st, kern, args...);
 }
 
 template <int W, int SL, int PRG>
 void leaf_one(const LeafLaunch& L) {
-    launch_split(leaf_gather_kernel<W, SL, PRG>, L.grid, L.tpb, L.smem, L.lsplit, L.st, L.F, L.cws,
-                 L.cw_out, L.off, L.entries, L.q_order, L.q_slot, L.t, L.levels, L.hl, L.bin, L.N,
-                 L.party, L.lsplit, L.te, L.rk, L.gq);
+    launch_split<1 << (W * SL), PRG>(leaf_gather_kernel<W, SL, PRG>, L.grid, L.tpb, L.smem,
+                                     L.lsplit, L.st, L.F, L.cws, L.cw_out, L.off, L.entries,
+                                     L.q_order, L.q_slot, L.t, L.levels, L.hl, L.bin, L.N, L.party,
+                                     L.lsplit, L.te, L.rk, L.gq);
 }
 
 template <int W, int SL, int PRG>
@@ -1048,8 +1059,9 @@ void leaf_multi_one(const LeafJob* jobs, int njobs, int lsplit, int tpb, size_t 
             tab.job[i].first = clusters;
             clusters += tab.job[i].gx * tab.job[i].gy * tab.job[i].gz;
         }
-        launch_split(leaf_gather_multi_kernel<W, SL, PRG>, dim3(clusters << lsplit), tpb, smem,
-                     lsplit, st, tab, n, lsplit, te, rk);
+        launch_split<1 << (W * SL), PRG>(leaf_gather_multi_kernel<W, SL, PRG>,
+                                         dim3(clusters << lsplit), tpb, smem, lsplit, st, tab, n,
+                                         lsplit, te, rk);
     }
 }
 
