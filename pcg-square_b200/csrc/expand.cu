@@ -244,9 +244,7 @@ struct pcgb_expander {
     uint64_t* d_img = nullptr;   // Q*N
     uint64_t* d_aR = nullptr;    // (c-i0)*N: a_i0 .. a_{c-1}, Montgomery form
     int i0 = 1;                  // 1: a_0 = 1 (the reference); 0: a_0 public
-    pcgb::Blk* d_F = nullptr;
-    pcgb::Blk* d_tops = nullptr;
-    uint64_t* d_g = nullptr;     // Q*N
+    pcgb::Blk* d_F = nullptr;    // own workspace, laid out by workspace_carve
     uint32_t* d_rk = nullptr;    // AES sub-key schedules
     size_t scratch_bytes = 0;
     size_t own_ws_bytes = 0;     // size of d_F when allocated
@@ -609,7 +607,8 @@ void digest_multi_device(int count, const uint64_t* const* v, const size_t* n, u
 }
 
 // The expander's own workspace, allocated on first use (plans held by the
-// server never need it: requests bring their own).
+// server never need it: requests bring their own).  Its layout follows the leaf
+// shape of the moment (own_workspace), which can change while the memory stays.
 void ensure_own_workspace(pcgb_expander* e) {
     if (e->d_F && e->own_ws_bytes >= e->scratch_bytes) return;
     if (e->d_F) {
@@ -624,9 +623,10 @@ void ensure_own_workspace(pcgb_expander* e) {
     }
     PCGB_CK(cudaMalloc(&e->d_F, e->scratch_bytes));
     e->own_ws_bytes = e->scratch_bytes;
-    const Workspace ws = workspace_carve(e, e->d_F);
-    e->d_tops = ws.tops;
-    e->d_g = ws.g;
+}
+Workspace own_workspace(pcgb_expander* e) {
+    ensure_own_workspace(e);
+    return workspace_carve(e, e->d_F);
 }
 
 // With graphs on, the first call runs directly (plans, tables and kernel
@@ -638,12 +638,9 @@ void expand_device(pcgb_expander* e, int party, const Blk* roots, const Blk* cws
                    const uint64_t* cw_out, const uint64_t* pos, const uint64_t* val, uint64_t* x,
                    uint64_t* z, cudaStream_t st) {
     ensure_own_workspace(e);
-    Workspace ws;
-    ws.F = e->d_F;
-    ws.tops = e->d_tops;
-    ws.g = e->d_g;
     const bool profiling = e->prof_slots > 0 && e->prof_used < e->prof_slots;
     if (!e->use_graph || profiling || !e->graph_warm) {
+        const Workspace ws = workspace_carve(e, e->d_F);
         expand_device_ws(e, ws, party, roots, cws, cw_out, pos, val, x, z, st);
         e->graph_warm = true;
         return;
@@ -654,6 +651,7 @@ void expand_device(pcgb_expander* e, int party, const Blk* roots, const Blk* cws
         note_launches(e->graph_kernels);
         return;
     }
+    const Workspace ws = workspace_carve(e, e->d_F);
     Fork& f = e->graph_fork;
     if (!f.begin) PCGB_CK(cudaEventCreateWithFlags(&f.begin, cudaEventDisableTiming));
     if (!f.end) PCGB_CK(cudaEventCreateWithFlags(&f.end, cudaEventDisableTiming));
@@ -861,7 +859,7 @@ void expand_host_async(pcgb_expander* e, int party, const Blk* roots, const Blk*
     const size_t in_bytes = b_roots + b_cws + b_cwo + 2 * b_noise;
     const size_t dev_bytes = in_bytes + 2 * b_out;
     if (!e->async_compute) PCGB_CK(cudaEventCreateWithFlags(&e->async_compute, cudaEventDisableTiming));
-    ensure_own_workspace(e);
+    const Workspace ws = own_workspace(e);
     auto& a = e->aslot[e->aturn];
     e->aturn ^= 1;
     if (!a.st) PCGB_CK(cudaStreamCreateWithFlags(&a.st, cudaStreamNonBlocking));
@@ -886,10 +884,6 @@ void expand_host_async(pcgb_expander* e, int party, const Blk* roots, const Blk*
     PCGB_CK(cudaMemcpyAsync(d_pos, pos, b_noise, cudaMemcpyHostToDevice, a.st));
     PCGB_CK(cudaMemcpyAsync(d_val, val, b_noise, cudaMemcpyHostToDevice, a.st));
     if (e->async_pending) PCGB_CK(cudaStreamWaitEvent(a.st, e->async_compute, 0));
-    Workspace ws;
-    ws.F = e->d_F;
-    ws.tops = e->d_tops;
-    ws.g = e->d_g;
     expand_device_ws(e, ws, party, d_roots, d_cws, d_cwo, d_pos, d_val, d_x, d_z, a.st);
     PCGB_CK(cudaEventRecord(e->async_compute, a.st));
     e->async_pending = true;
@@ -938,24 +932,24 @@ void expand_from_g_device(pcgb_expander* e, const uint64_t* g, const uint64_t* p
                           const uint64_t* val, uint64_t* x, uint64_t* z, cudaStream_t st) {
     if (!g || !pos || !val || !x || !z) fail(PCGB_EINVAL, "expand_from_g: null pointer");
     if (e->gp.world != 1) fail(PCGB_EINVAL, "expand_from_g: needs an unsharded expander");
-    ensure_own_workspace(e);
+    const Workspace ws = own_workspace(e);
     const size_t NN = static_cast<size_t>(e->N);
-    pair_merge_kernel<<<dim3(blocks_for(NN, 256), e->Q), 256, 0, st>>>(g, e->c, NN, e->d_g);
+    pair_merge_kernel<<<dim3(blocks_for(NN, 256), e->Q), 256, 0, st>>>(g, e->c, NN, ws.g);
     PCGB_POST_LAUNCH();
     const size_t sm = sizeof(uint64_t) * 2 * static_cast<size_t>(e->c) * e->t;
     const size_t words = NN * sizeof(uint64_t);
     const bool early = !overlap(range_of(x, words), range_of(g, words * e->c * e->c));
     launch({blocks_for(NN, 256), 256, sm, early}, st, x_kernel, pos, val, e->d_aR, e->c, e->t, e->i0,
            NN, x);
-    ntt_mac_inverse(*e->ntt, e->d_g, e->d_img, e->Q, z, st);
+    ntt_mac_inverse(*e->ntt, ws.g, e->d_img, e->Q, z, st);
 }
 
 void expand_g_device(pcgb_expander* e, int party, const Blk* roots, const Blk* cws,
                      const uint64_t* cw_out, uint64_t* d_g, cudaStream_t st) {
     if (!roots || !cws || !cw_out || !d_g) fail(PCGB_EINVAL, "expand_g: null pointer");
-    ensure_own_workspace(e);
-    keyed_expand_tops(e->K, e->n, e->w, e->prg, roots, cws, e->d_rk, e->gp.hl, e->d_F, e->d_tops, st);
-    keyed_leaf_gather(e->gp, party, e->prg, e->d_F, cws, cw_out, e->d_rk, d_g, st);
+    const Workspace ws = own_workspace(e);
+    keyed_expand_tops(e->K, e->n, e->w, e->prg, roots, cws, e->d_rk, e->gp.hl, ws.F, ws.tops, st);
+    keyed_leaf_gather(e->gp, party, e->prg, ws.F, cws, cw_out, e->d_rk, d_g, st);
 }
 
 // out (device, one word) = digest of d[0..n); accumulates, so zero it first.
