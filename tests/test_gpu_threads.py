@@ -48,3 +48,35 @@ def test_stages_of_different_shared_memory(pcg):
     pcg.synchronize()
     for a, w in zip(args, want):
         assert (a[-1][2].download(np.uint64, 2 * a[0] << a[1]) == w).all()
+
+
+def test_large_host_transfers(pcg):
+    """Arrays of 24 MB, moved by helper threads where a call has the staging
+    buffer and directly where another call has it; each thread has operands of
+    its own (b = X^k), so a crossed buffer shows."""
+    N, batch = 1 << 20, 3
+    rng = np.random.default_rng(8)
+    a = [rng.integers(0, pcg.P, batch * N, dtype=np.uint64) for _ in range(3)]
+    ks = [5, 70001, N - 3]
+    want, b = [], []
+    for v, k in zip(a, ks):
+        r = np.roll(v.reshape(batch, N), k, axis=1)
+        r[:, :k] = (np.uint64(pcg.P) - r[:, :k]) % np.uint64(pcg.P)
+        want.append(r.reshape(-1))
+        m = np.zeros((batch, N), np.uint64)
+        m[:, k] = 1
+        b.append(m.reshape(-1))
+    bad = []
+
+    def work(i):
+        for _ in range(4):
+            got, _ = pcg.poly_mul_u64_gpuntt(a[i], b[i], batch, N)
+            if not (got == want[i]).all():
+                bad.append(i)
+
+    th = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not bad
