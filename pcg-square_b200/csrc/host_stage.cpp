@@ -175,7 +175,8 @@ bool HostStage::reserve(size_t total) {
 }
 
 HostStage::~HostStage() {
-    if (pending) cudaStreamSynchronize(pending);   // a call that failed half way
+    // A call that failed half way; its own error is the one reported.
+    if (pending && cudaStreamSynchronize(pending) != cudaSuccess) cudaGetLastError();
     delete im;
 }
 

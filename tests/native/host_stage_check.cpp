@@ -19,13 +19,17 @@
 namespace pcgb {
 void fail(int code, const std::string& msg) { throw Error(code, msg); }
 void check_cuda(cudaError_t e, const char* what) {
-    if (e != cudaSuccess) throw Error(PCGB_ECUDA, what);
+    if (e == cudaSuccess) return;
+    cudaGetLastError();
+    throw Error(PCGB_ECUDA, what);
 }
 }  // namespace pcgb
 
 static std::atomic<int> event_delay_ms{0};   // of the next event wait
 static std::atomic<int> events_left{-1};     // event waits until one fails; < 0: none does
 static std::atomic<int> in_flight{0};        // copies the stream was not waited for since
+static bool sync_fails = false;
+static cudaError_t last_error = cudaSuccess;
 static const void* pinned_at = nullptr;      // an address that counts as pinned memory
 // Allocations until one throws (those of a transfer are its threads' states); < 0: none does.
 static thread_local int allocations_left = -1;
@@ -42,7 +46,11 @@ void operator delete(void* p, std::size_t) noexcept { std::free(p); }
 extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = last_error;
+    last_error = cudaSuccess;
+    return e;
+}
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     a->type = p == pinned_at ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
     return cudaSuccess;
@@ -56,7 +64,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t) {
     in_flight = 0;
-    return cudaSuccess;
+    return last_error = sync_fails ? cudaErrorStreamCaptureUnsupported : cudaSuccess;
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
     *e = reinterpret_cast<cudaEvent_t>(1);
@@ -65,7 +73,7 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) {
     std::this_thread::sleep_for(std::chrono::milliseconds(event_delay_ms.exchange(0)));
-    if (events_left == 0) return cudaErrorUnknown;
+    if (events_left == 0) return last_error = cudaErrorUnknown;
     if (events_left > 0) --events_left;
     return cudaSuccess;
 }
@@ -173,6 +181,17 @@ int run_failed(size_t mb) {
                 expect(at < static_cast<size_t>(good) << 20 || a.out[i][k] == 0x5a,
                        "outputs a failed call does not reach");
     }
+    // Nor an error for the next launch's check to find.
+    try {
+        pcgb::HostStage io;
+        events_left = 0;
+        sync_fails = true;
+        io.download(dst, a.len, 3, a.dev.data(), kStream);
+    } catch (const pcgb::Error&) {
+    }
+    events_left = -1;
+    sync_fails = false;
+    expect(cudaGetLastError() == cudaSuccess, "no error left behind");
     return 0;
 }
 
