@@ -175,6 +175,30 @@ void upload_blocking(void* d_dst, const void* src, size_t bytes) {
     check_cuda(cudaStreamSynchronize(st), "upload sync");
 }
 
+void upload_table(void* d_dst, const void* src, size_t bytes, cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    check_cuda(cudaStreamIsCapturing(st, &status), "cudaStreamIsCapturing");
+    if (status != cudaStreamCaptureStatusNone && bytes) {
+        // The graph copies at every replay: it gets a table of its own.
+        unsigned long long id = 0;
+        cudaGraph_t graph = nullptr;
+        check_cuda(cudaStreamGetCaptureInfo(st, &status, &id, &graph), "cudaStreamGetCaptureInfo");
+        char* own = new char[bytes];
+        std::memcpy(own, src, bytes);
+        cudaUserObject_t obj = nullptr;
+        const cudaError_t e = cudaUserObjectCreate(
+            &obj, own, [](void* p) { delete[] static_cast<char*>(p); }, 1,
+            cudaUserObjectNoDestructorSync);
+        if (e != cudaSuccess) delete[] own;
+        check_cuda(e, "cudaUserObjectCreate");
+        const cudaError_t r = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+        if (r != cudaSuccess) cudaUserObjectRelease(obj, 1);
+        check_cuda(r, "cudaGraphRetainUserObject");
+        src = own;
+    }
+    check_cuda(cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, st), "table upload");
+}
+
 int sm_count() {
     int dev = 0, n = 0;
     check_cuda(cudaGetDevice(&dev), "cudaGetDevice");

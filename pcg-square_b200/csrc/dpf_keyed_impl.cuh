@@ -945,8 +945,7 @@ void tops_multi_launch(const std::vector<TopsJob>& all, TopsJob* d_jobs, const u
         }
     }
     if (!first.empty()) {
-        PCGB_CK(cudaMemcpyAsync(d_jobs, first.data(), first.size() * sizeof(TopsJob),
-                                cudaMemcpyHostToDevice, st));
+        upload_table(d_jobs, first.data(), first.size() * sizeof(TopsJob), st);
         allow_smem(tops_bfs_multi_kernel<W, PRG>, bfs_smem, tops_bfs_smem_max(PRG));
         tops_bfs_multi_kernel<W, PRG><<<static_cast<unsigned>(ctas), threads, bfs_smem, st>>>(
             d_jobs, static_cast<int>(first.size()), te, rk);
@@ -974,8 +973,7 @@ void tops_multi_launch(const std::vector<TopsJob>& all, TopsJob* d_jobs, const u
                 byd[i].first = seg_total[k];
                 seg_total[k] += static_cast<unsigned long long>(byd[i].K) << byd[i].src_lvl;
             }
-        PCGB_CK(cudaMemcpyAsync(d_jobs, byd.data(), byd.size() * sizeof(TopsJob),
-                                cudaMemcpyHostToDevice, st));
+        upload_table(d_jobs, byd.data(), byd.size() * sizeof(TopsJob), st);
         for (size_t k = 0; k + 1 < seg.size(); ++k) {
             const unsigned long long tot = seg_total[k];
             if (tot == 0) continue;
@@ -995,8 +993,7 @@ void tops_multi_launch(const std::vector<TopsJob>& all, TopsJob* d_jobs, const u
         }
         return;
     }
-    PCGB_CK(cudaMemcpyAsync(d_jobs, jobs.data(), jobs.size() * sizeof(TopsJob),
-                            cudaMemcpyHostToDevice, st));
+    upload_table(d_jobs, jobs.data(), jobs.size() * sizeof(TopsJob), st);
     if constexpr (PRG == kPrgAes) {
         if (total >= aes_prmt_wave()) {   // as launch_tops
             PCGB_CK(cudaFuncSetAttribute(expand_tops_multi_prmt_kernel<W>,

@@ -526,7 +526,7 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
         for (const Range& k : key_ranges(E, roots[i], cws[i], cw_out[i])) keys.push_back(k);
     }
     char* tab = static_cast<char*>(pool_alloc(sizeof(XJob) * count, st));
-    PCGB_CK(cudaMemcpyAsync(tab, xj.data(), sizeof(XJob) * count, cudaMemcpyHostToDevice, st));
+    upload_table(tab, xj.data(), sizeof(XJob) * count, st);
     // Stage 2: the fused leaf kernel over every expansion's tiles.
     const size_t leaf_smem = static_cast<size_t>(tpb) * (S + 1) * 2 * sizeof(uint64_t);
     double leaves = 0;
@@ -580,7 +580,7 @@ void deal_noise_multi_device(int count, pcgb_expander* const* e, const uint64_t*
     std::memcpy(host.data(), deal.data(), b_deal);
     std::memcpy(host.data() + o_noise, noise.data(), sizeof(NoiseJob) * count);
     char* tab = static_cast<char*>(pool_alloc(total, st));
-    PCGB_CK(cudaMemcpyAsync(tab, host.data(), total, cudaMemcpyHostToDevice, st));
+    upload_table(tab, host.data(), total, st);
     deal_multi_chacha_launch(w, reinterpret_cast<const DealJob*>(tab), count, ctas, r2_mod_p(), st);
     noise_multi_kernel<<<count, 128, 0, st>>>(reinterpret_cast<const NoiseJob*>(tab + o_noise));
     PCGB_POST_LAUNCH();
@@ -599,7 +599,7 @@ void digest_multi_device(int count, const uint64_t* const* v, const size_t* n, u
     }
     const unsigned per = static_cast<unsigned>(std::min<size_t>((longest + 255) / 256, 256));
     DigestJob* d = static_cast<DigestJob*>(pool_alloc(sizeof(DigestJob) * count, st));
-    PCGB_CK(cudaMemcpyAsync(d, jobs.data(), sizeof(DigestJob) * count, cudaMemcpyHostToDevice, st));
+    upload_table(d, jobs.data(), sizeof(DigestJob) * count, st);
     for (int i = 0; i < count; ++i) PCGB_CK(cudaMemsetAsync(out[i], 0, sizeof(uint64_t), st));
     digest_multi_kernel<<<per * static_cast<unsigned>(count), 256, 0, st>>>(d, per);
     PCGB_POST_LAUNCH();

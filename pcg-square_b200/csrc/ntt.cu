@@ -1338,9 +1338,9 @@ void poly_mul_device_mixed(int count, uint64_t* const* c, const uint64_t* const*
     const size_t o_col = (b_polys + 255) & ~size_t{255};
     const size_t o_row = (o_col + b_col + 255) & ~size_t{255};
     char* tab = static_cast<char*>(pool_alloc(o_row + b_row, st));
-    PCGB_CK(cudaMemcpyAsync(tab, polys.data(), b_polys, cudaMemcpyHostToDevice, st));
-    PCGB_CK(cudaMemcpyAsync(tab + o_col, col.data(), b_col, cudaMemcpyHostToDevice, st));
-    PCGB_CK(cudaMemcpyAsync(tab + o_row, row.data(), b_row, cudaMemcpyHostToDevice, st));
+    upload_table(tab, polys.data(), b_polys, st);
+    upload_table(tab + o_col, col.data(), b_col, st);
+    upload_table(tab + o_row, row.data(), b_row, st);
     const MixedPoly* d_polys = reinterpret_cast<const MixedPoly*>(tab);
     const MixedCta* d_col = reinterpret_cast<const MixedCta*>(tab + o_col);
     const MixedCta* d_row = reinterpret_cast<const MixedCta*>(tab + o_row);
@@ -1423,7 +1423,7 @@ void ntt_mac_inverse_multi(int count, uint64_t* const* g, const uint64_t* const*
     for (int i = 0; i < 4; ++i)
         std::memcpy(host.data() + o[i], lists[i]->data(), sizeof(MacCta) * lists[i]->size());
     char* tab = static_cast<char*>(pool_alloc(total, st));
-    PCGB_CK(cudaMemcpyAsync(tab, host.data(), total, cudaMemcpyHostToDevice, st));
+    upload_table(tab, host.data(), total, st);
     const MacReq* d_req = reinterpret_cast<const MacReq*>(tab);
     auto ctas = [&](int i) { return reinterpret_cast<const MacCta*>(tab + o[i]); };
     auto grid = [&](int i) { return static_cast<unsigned>(lists[i]->size()); };

@@ -83,6 +83,10 @@ class HostStage {
     cudaStream_t pending = nullptr;   // the stream with copies that may not have ended
 };
 void upload_blocking(void* d_dst, const void* src, size_t bytes);
+// A job table from host memory that goes away after the call, copied on st.
+// While st captures a graph, the copy reads from memory that the graph owns: a
+// replay would otherwise take its pointers from whatever the heap holds by then.
+void upload_table(void* d_dst, const void* src, size_t bytes, cudaStream_t st);
 // Stream-ordered allocation from the library's own per-device pool, which
 // keeps freed memory mapped for the next request (release with
 // pcgb_trim_pool).  Free with cudaFreeAsync.
