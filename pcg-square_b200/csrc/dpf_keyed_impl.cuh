@@ -802,8 +802,8 @@ void launch_tops(const Blk* src, int K, int src_lvl, int nlev, int levels, const
         }
     }
     const size_t smem = PRG == kPrgAes ? sizeof(AesSmem) : 0;
-    launch({grid, TPB, smem, chained}, st, expand_tops_kernel<W, PRG>, src, K, src_lvl, nlev, levels,
-           cws, te, rk, dst);
+    launch({grid, TPB, smem, chained}, st, expand_tops_kernel<W, PRG>, src, K, src_lvl, nlev,
+           levels, cws, te, rk, dst);
 }
 
 template <int W, int PRG>
@@ -1063,7 +1063,8 @@ void leaf_multi_one(const LeafJob* jobs, int njobs, int lsplit, int tpb, size_t 
 }
 
 template <int PRG>
-void leaf_multi_for_prg(int w, int sl, const LeafJob* jobs, int njobs, int lsplit, int tpb, size_t smem, const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
+void leaf_multi_for_prg(int w, int sl, const LeafJob* jobs, int njobs, int lsplit, int tpb,
+                        size_t smem, const uint32_t* te, const uint32_t* rk, cudaStream_t st) {
     switch (w * 8 + sl) {
 #define PCGB_LM(W_, SL_)                                                              \
     case W_ * 8 + SL_:                                                                \

@@ -7,9 +7,9 @@
 //   z      = sum_{i,j} a_i a_j g_ij = INTT( sum_{i<=j} (a^_i a^_j) . NTT(g_ij + g_ji) )
 //
 // The expander keeps, per shape, the a_i coefficients (Montgomery form, for
-// the sparse x product) and the c(c+1)/2 evaluation images a^_i a^_j resident, so an expansion is four device stages:
-// keyed tops -> fused leaf/convert/gather -> sparse x -> NTT multiply-
-// accumulate + inverse.  Blocks (i,j) and (j,i) are merged while g is
+// the sparse x product) and the c(c+1)/2 evaluation images a^_i a^_j resident,
+// so an expansion is four device stages: keyed tops -> fused leaf/convert/gather
+// -> sparse x -> NTT multiply-accumulate + inverse.  Blocks (i,j) and (j,i) are merged while g is
 // produced (a_i a_j = a_j a_i), so only c(c+1)/2 forward transforms run.
 #include "pcgb_internal.h"
 
@@ -405,7 +405,7 @@ static std::array<Range, 3> key_ranges(const pcgb_expander* e, const Blk* roots,
 
 // fork (while a graph is captured): x becomes a branch of its own beside the
 // walk and the leaf kernel, which leave the multiplier pipe and the L2 idle (its
-// 0.14 ms of the headline's 15.06, 4 of the 39 us at N = 2^12).  Launched directly
+// 0.14 ms of the headline's 15.06; 36.9 -> 34.9 us at N = 2^12).  Launched directly
 // it follows the leaf kernel and fills its last wave (x_kernel).
 static void expand_stages(pcgb_expander* e, const Workspace& ws, int party, const Blk* roots,
                           const Blk* cws, const uint64_t* cw_out, const uint64_t* pos,
@@ -456,8 +456,7 @@ void expand_device_ws(pcgb_expander* e, const Workspace& ws, int party, const Bl
 // depth sl for all): one launch per top-walk stage, one fused leaf launch,
 // one x launch and four NTT launches for the whole batch, each CTA finding
 // its expansion in a job table (the leaf launch holds up to 32 expansions).
-// Outputs equal expand_device_ws's, request by request.  All job tables travel in one copy from pinned or pageable host
-// memory on `st`.
+// Outputs equal expand_device_ws's, request by request.
 void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, const int* party,
                      const Blk* const* roots, const Blk* const* cws,
                      const uint64_t* const* cw_out, const uint64_t* const* pos,
@@ -537,9 +536,11 @@ void expand_batch_ws(int count, pcgb_expander* const* e, const Workspace* ws, co
         while (lsplit > 0 && (2 * e[i]->t >> lsplit) < 2) --lsplit;
     }
     lsplit = std::min(lsplit, leaf_lsplit(leaves, S, t_max));
-    keyed_leaf_multi_chacha(w, sl, leaf.data(), count, lsplit, tpb, leaf_smem, nullptr, nullptr, st);
+    keyed_leaf_multi_chacha(w, sl, leaf.data(), count, lsplit, tpb, leaf_smem, nullptr, nullptr,
+                            st);
     // Stage 3: the sparse x products.
-    launch({x_ctas, 256, x_smem, !any_overlap(outs, keys)}, st, x_multi_kernel, reinterpret_cast<const XJob*>(tab), count);
+    launch({x_ctas, 256, x_smem, !any_overlap(outs, keys)}, st, x_multi_kernel,
+           reinterpret_cast<const XJob*>(tab), count);
     // Stage 4: NTT multiply-accumulate and inverse, all lengths at once.
     std::vector<uint64_t*> g(count), zz(count);
     std::vector<const uint64_t*> img(count);
@@ -939,8 +940,8 @@ void expand_from_g_device(pcgb_expander* e, const uint64_t* g, const uint64_t* p
     const size_t sm = sizeof(uint64_t) * 2 * static_cast<size_t>(e->c) * e->t;
     const size_t words = NN * sizeof(uint64_t);
     const bool early = !overlap(range_of(x, words), range_of(g, words * e->c * e->c));
-    launch({blocks_for(NN, 256), 256, sm, early}, st, x_kernel, pos, val, e->d_aR, e->c, e->t, e->i0,
-           NN, x);
+    launch({blocks_for(NN, 256), 256, sm, early}, st, x_kernel, pos, val, e->d_aR, e->c, e->t,
+           e->i0, NN, x);
     ntt_mac_inverse(*e->ntt, ws.g, e->d_img, e->Q, z, st);
 }
 

@@ -29,8 +29,8 @@ constexpr size_t kChunk = size_t{1} << 20;
 constexpr int kChunks = static_cast<int>(kStageBytes / kChunk);
 constexpr size_t kPage = 4096;
 // Ranges up to kSmall are staged by this thread alone: one copy instead of one
-// per array.  From kLarge on helper threads pay for their start (16 x 2 MB each
-// way: 2.27 -> 2.07 ms; 3 x 32 MB: 13.0 -> 6.5 ms).  Between the two the
+// per array.  From kLarge on helper threads pay for their start (a product with
+// 3 x 16 MB: 2.9 -> 2.6 ms; 3 x 32 MB: 12.9 -> 5.9 ms).  Between the two the
 // driver's own staging is as good.
 constexpr size_t kSmall = size_t{4} << 20, kLarge = size_t{16} << 20;
 

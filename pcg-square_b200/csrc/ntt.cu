@@ -294,8 +294,9 @@ __device__ __forceinline__ int64_t load_raw(const uint64_t* src, const uint64_t*
 
 // Column pass, forward, for columns [tile*C, tile*C + C).  src may equal
 // dst (every CTA loads its columns before its first store).  Inputs are any
-// 64-bit words.  Outputs within 1.6p, without the four-step twiddle: the row pass applies it together with its own first root.  L2
-// fixes log2(n2) at compile time (element offsets become immediates).
+// 64-bit words.  Outputs within 1.6p, without the four-step twiddle: the row pass
+// applies it together with its own first root.  L2 fixes log2(n2) at compile time
+// (element offsets become immediates).
 template <int L, int C, int L2>
 __device__ __forceinline__ void col_fwd_body(const uint64_t* src, const uint64_t* add,
                                              uint64_t* dst, size_t tile,
@@ -877,8 +878,11 @@ NttTw* upload_root_table(uint64_t psi_n, int logn) {
 // polynomial, so there are no column passes.  Longer ones would keep a single
 // SM busy where the four-step passes spread over several (2^12, three
 // transforms: 18 us against 10).  A product is one launch instead of four
-// passes, so it stays one row up to 2^12: 18.5 us against about 22; at 2^13, 55
-// against 24.7.
+// passes, so it stays one row up to 2^12.  In us, one launch / four chained
+// passes: 10.3 / 14.4 at 2^10; at 2^12 18.5 / 16.5 for one to three products,
+// equal from four on, 18.6 / 28.3 for 74 and 121 / 138.7 for 1000; 55 / 24.7 at 2^13.
+// The 2 us of one to three products at 2^12 would cost three more launches and a
+// scratch allocation on the host, so there is no rule for them.
 constexpr int kDirectLogN = 9, kOneRowLogN = 12;
 
 NttPlan* build_plan(int logN) {

@@ -51,9 +51,6 @@ inline cudaStream_t as_stream(void* s) {
     return s ? static_cast<cudaStream_t>(s) : default_stream();
 }
 
-// Host-to-device copy that has landed when the call returns: a plain
-// cudaMemcpy from pageable memory may return before its DMA completes, and
-// work on the library's non-blocking streams is not ordered after it.
 // Host buffers to and from the device through a pinned buffer (host_stage.cpp).
 // One object per call: it holds the device's buffer until it goes out of scope
 // (another thread's call then copies directly).  `pieces` host ranges of len
@@ -82,6 +79,9 @@ class HostStage {
     size_t used = 0;                  // bytes of the buffer that copies may still read
     cudaStream_t pending = nullptr;   // the stream with copies that may not have ended
 };
+// Host-to-device copy that has landed when the call returns: a plain
+// cudaMemcpy from pageable memory may return before its DMA completes, and
+// work on the library's non-blocking streams is not ordered after it.
 void upload_blocking(void* d_dst, const void* src, size_t bytes);
 // A job table from host memory that goes away after the call, copied on st.
 // While st captures a graph, the copy reads from memory that the graph owns: a
@@ -124,9 +124,10 @@ void keyed_tops_multi(int groups, const int* K, const int* n, const int* to_leve
 void keyed_full_eval_multi(int groups, const int* K, const int* n, int w, int prg,
                            const Blk* const* roots, const Blk* const* cws, const uint32_t* d_rk,
                            Blk* const* leaves, cudaStream_t st);
-void keyed_tops_multi_chacha(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs, cudaStream_t st);
-void keyed_tops_multi_aes(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs, const uint32_t* te, const uint32_t* rk,
-                          cudaStream_t st);
+void keyed_tops_multi_chacha(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
+                             cudaStream_t st);
+void keyed_tops_multi_aes(int w, const std::vector<TopsJob>& jobs, TopsJob* d_jobs,
+                          const uint32_t* te, const uint32_t* rk, cudaStream_t st);
 void keyed_expand_tops(int K, int n, int w, int prg, const Blk* roots, const Blk* cws,
                        const uint32_t* d_aes_rk, int to_level, Blk* out, Blk* scratch,
                        cudaStream_t st);
@@ -136,11 +137,11 @@ void keyed_expand_tops(int K, int n, int w, int prg, const Blk* roots, const Blk
 // [r*bin, (r+1)*bin) of the folded g (see gather_plan in dpf_keyed.cu).
 // Keyed top-level expansion runs in stages.  The first is breadth first
 // (tops_bfs_kernel), until K * m^l reaches the thread count below (and, for w =
-// 1, one depth-first stage can take the rest) or a key has 2^10 nodes.  Each later stage gives every node of its start level a thread
-// that walks its subtree depth first down to the next boundary; the thread
-// count grows at most 32-fold per stage (so narrow stages do short walks)
-// until K * m^l reaches this many subtrees, and the final stage walks from
-// there to the target level.
+// 1, one depth-first stage can take the rest) or a key has 2^10 nodes.  Each
+// later stage gives every node of its start level a thread that walks its
+// subtree depth first down to the next boundary; the thread count grows at most
+// 32-fold per stage (so narrow stages do short walks) until K * m^l reaches this
+// many subtrees, and the final stage walks from there to the target level.
 // 2^19 threads keep every SM busy and the final walks shallow.
 constexpr size_t kTopsStage2Threads = size_t{1} << 19;
 // w = 1 ChaCha8 stages of up to this many levels walk a depth fixed at
@@ -242,7 +243,8 @@ void deal_multi_chacha_launch(int w, const DealJob* d_jobs, int njobs, unsigned 
                            const uint32_t* te, const uint32_t* rk, int to_level, Blk* out,     \
                            Blk* scratch, cudaStream_t st);                                     \
     void keyed_leaf_##NAME(int w, int sl, const LeafLaunch& L);                                 \
-    void keyed_leaf_multi_##NAME(int w, int sl, const LeafJob* jobs, int njobs, int lsplit, int tpb, size_t smem, const uint32_t* te, const uint32_t* rk,  \
+    void keyed_leaf_multi_##NAME(int w, int sl, const LeafJob* jobs, int njobs, int lsplit,     \
+                                 int tpb, size_t smem, const uint32_t* te, const uint32_t* rk,  \
                                  cudaStream_t st);                                              \
     void keyed_deal_##NAME(int w, unsigned grid, size_t smem, uint64_t seed, int c, int t,      \
                            int n, uint64_t bin, Blk* roots0, Blk* roots1, Blk* cws,            \
